@@ -482,13 +482,22 @@ template <int BN> struct Tc2Cfg {
   static constexpr int SMEM = 1024 + STAGES * STAGE + 1024 + TC2_STAGING;
 };
 
+// Tile `i` of tiles_m x tiles_n in bands of `band` row tiles: a band's tiles run column after
+// column (row tiles fastest) before the next band begins, so that the band's token rows stay in
+// L2 for all of its columns. Returns (row tile, column tile).
+__device__ __forceinline__ int2 banded_tile(int i, int tiles_m, int tiles_n, int band) {
+  const int b = i / (band * tiles_n), first = b * band;
+  const int rows = min(band, tiles_m - first), r = i - first * tiles_n;
+  return make_int2(first + r % rows, r / rows);
+}
+
 template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     void* __restrict__ C, int c_dtype, long long ldc, int M, int N, int K,
                     int kb_per_split, int mode_act, float* __restrict__ partial,
                     long long partial_stride, long long partial_ld, int tiles_m, int tiles_n,
-                    int num_tiles, int* __restrict__ error) {
+                    int band, int num_tiles, int* __restrict__ error) {
   const int mode = mode_act & 255, act = mode_act >> 8;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -543,9 +552,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       int s = 0;
       uint32_t ph = 0;
       for (int w = pair; w < num_tiles; w += pairs) {
-        const int rem = w % tiles_mn;
-        const int m0 = (rem % tiles_m) * 256 + (int)rank * 128;
-        const int n0 = (rem / tiles_m) * BN + (int)rank * (BN / 2);
+        const int2 mn = banded_tile(w % tiles_mn, tiles_m, tiles_n, band);
+        const int m0 = mn.x * 256 + (int)rank * 128;
+        const int n0 = mn.y * BN + (int)rank * (BN / 2);
         const int kb0 = (w / tiles_mn) * kb_per_split;
         const int nkb = min(kb_per_split, nkb_total - kb0);
         for (int i = 0; i < nkb; ++i) {
@@ -590,9 +599,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int lane_row = q * 32 + lane;
     int it = 0;
     for (int w = pair; w < num_tiles; w += pairs, ++it) {
-      const int rem = w % tiles_mn, z = w / tiles_mn;
-      const int n0 = (rem / tiles_m) * BN;
-      const int a = (rem % tiles_m) * 256 + (int)rank * 128 + lane_row;
+      const int z = w / tiles_mn;
+      const int2 mn = banded_tile(w % tiles_mn, tiles_m, tiles_n, band);
+      const int n0 = mn.y * BN;
+      const int a = mn.x * 256 + (int)rank * 128 + lane_row;
       const int b = it & 1;
       mbar_wait(acc_full0 + 8 * b, (it >> 1) & 1, error, 13);
       tc_fence_after_sync();
@@ -686,6 +696,20 @@ static cudaError_t mb_launch_pair(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// Row tiles of a band (see banded_tile): token rows of about 24 MB, a fifth of L2, beside which
+// the weight tiles of the moment and the output on its way out have room; all row tiles where
+// they are no more than twice that anyway. Without bands every column of tiles reads all token
+// rows from DRAM again once they no longer fit L2 (60,865 tokens, 4,096 x 1,024: 457 -> 360 us;
+// 16,384 tokens, 24,576 x 4,096: 2,361 -> 1,990 us); 16 and 32 MB measure alike, 64 MB loses it.
+static int pair_band(int tiles_m, int K) {
+  const long long tile_bytes = 256ll * K * 2, room = 24ll << 20;
+  if (tiles_m * tile_bytes <= 2 * room) return tiles_m;
+  long long most = room / tile_bytes;
+  if (most < 8) most = 8;
+  const int bands = (int)((tiles_m + most - 1) / most);
+  return (tiles_m + bands - 1) / bands;
+}
+
 template <int BN>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, int c_dtype,
                        long long ldc, int M, int N, int K, int kb_per_split, int mode,
@@ -702,9 +726,10 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, 
   }
   const int num_tiles = tiles_m * tiles_n * splits;
   const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
+  const int band = pair_band(tiles_m, K);
   mb_launch_pair(gemm_tc_pair_kernel<BN>, dim3(grid), dim3(TC_THREADS), Tc2Cfg<BN>::SMEM, s, tmA,
                  tmB, C, c_dtype, ldc, M, N, K, kb_per_split, mode, partial, (long long)M * N,
-                 (mode & 255) >= TC_SWIGLU ? limit_bits() : (long long)N, tiles_m, tiles_n,
+                 (mode & 255) >= TC_SWIGLU ? limit_bits() : (long long)N, tiles_m, tiles_n, band,
                  num_tiles, error);
   cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) MB_FAIL("mb_gemm_tc (pairs): %s", cudaGetErrorString(le));
@@ -726,6 +751,15 @@ static int pair_tile_width(int N, int tiles_m, int pairs) {
   return best;
 }
 
+// Whether K cut into `splits` pays where a kernel of its own adds the sums up: a tile's K step
+// takes (w + 40) * 1.4 ns; the sums are written, read and added into the output at about 10 TB/s
+// (they lie in L2), after 2 us for the kernel (measured with the products' sizes of 1,024 to
+// 5,120 columns and 160 to 4,096 tokens).
+static bool split_pays(int nkb, int splits, int width, long long outputs) {
+  const double saved = (nkb - (nkb + splits - 1) / splits) * (width + 40) * 1.4e-3;
+  return saved > 2.0 + outputs * 4.0 * (2 * splits + 2) / 1e7;
+}
+
 // C[M, N] = (or +=) the sum over the splits, added in split order
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits,
                                      long long stride, void* __restrict__ C, int c_dtype,
@@ -740,6 +774,61 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int spli
     const size_t r = i / N, c = i - r * N;
     store_out(C, c_dtype, r * ldc + c, v, mode);
   }
+}
+
+// The same four values a thread: N, ldc and the strides are multiples of 4 and everything lies on
+// 16-byte boundaries. blockIdx.y walks the rows, so no value's place costs a division.
+template <bool ADD, bool F32>
+__global__ void __launch_bounds__(256)
+splitk_reduce4_kernel(const float* __restrict__ partial, int splits, long long stride,
+                      void* __restrict__ C, long long ldc, int M, int N) {
+  mb_grid_wait();
+  mb_grid_launch_next();
+  const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (c >= N) return;
+  for (int r = blockIdx.y; r < M; r += gridDim.y) {
+    const float* p = partial + (size_t)r * N + c;
+    float4 v = *(const float4*)p;
+    for (int s = 1; s < splits; ++s) {
+      const float4 w = *(const float4*)(p + s * stride);
+      v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+    }
+    if (F32) {
+      float4* o = (float4*)((float*)C + r * ldc + c);
+      if (ADD) {
+        const float4 w = *o;
+        v.x = w.x + v.x; v.y = w.y + v.y; v.z = w.z + v.z; v.w = w.w + v.w;
+      }
+      *o = v;
+    } else {
+      __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      uint2 u;
+      u.x = *(uint32_t*)&lo;
+      u.y = *(uint32_t*)&hi;
+      *(uint2*)((__nv_bfloat16*)C + r * ldc + c) = u;
+    }
+  }
+}
+
+static int reduce_splits(const float* partial, int splits, void* C, int c_dtype, long long ldc,
+                         int M, int N, int epilogue, cudaStream_t s) {
+  const long long stride = (long long)M * N;
+  if (N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)partial & 15) == 0 && ((uintptr_t)C & 15) == 0 &&
+      (epilogue == TC_STORE || (epilogue == TC_ADD && c_dtype == MB_F32))) {
+    const dim3 grid((N / 4 + 255) / 256, M < 4096 ? M : 4096);
+#define GO(ADD_, F32_)                                                                          \
+  mb_launch(splitk_reduce4_kernel<ADD_, F32_>, grid, dim3(256), 0, s, partial, splits, stride, C, \
+            ldc, M, N)
+    if (epilogue == TC_ADD) GO(true, true);
+    else if (c_dtype == MB_F32) GO(false, true);
+    else GO(false, false);
+#undef GO
+  } else {
+    const long long blocks = (stride + 255) / 256;
+    mb_launch(splitk_reduce_kernel, dim3((unsigned)(blocks < 4096 ? blocks : 4096)), dim3(256), 0, s,
+              partial, splits, stride, C, c_dtype, ldc, M, N, epilogue);
+  }
+  MB_CHECK_LAUNCH("mb_gemm_tc reduce");
 }
 
 struct TcPlan {
@@ -859,10 +948,10 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     p.smem += 4 * 4096;  // the epilogue warps' staging rows
     const int tiles = ((rowsA + TC_BM - 1) / TC_BM) * ((rowsB + bn - 1) / bn);
     if (workspace && epilogue < TC_SWIGLU && tiles < sms && nkb >= 8) {
-      int want = (2 * sms + tiles - 1) / tiles;
-      // sums that stay pending are read once more by their consumer, a full pass over the
-      // output per split: then only as many splits as fill the device once
-      if (defer && want > sms / tiles) want = sms / tiles;
+      // as many splits as fill the device once: each more costs a second round and one more pass
+      // over the output by whoever adds the sums up (4,096 x 4,096, 128 tokens: 9 splits 14.6 us,
+      // 16 splits 21.6; 4,096 x 12,288: 30.7 and 35.0)
+      int want = sms / tiles;
       if (defer && want > TC_MAX_SPLITS) want = TC_MAX_SPLITS;
       if (want > nkb / 4) want = nkb / 4;
       const long long per = (long long)M * N;
@@ -882,12 +971,16 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     const int tiles = tiles_m * tiles_n;
     p.splits = 1;
     if (workspace && epilogue < TC_SWIGLU && tiles < pairs && nkb >= 8) {
-      int want = (2 * pairs + tiles - 1) / tiles;
-      if (defer && want > pairs / tiles) want = pairs / tiles;   // as above
+      // as many splits as fill the pairs once: more give a second round and their sums one more
+      // pass over the output each (4,096 x 12,288, 1,024 tokens: none 77 us, 3 splits 108; 2,048 x
+      // 2,048, 2,048 tokens: none 23, 3 splits 48; 4,096 x 12,288, 160 tokens: none 46, 2 splits 30)
+      int want = pairs / tiles;
       if (defer && want > TC_MAX_SPLITS) want = TC_MAX_SPLITS;
       if (want > nkb / 4) want = nkb / 4;
       const long long per = (long long)M * N;
       if (want > workspace_floats / per) want = (int)(workspace_floats / per);
+      // sums added up here: only where that costs less than the shorter K loops save
+      while (!defer && want > 1 && !split_pays(nkb, want, bn, per)) --want;
       if (want > 1) p.splits = want;
     }
     p.kb_per_split = (nkb + p.splits - 1) / p.splits;
@@ -912,13 +1005,8 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     if (rc) return rc;
     g_last_launches = (p.splits > 1 && !defer) ? 2 : 1;
     g_last_splits = p.splits;
-    if (p.splits > 1 && !defer) {
-      const size_t total = (size_t)M * N;
-      const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-      mb_launch(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, s, workspace, p.splits,
-                (long long)M * N, C, c_dtype, (long long)ldc, M, N, epilogue);
-      MB_CHECK_LAUNCH("mb_gemm_tc reduce");
-    }
+    if (p.splits > 1 && !defer)
+      return reduce_splits(workspace, p.splits, C, c_dtype, ldc, M, N, epilogue, s);
     return 0;
   }
   CUtensorMap tmA, tmB;
@@ -945,13 +1033,8 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
   if (rc) return rc;
   g_last_launches = (p.splits > 1 && !defer) ? 2 : 1;
   g_last_splits = p.splits;
-  if (p.splits > 1 && !defer) {
-    const size_t total = (size_t)M * N;
-    const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-    mb_launch(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, s, workspace, p.splits, pstride, C, c_dtype, ldc, M,
-                                                N, epilogue);
-    MB_CHECK_LAUNCH("mb_gemm_tc reduce");
-  }
+  if (p.splits > 1 && !defer)
+    return reduce_splits(workspace, p.splits, C, c_dtype, ldc, M, N, epilogue, s);
   return 0;
 }
 
