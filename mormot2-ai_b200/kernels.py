@@ -6,6 +6,7 @@ PyTorch, and nothing falls back: without a GPU or the compiled libraries it rais
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -45,6 +46,16 @@ def _stream() -> int:
     if _raw_stream is not None:                     # the short way (no Stream object)
         return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+@functools.lru_cache(maxsize=None)
+def _sms_of(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+def _sms() -> int:
+    """How many multiprocessors the current device has."""
+    return _sms_of(torch.cuda.current_device())
 
 
 def require_gpu() -> None:
@@ -1246,13 +1257,14 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, step, line
     assert gate is None or gate.dtype == out.dtype
     assert keep_first == 0 or line.ring_pages == 0
     _call("attention_simt", "mb_attention_simt",
-          [_vp, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f,
-           _i, _vp, _f, _vp, _i, _i, _vp, _i, _vp],
+          [_vp, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
+           _i, _f, _i, _vp, _f, _vp, _i, _i, _vp, _i, _i, _vp],
           _ptr(q), q_stride, _ptr(out), out.stride(0), _ptr(line.k), _ptr(line.v),
           code_of(out.dtype), _ptr(line.page_table), line.max_pages, line.ring_pages,
-          _ptr(step.tok_seq), _ptr(step.tok_pos), _ptr(step.seq_slot), T, nh, nkv, hd,
+          _ptr(step.tok_seq), _ptr(step.tok_pos), _ptr(step.seq_slot), _ptr(step.seq_start), step.B,
+          step.max_new, T, nh, nkv, hd,
           window, float(scale), vd or hd, _ptr(sink), float(softcap), _ptr(gate), gate_stride,
-          int(gate_dim), _ptr(slopes), int(keep_first), _stream())
+          int(gate_dim), _ptr(slopes), int(keep_first), _sms(), _stream())
 
 
 # ------------------------------------------------------------------------------ sampling
