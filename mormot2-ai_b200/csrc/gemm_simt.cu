@@ -8,7 +8,11 @@
 // Epilogues: store; add into a float32 residual; SwiGLU over a weight [2N, K] (out =
 // silu(gate) * up) whose rows are either [0, N) gate and [N, 2N) up, or alternate gate, up,
 // gate, up ... (the layout that the tensor-core kernel's fused epilogue uses).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 MB_DEFINE_LAST_ERROR
 
@@ -29,19 +33,20 @@ __device__ __forceinline__ void put_out(void* C, int c_bf16, size_t at, float v,
   }
 }
 
-template <typename TA, typename TW, int EPI>
+// SwiGLU over a weight whose gate rows come first and whose up rows follow, for more rows of A than
+// gemm_few_rows_kernel takes: 64 x 64 outputs a block, two sums each.
+template <typename TA, typename TW>
 __global__ void __launch_bounds__(256)
-gemm_simt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, void* __restrict__ C,
-                 int c_bf16, int ldc, int M, int N, int K) {
-  constexpr int NW = (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_PAIRS) ? 2 : 1;
+gemm_swiglu_halves_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
+                          void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K) {
   __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[NW][BK][BN + 4];
+  __shared__ float Ws[2][BK][BN + 4];
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int tr = (tid / 16) * 4, tc = (tid % 16) * 4;
-  float acc[NW][4][4];
+  float acc[2][4][4];
 #pragma unroll
-  for (int w = 0; w < NW; ++w)
+  for (int w = 0; w < 2; ++w)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -57,11 +62,8 @@ gemm_simt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, vo
       As[c][r] = (gm < M && gk < K) ? to_f32<TA>(A[(size_t)gm * lda + gk]) : 0.f;
       const int gn = n0 + r;
 #pragma unroll
-      for (int w = 0; w < NW; ++w)
-        Ws[w][c][r] = (gn < N && gk < K)
-                          ? to_f32<TW>(W[(EPI == EPI_SWIGLU_PAIRS ? (size_t)gn * 2 + w
-                                                                   : (size_t)w * N + gn) * K + gk])
-                          : 0.f;
+      for (int w = 0; w < 2; ++w)
+        Ws[w][c][r] = (gn < N && gk < K) ? to_f32<TW>(W[((size_t)w * N + gn) * K + gk]) : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -70,7 +72,7 @@ gemm_simt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, vo
 #pragma unroll
       for (int i = 0; i < 4; ++i) a[i] = As[k][tr + i];
 #pragma unroll
-      for (int w = 0; w < NW; ++w) {
+      for (int w = 0; w < 2; ++w) {
         float b[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) b[j] = Ws[w][k][tc + j];
@@ -90,22 +92,21 @@ gemm_simt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, vo
     for (int j = 0; j < 4; ++j) {
       const int gn = n0 + tc + j;
       if (gn >= N) continue;
-      const size_t at = (size_t)gm * ldc + gn;
-      if (EPI == EPI_STORE || EPI == EPI_ADD) {
-        put_out(C, c_bf16, at, acc[0][i][j], EPI == EPI_ADD);
-      } else {
-        const float g = acc[0][i][j];
-        put_out(C, c_bf16, at, g / (1.0f + expf(-g)) * acc[NW - 1][i][j], false);
-      }
+      const float g = acc[0][i][j];
+      put_out(C, c_bf16, (size_t)gm * ldc + gn, g / (1.0f + expf(-g)) * acc[1][i][j], false);
     }
   }
 }
 
 // ---------------------------------------------------------------------------- few rows
-// The same product for at most 16 rows of A (a decode step): the weight streams through once.
-// A warp owns four weight rows (four output features, or two with their gate and up rows) and
-// walks K in chunks of 128 (every lane 4 consecutive values of each of its rows, 16 bytes of
-// float32), against up to eight rows of A at a time; 32 sums a warp, reduced by shuffles.
+// The same product for at most 16 rows of A (a decode step): the weight streams through once, and
+// its bytes are what bounds it. A warp owns four weight rows (four output features, or two with
+// their gate and up rows) and walks K in chunks of 128 (every lane 4 consecutive values of each of
+// its rows, 16 bytes of float32, the next chunk's asked for before this one is multiplied), against
+// up to eight rows of A at a time. Its 32 sums are reduced by halves, a value a lane at the end. A
+// weight with few rows has KW warps of a block share each four rows along K, so that enough warps
+// ask for it: 1,024 x 3,072 with 8 rows of A, float32: 51 -> 7.8 us; 151,936 x
+// 1,024: 193 -> 147 us (4.2 TB/s).
 // a weight row's values are used once: they pass by the L1 cache, which keeps the rows of A
 template <typename T> __device__ __forceinline__ float4 load4_once(const T* p);
 template <> __device__ __forceinline__ float4 load4_once<float>(const float* p) {
@@ -128,16 +129,30 @@ template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __
 #define FEW_ROWS 8   // rows of A in one pass
 #define FEW_MAX 16   // the most rows that take this kernel
 
+// v[i] summed over the warp's lanes, value i's sum in lane i: every round halves what a lane keeps.
+__device__ __forceinline__ float sum32_by_lane(float* v, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+
 template <typename TA, typename TW, int EPI>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
-                     void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K) {
+                     void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K, int KW) {
   constexpr bool GLU = EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_PAIRS;
   constexpr int FEATS = GLU ? 2 : 4;  // output features of a warp
+  __shared__ float part[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * 8 + warp) * FEATS;
-  if (n0 >= N) return;
-  // the warp's four weight rows; a row beyond the weight is read as row n0's and not stored
+  const int n0 = (blockIdx.x * (8 / KW) + warp / KW) * FEATS, kw = warp % KW;
+  // the warp's four weight rows; a row beyond the weight is read as its last and not stored
   const TW* wr[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -147,58 +162,79 @@ gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
     else row = min(n0 + j, N - 1);
     wr[j] = W + (size_t)row * K;
   }
-  for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
-    float acc[4][FEW_ROWS];
+  const int k_first = kw * 128 + lane * 4, k_step = KW * 128;
+  float4 next[4];
+  auto ask = [&](int k) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
+      next[j] = k < K ? load4_once<TW>(wr[j] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  ask(k_first);      // weights depend on no earlier kernel
+  mb_grid_wait();
+  mb_grid_launch_next();
+  for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
+    float acc[4 * FEW_ROWS];
 #pragma unroll
-      for (int m = 0; m < FEW_ROWS; ++m) acc[j][m] = 0.f;
-    for (int k = lane * 4; k < K; k += 128) {
+    for (int j = 0; j < 4 * FEW_ROWS; ++j) acc[j] = 0.f;
+    if (m0) ask(k_first);
+    for (int k = k_first; k < K; k += k_step) {
       float4 w[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = load4_once<TW>(wr[j] + k);
+      for (int j = 0; j < 4; ++j) w[j] = next[j];
+      ask(k + k_step);
 #pragma unroll
       for (int m = 0; m < FEW_ROWS; ++m) {
         if (m0 + m >= M) break;  // uniform over the warp
         const float4 a = load4<TA>(A + (size_t)(m0 + m) * lda + k);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[j][m] = fmaf(a.x, w[j].x, fmaf(a.y, w[j].y, fmaf(a.z, w[j].z, fmaf(a.w, w[j].w, acc[j][m]))));
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int m = 0; m < FEW_ROWS; ++m) acc[j][m] = warp_sum(acc[j][m]);
-    // lane m stores row m0 + m
-#pragma unroll
-    for (int m = 0; m < FEW_ROWS; ++m) {
-      if (lane != m || m0 + m >= M) continue;
-#pragma unroll
-      for (int f = 0; f < FEATS; ++f) {
-        if (n0 + f >= N) continue;
-        const size_t at = (size_t)(m0 + m) * ldc + n0 + f;
-        if (EPI == EPI_STORE || EPI == EPI_ADD) {
-          put_out(C, c_bf16, at, acc[f][m], EPI == EPI_ADD);
-        } else {
-          const float g = EPI == EPI_SWIGLU ? acc[f][m] : acc[2 * f][m];
-          const float u = EPI == EPI_SWIGLU ? acc[2 + f][m] : acc[2 * f + 1][m];
-          put_out(C, c_bf16, at, g / (1.0f + expf(-g)) * u, false);
+        for (int j = 0; j < 4; ++j) {
+          float& s = acc[j * FEW_ROWS + m];
+          s = fmaf(a.x, w[j].x, fmaf(a.y, w[j].y, fmaf(a.z, w[j].z, fmaf(a.w, w[j].w, s))));
         }
       }
     }
+    float v = sum32_by_lane(acc, lane);      // lane 8 j + m: weight row j, row m0 + m of A
+    if (KW > 1) {
+      __syncthreads();      // the sums of the rows of A before have been read
+      part[warp][lane] = v;
+      __syncthreads();
+      if (kw == 0)
+        for (int i = 1; i < KW; ++i) v += part[warp + i][lane];
+    }
+    const int j = lane >> 3, m = m0 + (lane & 7);
+    const float up = GLU ? __shfl_sync(0xffffffffu, v, (lane + (EPI == EPI_SWIGLU ? 16 : 8)) & 31) : 0.f;
+    if (kw != 0 || m >= M) continue;
+    int f = j;
+    if (EPI == EPI_SWIGLU_PAIRS) {
+      if (j & 1) continue;
+      f = j >> 1;
+    }
+    if (EPI == EPI_SWIGLU && j >= 2) continue;
+    if (n0 + f >= N) continue;
+    const float out = GLU ? v / (1.0f + expf(-v)) * up : v;
+    put_out(C, c_bf16, (size_t)m * ldc + n0 + f, out, EPI == EPI_ADD);
   }
 }
 
 // ---------------------------------------------------------------------------- many rows
-// The same product for many rows: 128 x 128 tiles, 8 x 8 results a thread (two 4 x 4 quarters
-// 64 apart in each direction, so that the shared-memory reads are 16 bytes wide and free of
-// bank conflicts), K in steps of 16 through two buffers with the next step's global loads under
-// way while this one is multiplied. Epilogues: store, residual add, and SwiGLU over weight rows
-// that alternate gate and up (NW = 2 N weight rows, neighbouring columns of the tile pair up).
-#define LM 128
+// The same product for many rows, bound by float32 multiply-adds and, close behind, by reads of
+// shared memory: a 16-byte read of a warp takes four cycles whatever its lanes share, so a thread
+// has 16 x 8 results (six reads per 128 multiply-adds; 8 x 8 would need as many cycles for the one
+// as for the other). Multiply-adds go two rows an instruction (`fma.rn.f32x2`, each half rounded
+// like a single one), which leaves issue slots for the reads. Blocks are small (64 threads, 64 x
+// 128 results, four to a multiprocessor), K goes in steps of 8 through two buffers with the next
+// step's global loads under way; where tiles are few or would leave a last round half empty, K is
+// dealt out over a cluster whose CTAs add their sums up through shared memory, in K's order.
+// Epilogues: store, residual add, and SwiGLU over weight rows that alternate gate and up (NW = 2 N
+// weight rows, neighbouring columns pair up). 1,728 rows, 6,144 x 1,024 (SwiGLU): 639 us
+// with 128 x 128 tiles, 8 x 8 results a thread -> 519 (42 TFLOP/s); 1,024 x 2,048: 247 -> 216,
+// with 400 rows 246 -> 68. Lanes of a row-wise load that stand in 32 rows cost a tenth of it: a
+// row's LK values lie with neighbouring lanes.
+#define LM 64
 #define LN 128
-#define LK 16
+#define LK 8
+#define LMP (LM + 4)
+#define LNP (LN + 4)
 
 // four values k .. k + 3 of a row as float32, zeros beyond K or for a row that does not exist
 template <typename T>
@@ -214,86 +250,150 @@ __device__ __forceinline__ float4 row_piece(const T* __restrict__ base, bool row
   return v;
 }
 
+__device__ __forceinline__ void fma_pair(unsigned long long& s, unsigned long long a,
+                                         unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long twice(float v) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+
 template <typename TA, typename TW, int EPI>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(64, 4)
 gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
                       void* __restrict__ C, int c_bf16, int ldc, int M, int NW, int K, int vec_a,
-                      int vec_w) {
-  __shared__ __align__(16) float As[2][LK][LM + 4];
-  __shared__ __align__(16) float Ws[2][LK][LN + 4];
+                      int vec_w, int splits, int k_split) {
+  // [buffer][K step][rows of A | rows of W]; a split's sums [LM][LN] reuse it
+  extern __shared__ __align__(16) float sm[];
+  constexpr int BUF = LK * (LMP + LNP);
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * LM, n0 = blockIdx.x * LN;
-  // loads: thread t brings values 8 (t % 2) .. + 7 of row t / 2 of both tiles
-  const int lr = tid >> 1, lk = (tid & 1) * 8;
-  const bool a_ok = m0 + lr < M, w_ok = n0 + lr < NW;
-  const TA* arow = A + (size_t)(m0 + lr) * lda;
-  const TW* wrow = W + (size_t)(n0 + lr) * K;
+  const int split = blockIdx.x % splits;
+  const int m0 = blockIdx.y * LM, n0 = (blockIdx.x / splits) * LN;
+  const int k_lo = split * k_split, k_hi = min(K, k_lo + k_split);
+  // loads: a row's LK values lie with LK / 4 neighbouring lanes; a pass brings RP rows
+  constexpr int PER = LK / 4, RP = 64 / PER, PA = LM / RP, PW = LN / RP;
+  const int lr = tid / PER, lk = 4 * (tid % PER);
   const int ty = tid >> 4, tx = tid & 15;
-  float acc[8][8];
+  // rows 16 g + 4 ty + (0 .. 3), two a pair; columns 64 h + 4 tx + (0 .. 3)
+  unsigned long long acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+  mb_grid_wait();
+  mb_grid_launch_next();
 
-  float4 ra[2], rw[2];
+  float4 r[PA + PW];
   auto fetch = [&](int k) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      ra[h] = row_piece<TA>(arow, a_ok, k + lk + 4 * h, K, vec_a);
-      rw[h] = row_piece<TW>(wrow, w_ok, k + lk + 4 * h, K, vec_w);
+    for (int i = 0; i < PA; ++i) {
+      const int m = m0 + lr + RP * i;
+      r[i] = row_piece<TA>(A + (size_t)m * lda, m < M, k + lk, k_hi, vec_a);
+    }
+#pragma unroll
+    for (int i = 0; i < PW; ++i) {
+      const int n = n0 + lr + RP * i;
+      r[PA + i] = row_piece<TW>(W + (size_t)n * K, n < NW, k + lk, k_hi, vec_w);
     }
   };
-  auto put = [&](int buf) {
+  auto put = [&](float* buf) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = lk + 4 * h;
-      As[buf][k][lr] = ra[h].x; As[buf][k + 1][lr] = ra[h].y;
-      As[buf][k + 2][lr] = ra[h].z; As[buf][k + 3][lr] = ra[h].w;
-      Ws[buf][k][lr] = rw[h].x; Ws[buf][k + 1][lr] = rw[h].y;
-      Ws[buf][k + 2][lr] = rw[h].z; Ws[buf][k + 3][lr] = rw[h].w;
+    for (int i = 0; i < PA + PW; ++i) {
+      const int pitch = i < PA ? LMP : LNP;
+      float* d = buf + (i < PA ? RP * i : LK * LMP + RP * (i - PA)) + lr + lk * pitch;
+      d[0] = r[i].x;
+      d[pitch] = r[i].y;
+      d[2 * pitch] = r[i].z;
+      d[3 * pitch] = r[i].w;
     }
   };
   int cur = 0;
-  fetch(0);
-  put(0);
+  fetch(k_lo);
+  put(sm);
   __syncthreads();
-  for (int k0 = 0; k0 < K; k0 += LK) {
-    const bool more = k0 + LK < K;
+  for (int k0 = k_lo; k0 < k_hi; k0 += LK) {
+    const bool more = k0 + LK < k_hi;
     if (more) fetch(k0 + LK);
+    const float* as = sm + cur * BUF + 4 * ty;
+    const float* ws = sm + cur * BUF + LK * LMP + 4 * tx;
 #pragma unroll
     for (int k = 0; k < LK; ++k) {
-      const float4 a0 = *(const float4*)&As[cur][k][ty * 4], a1 = *(const float4*)&As[cur][k][64 + ty * 4];
-      const float4 b0 = *(const float4*)&Ws[cur][k][tx * 4], b1 = *(const float4*)&Ws[cur][k][64 + tx * 4];
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      ulonglong2 a[4];
+      float4 b[2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int g = 0; g < 4; ++g) a[g] = *(const ulonglong2*)(as + k * LMP + 16 * g);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      for (int h = 0; h < 2; ++h) b[h] = *(const float4*)(ws + k * LNP + 64 * h);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 bq = b[j >> 2];
+        const unsigned long long bb = twice((j & 3) == 0 ? bq.x : ((j & 3) == 1 ? bq.y : ((j & 3) == 2 ? bq.z : bq.w)));
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          fma_pair(acc[2 * g][j], a[g].x, bb);
+          fma_pair(acc[2 * g + 1][j], a[g].y, bb);
+        }
+      }
     }
     if (more) {
-      put(cur ^ 1);
+      put(sm + (cur ^ 1) * BUF);
       __syncthreads();
       cur ^= 1;
     }
   }
+  auto half = [](unsigned long long v, int h) { return __uint_as_float((unsigned)(v >> (32 * h))); };
+  // four neighbouring columns of a row
+  auto finish = [&](int gm, int gn, float4 v) {
+    if (gm >= M) return;
+    const float c[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + (i >> 2) * 64 + ty * 4 + (i & 3);
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j >> 2) * 64 + tx * 4 + (j & 3);
-      if (gn >= NW) continue;
+    for (int j = 0; j < 4; ++j) {
+      if (gn + j >= NW) return;
       if (EPI == EPI_SWIGLU_PAIRS) {
-        if (j & 1) continue;  // gate at the even weight row, up at the odd one after it
-        const float g = acc[i][j];
-        put_out(C, c_bf16, (size_t)gm * ldc + (gn >> 1), g / (1.0f + expf(-g)) * acc[i][j + 1], false);
+        // gate at the even weight row, up at the odd one after it
+        if (!(j & 1))
+          put_out(C, c_bf16, (size_t)gm * ldc + ((gn + j) >> 1), c[j] / (1.0f + expf(-c[j])) * c[j + 1], false);
       } else {
-        put_out(C, c_bf16, (size_t)gm * ldc + gn, acc[i][j], EPI == EPI_ADD);
+        put_out(C, c_bf16, (size_t)gm * ldc + gn + j, c[j], EPI == EPI_ADD);
       }
     }
+  };
+  if (splits > 1) __syncthreads();      // the last step's reads are done
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int row = 16 * (i >> 2) + 4 * ty + (i & 3);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const unsigned long long* p = acc[i >> 1] + 4 * h;
+      const float4 v = make_float4(half(p[0], i & 1), half(p[1], i & 1), half(p[2], i & 1), half(p[3], i & 1));
+      if (splits == 1) finish(m0 + row, n0 + 64 * h + 4 * tx, v);
+      else *(float4*)(sm + row * LN + 64 * h + 4 * tx) = v;
+    }
   }
+  if (splits == 1) return;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  for (int e = 4 * (split * 64 + tid); e < LM * LN; e += 4 * 64 * splits) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < splits; ++k) {
+      const float4 o = *(const float4*)(cluster.map_shared_rank(sm, k) + e);
+      v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+    }
+    finish(m0 + e / LN, n0 + e % LN, v);
+  }
+  cluster.sync();      // nobody leaves while its sums are still read
+}
+
+static int sm_count() {
+  static const int n = [] {
+    int device = 0, count = 148;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+    return count;
+  }();
+  return n;
 }
 
 template <typename TA, typename TW>
@@ -304,10 +404,15 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
   if (M <= FEW_MAX && K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A & a_align) == 0 &&
       ((uintptr_t)W & w_align) == 0) {
     const int feats = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_PAIRS) ? 2 : 4;
-    const int blocks = (N + 8 * feats - 1) / (8 * feats);
+    const int groups = (N + feats - 1) / feats;
+    // warps that share a group's K: until some 3,000 warps ask for the weight (8 rows of A;
+    // 1,024 x 2,048: 39 us with one, 6 with eight), at least 128 values of K each
+    int kw = 1;
+    while (kw < 8 && groups * kw < 3000 && kw * 128 < K) kw *= 2;
+    const int blocks = (groups + 8 / kw - 1) / (8 / kw);
 #define FEW(E)                                                                                \
-  gemm_few_rows_kernel<TA, TW, E><<<blocks, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, C,  \
-                                                         c_bf16, ldc, M, N, K)
+  mb_launch(gemm_few_rows_kernel<TA, TW, E>, dim3(blocks), dim3(256), 0, s, (const TA*)A, lda, \
+            (const TW*)W, C, c_bf16, ldc, M, N, K, kw)
     if (epi == EPI_STORE) FEW(EPI_STORE);
     else if (epi == EPI_ADD) FEW(EPI_ADD);
     else if (epi == EPI_SWIGLU) FEW(EPI_SWIGLU);
@@ -315,15 +420,30 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
 #undef FEW
     MB_CHECK_LAUNCH("mb_gemm_simt");
   }
-  if (M >= 64 && epi != EPI_SWIGLU) {
+  if (epi != EPI_SWIGLU) {
     const int NW = epi == EPI_SWIGLU_PAIRS ? 2 * N : N;
-    dim3 big((NW + LN - 1) / LN, (M + LM - 1) / LM);
-    if (big.y > 65535) MB_FAIL("mb_gemm_simt: %d rows are too many for one launch", M);
+    const int tiles_n = (NW + LN - 1) / LN, tiles_m = (M + LM - 1) / LM;
+    if (tiles_m > 65535) MB_FAIL("mb_gemm_simt: %d rows are too many for one launch", M);
     const int vec_a = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A & a_align) == 0;
     const int vec_w = K % 4 == 0 && ((uintptr_t)W & w_align) == 0;
+    // splits of K, at least 128 values each: what a multiprocessor has to do in units of one whole
+    // tile, where fewer than three CTAs take as long as three
+    const int tiles = tiles_n * tiles_m, sms = sm_count();
+    int splits = 1;
+    double best = 1e30;
+    for (int n = 1; n <= 8 && (n == 1 || K >= 128 * n); ++n) {
+      const int each = (int)(((long long)tiles * n + sms - 1) / sms);
+      const double cost = (double)(each < 3 ? 3 : each) / n + 0.02 * n;
+      if (cost < best) { best = cost; splits = n; }
+    }
+    const int k_split = ((K + splits - 1) / splits + LK - 1) / LK * LK;
+    splits = (K + k_split - 1) / k_split;
+    const size_t buffers = 2 * LK * (LMP + LNP) * sizeof(float), sums = LM * LN * sizeof(float);
+    const size_t smem = splits > 1 && sums > buffers ? sums : buffers;
 #define MANY(E)                                                                               \
-  gemm_many_rows_kernel<TA, TW, E><<<big, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, C,    \
-                                                       c_bf16, ldc, M, NW, K, vec_a, vec_w)
+  mb_launch_clusters(gemm_many_rows_kernel<TA, TW, E>, dim3(tiles_n * splits, tiles_m), dim3(64), smem, s, \
+                     splits, (const TA*)A, lda, (const TW*)W, C, c_bf16, ldc, M, NW, K, vec_a, \
+                     vec_w, splits, k_split)
     if (epi == EPI_STORE) MANY(EPI_STORE);
     else if (epi == EPI_ADD) MANY(EPI_ADD);
     else MANY(EPI_SWIGLU_PAIRS);
@@ -332,14 +452,8 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
   }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) MB_FAIL("mb_gemm_simt: %d rows are too many for one launch", M);
-#define GO(E)                                                                                  \
-  gemm_simt_kernel<TA, TW, E><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, C, c_bf16,  \
-                                                   ldc, M, N, K)
-  if (epi == EPI_STORE) GO(EPI_STORE);
-  else if (epi == EPI_ADD) GO(EPI_ADD);
-  else if (epi == EPI_SWIGLU) GO(EPI_SWIGLU);
-  else GO(EPI_SWIGLU_PAIRS);
-#undef GO
+  gemm_swiglu_halves_kernel<TA, TW><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TW*)W, C, c_bf16,
+                                                         ldc, M, N, K);
   MB_CHECK_LAUNCH("mb_gemm_simt");
 }
 

@@ -1,0 +1,42 @@
+"""The float32 products' forms at their edges: rows up to 16 (warps that share a weight row's K)
+and more (tiles of 64 x 128, K dealt out over a cluster). Small whole numbers make every sum
+exact, so the results must equal the oracle's bit for bit; SwiGLU is compared in float64."""
+import pytest
+import torch
+
+from mormot2_ai_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def whole(shape, seed, most=3):
+    gen = torch.Generator().manual_seed(seed)
+    return torch.randint(-most, most + 1, shape, generator=gen).float().to(DEV)
+
+
+# K = 1030 and 37 leave no whole pieces of four values, 132 a ragged last step, 2,048 splits
+@pytest.mark.parametrize("M", [1, 9, 16, 17, 64, 65, 200])
+@pytest.mark.parametrize("N, Kd", [(3, 37), (130, 132), (96, 1030), (1024, 2048), (260, 4096)])
+def test_store_and_add(M, N, Kd):
+    a, w, c = whole((M, Kd), 1), whole((N, Kd), 2), whole((M, N), 3, 50)
+    exact = a @ w.t()
+    out = torch.empty((M, N), device=DEV)
+    K.gemm_simt(a, w, out)
+    assert torch.equal(out, exact)
+    K.gemm_simt(a, w, c_add := c.clone(), K.EPI_ADD)
+    assert torch.equal(c_add, c + exact)
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 70])
+@pytest.mark.parametrize("N, Kd", [(5, 40), (65, 132), (512, 2048)])
+@pytest.mark.parametrize("pairs", [True, False])
+def test_swiglu(M, N, Kd, pairs):
+    a, w = whole((M, Kd), 4) * 0.05, whole((2 * N, Kd), 5) * 0.25
+    z = a.double() @ w.double().t()
+    g, u = (z[:, 0::2], z[:, 1::2]) if pairs else (z[:, :N], z[:, N:])
+    want = torch.nn.functional.silu(g) * u
+    out = torch.empty((M, N), device=DEV)
+    K.gemm_simt(a, w, out, K.EPI_SWIGLU_PAIRS if pairs else K.EPI_SWIGLU)
+    # float32 sums of up to 2,048 terms: the error grows with their root
+    assert (out.double() - want).norm() <= 5e-6 * want.norm()
