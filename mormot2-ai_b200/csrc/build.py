@@ -56,6 +56,7 @@ SOURCES = {
     "norm_step": "norm_step.cu",
     "recurrent": "recurrent.cu",
     "linear_state": "linear_state.cu",
+    "state_walk": "state_walk.cu",
     "attention_diff": "attention_diff.cu",
     "attention_diff_tc": "attention_diff_tc.cu",
 }

@@ -97,7 +97,7 @@ CLASS_OF = {"mb_gemm_tc": "products", "mb_gemm_simt": "products",
             "mb_norm_add": "norms", "mb_cast_rows": "norms", "mb_norm_step": "norms",
             "mb_unary_act": "activation", "mb_softcap": "activation",
             "mb_pass_input": "embedding", "mb_wide_qk_norm": "rotary", "mb_rope_store": "rotary",
-            "mb_short_conv": "recurrence", "mb_linear_state_scan": "recurrence"}
+            "mb_short_conv": "recurrence", "mb_state_walk": "recurrence", "mb_linear_state_scan": "recurrence"}
 
 
 class Timing:
@@ -633,6 +633,42 @@ def tanh_rows(x: torch.Tensor, out: torch.Tensor) -> None:
           _ptr(out), code_of(out.dtype), x.shape[0], x.shape[1], _stream())
 
 
+class _WalkArgs(_c.Structure):
+    """``WalkArgs`` of csrc/state_walk.cu."""
+    _fields_ = ([(n, _vp) for n in ("q", "k", "v", "a", "s0", "s1", "gate", "abias", "u", "p0", "p1",
+                                    "normw", "state", "seq_start", "seq_slot", "h", "out", "raw")]
+                + [(n, _ll) for n in ("state_stride", "state_off", "head_stride")]
+                + [(n, _i) for n in ("ldq", "ldk", "ldv", "lda", "lds", "ldg", "group", "mode",
+                                     "gate_kind", "norm_stride", "T", "B", "H", "D", "DV", "W",
+                                     "out_bf16", "h_bf16", "vec")]
+                + [(n, _f) for n in ("q_scale", "inv_tau", "unit_eps", "cap", "eps")])
+
+
+WALK_GLA, WALK_DELTA, WALK_MLSTM, WALK_WKV = 0, 1, 2, 3
+# new tokens of a step's longest sequence from which on the recurrences go four tokens at a time
+WALK_TOKENS = 16
+
+
+def walks_by_fours(step, dim: int) -> bool:
+    """Whether a step goes through csrc/state_walk.cu: with fewer tokens a sequence its chunks of
+    16 are mostly empty and the walk token by token is as quick."""
+    return step.max_new >= WALK_TOKENS and dim <= 256
+
+
+def _at(t: torch.Tensor, col: int) -> int:
+    """The address of column ``col`` of a float32 tensor whose rows are dense."""
+    return _ptr(t) + 4 * int(col)
+
+
+def _state_walk(step, state, out, heads, dim, vdim, raw, **args) -> None:
+    a = _WalkArgs(state=_ptr(state), state_stride=state.stride(0), seq_start=_ptr(step.seq_start),
+                  seq_slot=_ptr(step.seq_slot), out=_ptr(out), raw=_ptr(raw), T=out.shape[0],
+                  B=step.B, H=heads, D=dim, DV=vdim, out_bf16=int(out.dtype == torch.bfloat16),
+                  group=args.pop("group", 1), **args)
+    _call("state_walk", "mb_state_walk", [_c.POINTER(_WalkArgs), _i, _vp], _c.byref(a), _sms(),
+          _stream(), launches=2)
+
+
 def wkv_scan(r, k, v, lw, g, w0, u, normw, eps: float, state: torch.Tensor,
              h: torch.Tensor, step, out: torch.Tensor, heads: int, dim: int) -> None:
     """The decaying matrix state, token after token (csrc/recurrent.cu). r, k, v, lw, g:
@@ -651,6 +687,13 @@ def wkv_scan(r, k, v, lw, g, w0, u, normw, eps: float, state: torch.Tensor,
     # where a step has few (sequence, head) pairs a head's columns are dealt over several
     # blocks, which leave their outputs here for the kernel that norms and gates them
     raw = torch.empty((T, heads * dim), dtype=torch.float32, device=out.device)
+    if walks_by_fours(step, dim):
+        _state_walk(step, state, out, heads, dim, dim, raw, mode=WALK_WKV, q=_ptr(r), k=_ptr(k),
+                    v=_ptr(v), a=_ptr(lw), gate=_ptr(g), ldq=ld, ldk=ld, ldv=ld, lda=ld, ldg=ld,
+                    abias=_ptr(w0), u=_ptr(u), normw=_ptr(normw), norm_stride=dim, eps=float(eps),
+                    q_scale=1.0, state_off=h.shape[1], head_stride=dim * dim, h=_ptr(h),
+                    h_bf16=int(h.dtype == torch.bfloat16), W=h.shape[1])
+        return
     _call("recurrent", "mb_wkv_scan",
           [_vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _f, _vp, _ll, _ll, _vp, _i, _i, _vp, _vp,
            _vp, _vp, _i, _i, _i, _i, _vp],
@@ -676,6 +719,17 @@ def mlstm_scan(z: torch.Tensor, cols, bi, bf, cap: float, q_scale: float, normw,
     _contig(out, "out")
     assert out.shape == (T, heads * vdim) and state.dtype == torch.float32
     assert state.stride(1) == 1 and state.shape[1] >= heads * (dim * vdim + dim + 1)
+    if walks_by_fours(step, dim):
+        # the outputs, their denominators and the running maxima after the step
+        raw = torch.empty((T * heads * (vdim + 1) + step.B * heads,), dtype=torch.float32,
+                          device=out.device)
+        ld, at = z.stride(0), lambda i: _at(z, cols[i])
+        _state_walk(step, state, out, heads, dim, vdim, raw, mode=WALK_MLSTM, q=at(0), k=at(1),
+                    v=at(2), gate=at(3), s0=at(4), s1=at(5), ldq=ld, ldk=ld, ldv=ld, lds=ld, ldg=ld,
+                    p0=_ptr(bi), p1=_ptr(bf), cap=float(cap), normw=_ptr(normw), norm_stride=vdim,
+                    eps=float(eps), q_scale=float(q_scale), gate_kind=1,
+                    head_stride=dim * vdim + dim + 1)
+        return
     raw = torch.empty((T, heads * vdim), dtype=torch.float32, device=out.device)   # as in wkv_scan
     _call("recurrent", "mb_mlstm_scan",
           [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _f, _vp, _f, _vp, _ll, _ll, _vp, _vp,
@@ -797,6 +851,18 @@ def linear_state_scan(mode: str, qkv: torch.Tensor, cols, group: int, gate: torc
     # blocks, which leave their outputs here for the kernel that norms and gates them
     sliced = step.B * heads < 96 and vdim > 32
     raw = torch.empty((T, heads * vdim), dtype=f32, device=out.device)
+    if walks_by_fours(step, dim):
+        ld, at = qkv.stride(0), lambda i: _at(qkv, cols[i])
+        more = (dict(mode=WALK_GLA, a=_at(decay_logits, decay_col), lda=decay_logits.stride(0),
+                     abias=_ptr(decay_bias), inv_tau=float(inv_tau)) if mode == "gla" else
+                dict(mode=WALK_DELTA, s0=_at(scalars, beta_col), s1=_at(scalars, rate_col),
+                     lds=scalars.stride(0), p0=_ptr(a_log), p1=_ptr(dt_bias),
+                     unit_eps=float(unit_eps)))
+        _state_walk(step, state, out, heads, dim, vdim, raw, q=at(0), k=at(1), v=at(2), ldq=ld,
+                    ldk=ld, ldv=ld, group=int(group), gate=_at(gate, gate_col), ldg=gate.stride(0),
+                    normw=_ptr(normw), eps=float(eps), q_scale=dim ** -0.5,
+                    head_stride=dim * vdim, **more)
+        return
     _call("linear_state", "mb_linear_state_scan",
           [_i, _vp, _i, _i, _i, _i, _i, _vp, _i, _i, _vp, _f, _vp, _i, _i, _i, _vp, _vp, _f,
            _vp, _i, _i, _vp, _f, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],

@@ -68,7 +68,7 @@ class GatedLinearAttention(Part):
         self.names = {k: prefix + v for k, v in p["names"].items()}
 
     def libraries(self, rt) -> List[str]:
-        return ["linear_state"]
+        return ["linear_state", "state_walk"]
 
     def tensors(self) -> List[TensorNeed]:
         n, W, H = self.names, self.hidden, self.nh
@@ -128,7 +128,7 @@ class GatedDelta(Part):
         self.channels = 2 * self.qkw + self.vw
 
     def libraries(self, rt) -> List[str]:
-        return ["linear_state"]
+        return ["linear_state", "state_walk"]
 
     def tensors(self) -> List[TensorNeed]:
         n, W, H = self.names, self.hidden, self.nh

@@ -105,7 +105,7 @@ class WkvMixer(Part):
                               "more than the kernel keeps on one multiprocessor")
 
     def libraries(self, rt) -> List[str]:
-        return ["recurrent"]
+        return ["recurrent", "state_walk"]
 
     def tensors(self) -> List[TensorNeed]:
         n, W, HD = self.names, self.hidden, self.width
@@ -174,7 +174,7 @@ class MlstmMixer(Part):
                               "more than the kernel keeps on one multiprocessor")
 
     def libraries(self, rt) -> List[str]:
-        return ["recurrent"]
+        return ["recurrent", "state_walk"]
 
     def tensors(self) -> List[TensorNeed]:
         n, W, H = self.names, self.hidden, self.nh

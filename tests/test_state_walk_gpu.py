@@ -1,0 +1,104 @@
+"""The recurrences four tokens at a time against the same walked token by token: outputs and the
+state that a step leaves, from a state that is not zero, at the edges of groups and chunks."""
+import pytest
+import torch
+
+from mormot2_ai_b200 import kernels as K
+from tests.gpu_helpers import DEV, make_step
+
+pytestmark = pytest.mark.gpu
+
+
+def rows(shape, seed, std=1.0, mean=0.0):
+    gen = torch.Generator().manual_seed(seed)
+    return (torch.randn(shape, generator=gen) * std + mean).to(DEV)
+
+
+def run(mode, step, state, T, heads, dim, vdim, group, shift, dtype):
+    out = torch.empty((T, heads * vdim), dtype=dtype, device=DEV)
+    qkw, vw = heads // group * dim, heads * vdim
+    z = rows((T, shift + 2 * qkw + 2 * vw + 2 * heads), 1)
+    z[:, shift:shift + 2 * qkw] *= dim ** -0.25
+    cols = [shift, shift + qkw, shift + 2 * qkw, shift + 2 * qkw + vw,
+            shift + 2 * qkw + 2 * vw, shift + 2 * qkw + 2 * vw + heads]
+    if mode == "mlstm":
+        K.mlstm_scan(z, cols, rows((heads,), 2), rows((heads,), 3, mean=4.0), 15.0, dim ** -0.5,
+                     rows((vw,), 4, 0.1, 1.0), 1e-6, state, step, out, heads, dim, vdim)
+    elif mode == "wkv":
+        r, k, v, g = (z[:, c:c + vw] for c in cols[:4])
+        h = rows((T, 24), 5).to(dtype)
+        lw = z.new_zeros(z.shape)[:, :vw]
+        lw.copy_(rows((T, vw), 6))
+        K.wkv_scan(r, k, v, lw, g, rows((vw,), 7, mean=-2.0), rows((vw,), 8), rows((vw,), 4, 0.1, 1.0),
+                   1e-6, state, h, step, out, heads, dim)
+    else:
+        more = (dict(decay_logits=rows((T, heads * dim + 3), 6), decay_col=3,
+                     decay_bias=rows((heads * dim,), 7), inv_tau=1 / 16) if mode == "gla" else
+                dict(scalars=z, beta_col=cols[4], rate_col=cols[5], a_log=rows((heads,), 2),
+                     dt_bias=rows((heads,), 3, mean=-2.0), unit_eps=1e-6))
+        K.linear_state_scan(mode, z, cols[:3], group, z, cols[3], rows((vdim,), 4, 0.1, 1.0), 1e-6,
+                            state, step, out, heads, dim, vdim, **more)
+    return out
+
+
+# 16 and 17 new tokens: a whole chunk and one more; 1 to 3: a group that is not full
+LENGTHS = [[16], [17, 1, 2], [3, 50, 33, 64]]
+
+
+@pytest.mark.parametrize("mode", ["gla", "delta", "mlstm", "wkv"])
+@pytest.mark.parametrize("heads, dim, vdim, group", [(2, 20, 24, 1), (4, 64, 128, 2), (2, 128, 36, 1),
+                                                     (1, 200, 72, 1), (40, 64, 64, 1)])
+@pytest.mark.parametrize("lens", LENGTHS)
+@pytest.mark.parametrize("shift", [0, 1])          # 1: rows that no 16-byte copy can take
+def test_four_tokens_at_a_time(monkeypatch, mode, heads, dim, vdim, group, lens, shift):
+    if mode in ("mlstm", "wkv"):
+        group = 1
+    if mode == "wkv":
+        vdim = dim
+    step = make_step([(i + 1, 5, [0] * n, []) for i, n in enumerate(lens)])
+    size = {"mlstm": heads * (dim * vdim + dim + 1), "wkv": 24 + heads * dim * dim}.get(
+        mode, heads * dim * vdim)
+    start = rows((len(lens) + 2, size + 3), 9, 0.3)
+    got = []
+    for fours in (False, True):
+        monkeypatch.setattr(K, "walks_by_fours", lambda *a: fours)
+        state = start.clone()
+        out = run(mode, step, state, sum(lens), heads, dim, vdim, group, shift, torch.float32)
+        got.append((out, state))
+    (want, state), (out, state4) = got
+    # float32 sums over the head and the tokens in another order, divided by a root mean square
+    assert (out - want).norm() <= 2e-5 * want.norm()
+    assert (state4 - state).norm() <= 2e-6 * state.norm()
+    assert torch.equal(state4[0], start[0]) and torch.equal(state4[-1], start[-1])
+    assert torch.equal(state4[:, size:], start[:, size:])
+
+
+def test_which_steps_go_by_fours():
+    long, short = make_step([(0, 0, [0] * 16, [])]), make_step([(0, 0, [0] * 15, [])])
+    assert K.walks_by_fours(long, 256)
+    assert not K.walks_by_fours(long, 257) and not K.walks_by_fours(short, 64)
+
+
+# four taps go four channels a thread in runs of 16 tokens, unless rows or channels do not allow it
+@pytest.mark.parametrize("taps, channels, shift", [(4, 40, 0), (4, 520, 4), (4, 42, 0), (4, 40, 1),
+                                                   (3, 40, 0)])
+@pytest.mark.parametrize("lens", [[1], [2, 1, 3], [15, 18], [1, 40, 16, 5]])
+def test_short_convolution(taps, channels, shift, lens):
+    T = sum(lens)
+    z = rows((T, channels + 8), 1)
+    w = rows((channels, taps), 2)
+    size = (taps - 1) * channels
+    states = rows((len(lens) + 1, 8 + size), 3)
+    step = make_step([(i + 1, 9, [0] * n, []) for i, n in enumerate(lens)])
+    before = states.clone()
+    out = torch.empty((T, channels), device=DEV)
+    K.short_conv(z, shift, w, states[:, 8:], step, out)
+    at = 0
+    for i, n in enumerate(lens):
+        past = before[i + 1, 8:].double().view(taps - 1, channels)
+        x = torch.cat([past, z[at:at + n, shift:shift + channels].double()])
+        want = torch.nn.functional.silu(sum(x[j:j + n] * w[:, j].double() for j in range(taps)))
+        # four products and a sigmoid in float32
+        assert (out[at:at + n].double() - want).abs().max() <= 1e-5
+        assert torch.equal(states[i + 1, 8:].view(taps - 1, channels), x[n:].float())
+        at += n
