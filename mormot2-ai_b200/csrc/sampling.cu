@@ -29,14 +29,8 @@ __device__ __forceinline__ bool better(const Best& a, const Best& b) {
   return a.v > b.v || (a.v == b.v && a.i < b.i);
 }
 
-__device__ Best block_argmax(const float* __restrict__ row, int V, Best* sh) {
-  Best b = {0.f, -1};
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float v = row[i];
-    if (v != v) continue;  // NaN
-    const Best c = {v, i};
-    if (better(c, b)) b = c;
-  }
+// the best of the block's threads (index 0 if none has one)
+__device__ Best block_best(Best b, Best* sh) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     Best c;
@@ -64,6 +58,17 @@ __device__ Best block_argmax(const float* __restrict__ row, int V, Best* sh) {
   __syncthreads();
   if (b.i < 0) b.i = 0;  // all NaN
   return b;
+}
+
+__device__ Best block_argmax(const float* __restrict__ row, int V, Best* sh) {
+  Best b = {0.f, -1};
+  for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    const float v = row[i];
+    if (v != v) continue;  // NaN
+    const Best c = {v, i};
+    if (better(c, b)) b = c;
+  }
+  return block_best(b, sh);
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
@@ -401,42 +406,58 @@ __device__ double block_sum_double(double v, double* sh) {
 
 // By a whole block: the sum of w[0 .. n) when `total_only`, else the first index whose running
 // sum (in index order) reaches `target` (strict: exceeds it), left in *found (n if none).
-// Every thread sums a contiguous run, one thread adds the runs up in order, the thread whose
-// run holds the target walks it. `runs` holds SAMPLE_THREADS doubles.
+// Every thread sums a contiguous run, the runs are added up by a scan over the block (one thread
+// adding 512 of them in turn took 10 us, three times a draw), and the thread between whose sum and
+// the next one's the target lies walks its run. `runs` holds SAMPLE_THREADS doubles.
 __device__ double block_walk(const double* __restrict__ w, int n, double target, bool strict,
                              bool total_only, double* runs, int* found) {
+  __shared__ double warp_sums[33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int per = (n + blockDim.x - 1) / blockDim.x;
   const int i0 = min(n, (int)threadIdx.x * per), i1 = min(n, i0 + per);
   double mine = 0.0;
   for (int i = i0; i < i1; ++i) mine += w[i];
-  runs[threadIdx.x] = mine;
+  double incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  double before = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) before = 0.0;
+  if (lane == 31) warp_sums[warp] = incl;
   if (threadIdx.x == 0) *found = n;
   __syncthreads();
-  __shared__ double total_sh;
-  if (threadIdx.x == 0) {
-    double total = 0.0;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      const double v = runs[t];
-      runs[t] = total;
-      total += v;
+  if (warp == 0) {
+    double t = lane < warps ? warp_sums[lane] : 0.0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += v;
     }
-    total_sh = total;
+    __syncwarp();
+    warp_sums[lane + 1] = t;      // what lies before warp lane + 1
+    if (lane == 0) warp_sums[0] = 0.0;
   }
   __syncthreads();
-  const double total = total_sh;
+  const double total = warp_sums[warps];
   if (!total_only) {
-    const double before = runs[threadIdx.x];
-    const bool here = strict ? (target >= before && target < before + mine)
-                             : (target > before && target <= before + mine);
-    if (here) {
+    before += warp_sums[warp];
+    runs[threadIdx.x] = before;
+    __syncthreads();
+    // the sums rise from 0 to the total, so some thread's step holds the target (a rounding may
+    // give a second one: the first counts)
+    const double after = threadIdx.x + 1 < blockDim.x ? runs[threadIdx.x + 1] : total;
+    const bool here = strict ? (target >= before && target < after)
+                             : (target > before && target <= after);
+    if (here && i1 > i0) {
       double cum = before;
-      for (int i = i0; i < i1; ++i) {
+      int i = i0;
+      for (; i < i1 - 1; ++i) {      // the last one is it if none before it is
         cum += w[i];
-        if (strict ? target < cum : cum >= target) {
-          atomicMin(found, i);
-          break;
-        }
+        if (strict ? target < cum : cum >= target) break;
       }
+      atomicMin(found, i);
     }
   }
   __syncthreads();
@@ -746,7 +767,12 @@ sample_filtered_kernel(const float* __restrict__ logits, size_t stride, int V, d
 // The filtered draw over a wide row: the passes over the vocabulary (best value, sum, counting
 // and gathering the candidates) are shared by a cluster of SAMPLE_CTAS CTAs that exchange their
 // counts and sums through each other's shared memory; the first CTA then sorts, filters and
-// draws as above. Every CTA takes the same decisions from the same exchanged numbers.
+// draws as above. Every CTA takes the same decisions from the same exchanged numbers. HELD: a CTA's
+// share stays in its shared memory and is read once for all passes (up to 393,216 tokens; 8 rows
+// of 151,936 at top-p 0.9, peaked: 60 us with every pass from L2 and sums added up by one
+// thread, 31 now).
+#define SAMPLE_HELD 49152      // tokens of a share: 192 KB
+template <bool HELD>
 __global__ void __launch_bounds__(SAMPLE_CL_THREADS)
 sample_filtered_cluster_kernel(const float* __restrict__ logits, size_t stride, int V,
                                double inv_t, int top_k, double top_p, double min_p,
@@ -768,11 +794,25 @@ sample_filtered_cluster_kernel(const float* __restrict__ logits, size_t stride, 
   const int share = (V + SAMPLE_CTAS - 1) / SAMPLE_CTAS;
   const int lo = min(V, (int)rank * share), hi = min(V, lo + share);
 
+  extern __shared__ float held[];      // every thread reads the places that it wrote
+  if (HELD) {
+#pragma unroll 8
+    for (int i = lo + (int)threadIdx.x; i < hi; i += SAMPLE_CL_THREADS) held[i - lo] = row[i];
+  }
+  // f(value, index) for this thread's tokens of the share
+  auto each = [&](auto f) {
+#pragma unroll 4
+    for (int i = lo + (int)threadIdx.x; i < hi; i += SAMPLE_CL_THREADS) f(HELD ? held[i - lo] : row[i], i);
+  };
   Best b = {0.f, -1};
-  if (hi > lo) {
-    b = block_argmax(row + lo, hi - lo, sh);
-    const float v = row[lo + b.i];
-    b = Best{v, v != v ? -1 : lo + b.i};
+  each([&](float v, int i) {
+    const Best c = {v, i};
+    if (v == v && better(c, b)) b = c;  // not a NaN
+  });
+  {
+    const bool any = __syncthreads_or(b.i >= 0);
+    b = block_best(b, sh);
+    if (!any) b.i = -1;
   }
   if (threadIdx.x == 0)
     mine_best = ((unsigned long long)__float_as_uint(b.v) << 32) | (unsigned)b.i;
@@ -816,7 +856,7 @@ sample_filtered_cluster_kernel(const float* __restrict__ logits, size_t stride, 
   double sum = 0.0;
   if (whole_mass) {
     double mine = 0.0;
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) mine += weight_of(row[i], best.v, inv_t);
+    each([&](float v, int) { mine += weight_of(v, best.v, inv_t); });
     mine = block_sum_double(mine, dsh);
     int unused;
     exchange(0, mine, unused, sum);
@@ -830,15 +870,14 @@ sample_filtered_cluster_kernel(const float* __restrict__ logits, size_t stride, 
     const double log_t = ts.log_t;
     int cnt = 0;
     double above = 0.0;
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      const float v = row[i];
+    each([&](float v, int) {
       const bool finite = (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u;
       const double x = ((double)v - (double)best.v) * inv_t;
       if (finite && x >= log_t) {
         ++cnt;
         if (whole_mass) above += exp(x);
       }
-    }
+    });
     if (whole_mass) above = block_sum_double(above, dsh);
     cnt = (int)(block_sum_double((double)cnt, dsh) + 0.5);
     double above_all;
@@ -852,14 +891,13 @@ sample_filtered_cluster_kernel(const float* __restrict__ logits, size_t stride, 
   // every share's candidates go behind those of the shares before it
   if (threadIdx.x == 0) fill_sh = 0;
   __syncthreads();
-  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    const float v = row[i];
+  each([&](float v, int i) {
     const bool finite = (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u;
     if (finite && ((double)v - (double)best.v) * inv_t >= log_t) {
       const int at = my_before + atomicAdd(&fill_sh, 1);
       keys[at] = ((unsigned long long)(~ordered_bits(v)) << 32) | (unsigned)i;
     }
-  }
+  });
   __threadfence();
   smp_cluster_sync();  // all keys are written (and nobody reads a mailbox any more)
   sort_candidates<SAMPLE_CTAS>(keys, n, (int)rank);  // ends at the cluster's barrier
@@ -883,8 +921,18 @@ MB_EXPORT int mb_sample_filtered(const float* logits, long long stride, int rows
   if (scratch_stride < V || (scratch_stride & (scratch_stride - 1)))
     MB_FAIL("mb_sample_filtered: a scratch row of %lld words for %d tokens", scratch_stride, V);
   if (V >= 16384 && rows <= 8192) {  // a wide row: a cluster of CTAs shares the passes over it
-    mb_launch_clusters(sample_filtered_cluster_kernel, dim3(rows * SAMPLE_CTAS),
-                       dim3(SAMPLE_CL_THREADS), 0, (cudaStream_t)stream, SAMPLE_CTAS, logits,
+    const int share = (V + SAMPLE_CTAS - 1) / SAMPLE_CTAS;
+    const bool held = share <= SAMPLE_HELD;
+    auto* kernel = held ? sample_filtered_cluster_kernel<true> : sample_filtered_cluster_kernel<false>;
+    const size_t smem = held ? (size_t)share * sizeof(float) : 0;
+    static bool configured = false;
+    if (!configured) {
+      cudaFuncSetAttribute(sample_filtered_cluster_kernel<true>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_HELD * (int)sizeof(float));
+      configured = true;
+    }
+    mb_launch_clusters(kernel, dim3(rows * SAMPLE_CTAS),
+                       dim3(SAMPLE_CL_THREADS), smem, (cudaStream_t)stream, SAMPLE_CTAS, logits,
                        (size_t)stride, V, 1.0 / temperature, top_k, top_p, min_p, state_index,
                        states, scratch, (size_t)scratch_stride, out);
     MB_CHECK_LAUNCH("mb_sample_filtered");
