@@ -255,7 +255,7 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 #define QK_PASSES 3  // groups of heads that a warp of the wide form takes, at most
-template <int HD, bool PARTIAL>
+template <int HD, bool PARTIAL, bool WIDE_W>   // WIDE_W: bfloat16 norm weights on 16-byte boundaries
 __global__ void __launch_bounds__(QK_WARPS * 32)
 qk_wide_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ partial, int parts,
                size_t part_stride, __nv_bfloat16* __restrict__ q_out,
@@ -277,6 +277,16 @@ qk_wide_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ partia
   const int group0 = (blockIdx.y * (blockDim.x >> 5) + warp) * passes;
   float cs[8], sn[8];
   bool have_angles = false;
+  // this lane's norm weights, eight of a head's first half and eight of its second, for q and k
+  uint4 nw[2][2];
+  const bool wide_w = WIDE_W && q_norm && !unit_after;
+  if (wide_w) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      nw[0][h] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)q_norm + h * HALF + 8 * sl);
+      nw[1][h] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)k_norm + h * HALF + 8 * sl);
+    }
+  }
   // every pass's values are asked for before the first pass is worked on: a pass's stores
   // may lie over the next one's source (q is rotated in place), so the compiler would not
   // move the loads up by itself, and three round trips to memory in a row would set the time
@@ -348,7 +358,17 @@ qk_wide_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ partia
       }
       if (live && (is_q || is_k)) {
         const void* w = is_q ? q_norm : k_norm;
-        if (w && !unit_after) {
+        if (wide_w) {
+          const float inv = 1.0f / sqrtf(sum / (float)HD + eps);
+          float wa[8], wb[8];
+          unpack8(is_q ? nw[0][0] : nw[1][0], wa);
+          unpack8(is_q ? nw[0][1] : nw[1][1], wb);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            a[j] = wa[j] * (a[j] * inv);
+            b[j] = wb[j] * (b[j] * inv);
+          }
+        } else if (w && !unit_after) {
           const float inv = 1.0f / sqrtf(sum / (float)HD + eps);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -439,18 +459,29 @@ MB_EXPORT int mb_qk_norm_rope_store(void* qkv, const float* partial, int parts,
 #undef QKN
       MB_CHECK_LAUNCH("mb_qk_norm_rope_store");
     }
-    // groups of 512 / hd heads: blocks of four warps that take three groups each
+    // groups of 512 / hd heads: a warp takes one to three, whichever costs least when a warp's own
+    // work (sines, cosines, weights) counts as 0.7 of a group's and idle places count too (8 groups
+    // of 16 heads on 8: two a warp, where three left the last of four warps without any)
     const int groups = ((nh + 2 * nkv) * hd + 511) / 512;
-    const int warps = QK_WARPS, passes = QK_PASSES;
+    const int warps = QK_WARPS;
+    int passes = QK_PASSES;
+    float best = 1e30f;
+    for (int n = QK_PASSES; n >= 1; --n) {
+      const float cost = (groups + warps * n - 1) / (warps * n) * warps * (n + 0.7f);
+      if (cost < best) { best = cost; passes = n; }
+    }
+    const bool wide_w = w_bf16 && q_norm && k_norm && (((uintptr_t)q_norm | (uintptr_t)k_norm) & 15) == 0;
     dim3 fgrid(T, (groups + warps * passes - 1) / (warps * passes));
-#define QKF(HD_, P_)                                                                           \
-  mb_launch(qk_wide_kernel<HD_, P_>, fgrid, dim3(warps * 32), 0, s, (bf*)qkv, partial, parts,  \
+#define QKF(HD_, P_, W_)                                                                       \
+  mb_launch(qk_wide_kernel<HD_, P_, W_>, fgrid, dim3(warps * 32), 0, s, (bf*)qkv, partial, parts,  \
       (size_t)part_stride, (bf*)q_out, q_norm, k_norm, w_bf16, eps, inv_freq, tok_slot,        \
       tok_pos, page_table, max_pages, ring_pages, (bf*)kpool, (bf*)vpool, nh, nkv,   \
       write_kv, passes, ld, unit_after)
+#define QKF_H(HD_, P_) if (wide_w) QKF(HD_, P_, true); else QKF(HD_, P_, false)
 #define QKF_V(P_)                                                                              \
-  if (hd == 64) QKF(64, P_); else if (hd == 128) QKF(128, P_); else QKF(256, P_)
+  if (hd == 64) { QKF_H(64, P_); } else if (hd == 128) { QKF_H(128, P_); } else { QKF_H(256, P_); }
     if (partial) { QKF_V(true); } else { QKF_V(false); }
+#undef QKF_H
 #undef QKF_V
 #undef QKF
     MB_CHECK_LAUNCH("mb_qk_norm_rope_store");
