@@ -34,11 +34,10 @@ MB_DEFINE_LAST_ERROR
 
 static thread_local int g_last_launches = 0;
 static thread_local int g_last_splits = 1;
-// splits of K in the last mb_gemm_tc of this thread; with `defer` and more than one split the
-// partial sums [splits][M][N] were left in the workspace for the caller's next kernel to add
-MB_EXPORT int mb_gemm_tc_last_splits() { return g_last_splits; }
-// kernels that the last mb_gemm_tc of this thread launched (2 when K was split)
-MB_EXPORT int mb_gemm_tc_last_launches() { return g_last_launches; }
+// of the last mb_gemm_tc of this thread: the splits of K (with `defer` and more than one the partial
+// sums [splits][M][N] were left in the workspace for the caller's next kernel to add) + 256 x the
+// kernels that it launched (2 when K was split and the sums were added up here)
+MB_EXPORT int mb_gemm_tc_last() { return g_last_splits | g_last_launches << 8; }
 
 // TC_SWIGLU and TC_GEGLU: the weight's rows alternate gate and up and the output is
 // act(gate) * up with act = SiLU or the tanh form of GELU. In these two modes nothing is split,
@@ -900,7 +899,7 @@ MB_EXPORT int mb_gemm_tc_supported(const void* A, int lda, const void* W, int M,
 // C[M, N / 2] = SwiGLU over a W whose rows alternate gate and up (3, bfloat16 C). `workspace` (float32, may be null) lets the K range be split;
 // `error` is a device word that receives a non-zero code if a wait in the kernel ran out
 // (1 load, 2 MMA, 3 epilogue). `sms`: the number of SMs of the device. `defer`: when K was split
-// (mb_gemm_tc_last_splits() > 1) the partial sums stay in the workspace as [splits][M][N] and C
+// (mb_gemm_tc_last() says so) the partial sums stay in the workspace as [splits][M][N] and C
 // is not touched: the caller's next kernel adds them up.
 MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_dtype, int ldc,
                          int M, int N, int K, int epilogue, float* workspace,

@@ -44,7 +44,7 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 def _stream() -> int:
     """The current CUDA stream of the current device as the integer that the kernels take."""
     if _raw_stream is not None:                     # the short way (no Stream object)
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(torch._C._cuda_getDevice())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -166,12 +166,22 @@ def read_trace() -> list:
     return rows
 
 
-def _call(libname: str, fn: str, argtypes, *args, launches: int = 1) -> None:
+_functions: dict = {}      # entry points by name, with their library, once they were called
+
+
+def _function(libname: str, fn: str, argtypes):
+    """The library's entry point with its argument types set, and the library. Found once: a
+    step of a few tokens is bound by what the host does for each of its launches."""
     lib = build.load_library(libname)
     f = getattr(lib, fn)
-    if f.argtypes is None:
-        f.argtypes = argtypes
-        f.restype = _i
+    f.argtypes = argtypes
+    f.restype = _i
+    _functions[fn] = f, lib
+    return f, lib
+
+
+def _call(libname: str, fn: str, argtypes, *args, launches: int = 1) -> None:
+    f, lib = _functions.get(fn) or _function(libname, fn, argtypes)
     timing = Timing.current
     if timing is not None:
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -1391,9 +1401,9 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, add: bool,
           workspace.numel() if workspace is not None else 0, 1 if defer else 0,
           _ptr(error), sms, _stream())
     # the split of K adds one kernel that sums the partial products
-    lib = build.load_library("gemm_tc")
-    Launches.count += lib.mb_gemm_tc_last_launches() - 1
-    return lib.mb_gemm_tc_last_splits()
+    last = _functions["mb_gemm_tc"][1].mb_gemm_tc_last()
+    Launches.count += (last >> 8) - 1
+    return last & 255
 
 
 def gemm_tc_gated(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, act: int,

@@ -40,7 +40,7 @@ class FastLinear:
         splits = K.gemm_tc(a, self.weight, c, False, buf, rt.error_word, rt.sms, defer=True)
         if splits <= 1:
             return Pending(c.unsqueeze(0))
-        return Pending(buf[:splits * M * N].view(splits, M, N))
+        return Pending(buf.as_strided((splits, M, N), (M * N, N, 1)))
 
     def __call__(self, a: torch.Tensor, out: Optional[torch.Tensor],
                  add_into: Optional[torch.Tensor]) -> bool:
