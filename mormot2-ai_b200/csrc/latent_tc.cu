@@ -13,8 +13,8 @@
 // one more block of 64 columns of the K tile, filled up with zeros: what lies behind a head's
 // rotated query part then counts nothing.
 //
-// A CTA takes 256 consecutive new tokens of one sequence and one query head (the only CTA of its
-// SM) as two row tiles of 128 that share every K and V tile:
+// A CTA takes 256 new tokens of one sequence and one query head (the only CTA of its SM) as two
+// row tiles of 128 that share the K and V tiles that both see:
 //   warp 0      loads Q once, then K and V of 64 keys after 64 keys into rings of stages;
 //   warp 1      issues S of both row tiles two steps ahead, each into one of two buffers of its
 //               tile, and O += P V when P of a step is ready: the products of one row tile run
@@ -162,7 +162,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
                          int out_stride, const int* __restrict__ seq_start,
                          const int* __restrict__ seq_past, int nh, int rot_dim, int window,
                          float scale_log2, int* __restrict__ error, const bf16* __restrict__ gate,
-                         int gate_stride) {
+                         int gate_stride, int apart) {
   constexpr int VD = 64 * VH, DIM = 64 * DH;
   constexpr int Q_BYTES = (DH + 1) * LT_Q_HALF, K_BYTES = (DH + 1) * LT_HALF, V_BYTES = VH * LT_HALF;
   extern __shared__ __align__(1024) uint8_t lt_smem[];
@@ -185,21 +185,31 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.z, h = blockIdx.x;
   const int start = seq_start[b], n_new = seq_start[b + 1] - start;
-  const int row0 = (int)(gridDim.y - 1 - blockIdx.y) * 2 * LT_ROWS;   // the longest first
-  if (row0 >= n_new) return;  // the whole CTA, before anything is set up
+  // `apart`: the CTA takes the i-th row tile and the i-th from the end, so that one round of CTAs
+  // ends together: neighbours give the last CTA twice the average's keys and the first next to none
+  // (2,048 tokens, 16 heads of 128 + 64: 73 -> 58 us). Otherwise neighbours, whose keys are nearly
+  // the same: with a window, and where the CTAs take several rounds, the longest first (four prompts
+  // of up to 1,000: 49 us, 53 apart).
+  const int tiles = (n_new + LT_ROWS - 1) / LT_ROWS;
+  const int pair = apart ? (int)blockIdx.y : (int)(gridDim.y - 1 - blockIdx.y);
+  if (pair >= (tiles + 1) / 2) return;  // the whole CTA, before anything is set up
+  const int row0 = (apart ? pair : 2 * pair) * LT_ROWS;
+  const int row1 = (!apart ? 2 * pair + 1 : 2 * pair + 1 == tiles ? tiles : tiles - 1 - pair) * LT_ROWS;
   const int past = seq_past[b];
   int lo_b;
   const int base = gathered_base(seq_start, seq_past, b, window, lo_b);
-  const int first_pos = past + row0, last_pos = past + min(row0 + 2 * LT_ROWS - 1, n_new - 1);
+  // the second tile may lie behind the last token: then it has no steps
+  const int first_pos = past + row0;
+  const int last_pos = past + min((row1 < n_new ? row1 : row0) + LT_ROWS - 1, n_new - 1);
   const int key_lo = (window > 0 && first_pos + 1 > window) ? first_pos + 1 - window : 0;
   const int steps = (last_pos - key_lo) / MB_PAGE + 1;
   // the steps of row tile m: from the first key of its first row to its last row
   auto tile_lo = [&](int m) {
-    const int p = first_pos + m * LT_ROWS;
+    const int p = past + (m ? row1 : row0);
     return p > last_pos ? 0 : ((window > 0 && p + 1 > window ? p + 1 - window : 0) - key_lo) / MB_PAGE;
   };
   auto tile_hi = [&](int m) {
-    const int p = first_pos + m * LT_ROWS;
+    const int p = past + (m ? row1 : row0);
     return p > last_pos ? 0 : (min(p + LT_ROWS - 1, last_pos) - key_lo) / MB_PAGE + 1;
   };
   const int lo0 = tile_lo(0), hi0 = tile_hi(0), lo1 = tile_lo(1), hi1 = tile_hi(1);
@@ -238,7 +248,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
       for (int m = 0; m < 2; ++m)
         for (int i = 0; i <= DH; ++i)
           tma_load_2d(sQ + m * Q_BYTES + i * LT_Q_HALF, &tmQ, h * (DIM + rot_dim) + 64 * i,
-                      start + row0 + m * LT_ROWS, q_full);
+                      start + (m ? row1 : row0), q_full);
       const int y0 = base + key_lo - lo_b;
       auto load_k = [&](int j) {
         const int st = j % LT_K_STAGES, y = y0 + j * MB_PAGE;
@@ -322,8 +332,8 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
   } else {
     const int m = warp >= 6;     // the row tile
     const int q = warp & 3;      // the TMEM lanes of this warp
-    const int row = m * LT_ROWS + q * 32 + lane;
-    const int pos = first_pos + row;    // position of this thread's token
+    const int row = (m ? row1 : row0) + q * 32 + lane;
+    const int pos = past + row;         // position of this thread's token
     const int lo = (window > 0 && pos + 1 > window) ? pos + 1 - window : 0;
     const int j_lo = m ? lo1 : lo0, n = (m ? hi1 : hi0) - j_lo;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
@@ -405,8 +415,8 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
       mbar_wait(o_done + 8 * ((n - 1) & 1), ((n - 1) >> 1) & 1, error, 18);
       tc_fence_after_sync();
       const float inv = 1.0f / l;
-      const bf16* gates = gate != nullptr && row0 + row < n_new
-                              ? gate + (size_t)(start + row0 + row) * gate_stride + (size_t)h * VD
+      const bf16* gates = gate != nullptr && row < n_new
+                              ? gate + (size_t)(start + row) * gate_stride + (size_t)h * VD
                               : nullptr;
       // the tile's Q memory is free now: a warp lays its 32 rows there (16-byte piece p of row r
       // at p ^ (r & 7): no bank conflicts either way) and writes whole rows out
@@ -439,7 +449,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
       }
       __syncwarp();
       constexpr int PIECES = VD / 8, AT_ONCE = 32 / PIECES;
-      const int pc = lane % PIECES, first_row = row0 + m * LT_ROWS + q * 32;
+      const int pc = lane % PIECES, first_row = (m ? row1 : row0) + q * 32;
 #pragma unroll 4
       for (int i = 0; i < 32 / AT_ONCE; ++i) {
         const int r = AT_ONCE * i + lane / PIECES;
@@ -481,6 +491,13 @@ MB_EXPORT int mb_latent_prefill_tc(const void* q, int q_stride, const void* kv, 
   if (!mb_make_map_bf16(&tmKV, kv, R, (long long)nh * (dim + vd), kv_stride, MB_PAGE, who)) return -1;
   if (!mb_make_map_bf16(&tmR, rot, R, 64, 64, MB_PAGE, who)) return -1;
   dim3 grid(nh, row_tiles, B);
+  static const int sms = [] {
+    int device = 0, n = 148;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+    return n;
+  }();
+  const int apart = window <= 0 && (long long)nh * row_tiles * B <= sms;
 #define GO(DH_, VH_)                                                                           \
   {                                                                                            \
     constexpr int smem = 2 * (DH_ + 1) * LT_Q_HALF + LT_K_STAGES * (DH_ + 1) * LT_HALF +       \
@@ -495,7 +512,7 @@ MB_EXPORT int mb_latent_prefill_tc(const void* q, int q_stride, const void* kv, 
     mb_launch(latent_prefill_tc_kernel<DH_, VH_>, grid, dim3(LT_THREADS), smem,                \
               (cudaStream_t)stream, tmQ, tmKV, tmR, (bf16*)out, out_stride, seq_start,         \
               seq_past, nh, rot_dim, window, scale * 1.4426950408889634f, error,               \
-              (const bf16*)gate, gate_stride);                                                 \
+              (const bf16*)gate, gate_stride, apart);                                          \
   }
   if (dim == 128) { if (vd == 128) GO(2, 2) else GO(2, 1) }
   else { if (vd == 128) GO(1, 2) else GO(1, 1) }
