@@ -99,3 +99,24 @@ def test_an_infinite_value_reaches_only_the_tokens_that_see_it(n):
     assert torch.isinf(got[bad:, :, 3]).all()
     got[bad:, :, 3] = 0
     assert torch.isfinite(got).all()
+
+
+# more CTAs than run at once: they take the sequences by length, equal lengths among them
+@pytest.mark.parametrize("count, splits", [(50, 1), (38, 1), (160, 1), (161, 1), (20, 2)])
+def test_decode_takes_sequences_by_length(count, splits):
+    nh, nkv, hd = 16, 8, 64
+    rng = np.random.default_rng(count)
+    lens = [int(n) for n in rng.choice([1, 2, 63, 64, 65, 130, 200], count)]
+    line = make_line(count, 256, nkv, hd, torch.bfloat16, seed=count)
+    line.k.copy_(torch.tensor(rng.standard_normal(line.k.shape)))
+    line.v.copy_(torch.tensor(rng.standard_normal(line.v.shape)))
+    step = make_step([(i, n - 1, [0], []) for i, n in enumerate(lens)], max_seqs=count)
+    q = torch.tensor(rng.standard_normal((count, nh * hd))).to(torch.bfloat16).to(DEV)
+    got, want = torch.empty_like(q), torch.empty((count, nh * hd), device=DEV)
+    error = torch.zeros(1, dtype=torch.int32, device=DEV)
+    K.attention_decode_clusters(q, nh * hd, got, step, line, nh, nkv, hd, 0, 0.125, splits, error)
+    assert int(error.item()) == 0
+    line32 = type(line)(line.k.float(), line.v.float(), line.page_table, line.max_pages, 0, 0, nkv, hd)
+    K.attention_simt(q.float(), nh * hd, want, step, line32, nh, nkv, hd, 0, 0.125)
+    # probabilities and outputs rounded to bfloat16, 2^-9 each
+    assert ((got.float() - want).norm(dim=1) <= 1e-2 * want.norm(dim=1)).all()
