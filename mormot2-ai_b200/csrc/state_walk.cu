@@ -537,10 +537,11 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
       // the outputs, a token a lane (a column's two lanes, P = 4, have two each)
       auto output = [&](int t, float r, float4 n4, float factor, float floor_) {
         float o = CHANNEL ? r : r * factor;
+        // not by zeros for the later ones: an infinity of theirs must not reach this token
         o = fmaf(n4.x, x[0], o);
-        o = fmaf(n4.y, x[1], o);
-        o = fmaf(n4.z, x[2], o);
-        o = fmaf(n4.w, x[3], o);
+        if (t >= 1) o = fmaf(n4.y, x[1], o);
+        if (t >= 2) o = fmaf(n4.z, x[2], o);
+        if (t >= 3) o = fmaf(n4.w, x[3], o);
         // the normalizer's column leaves the denominator
         if (MODE == WALK_MLSTM && norm_col) o = fmaxf(fabsf(o), floor_) + 1e-6f;
         so[((ci & 1) * CT + 4 * gr + t) * CW + mine] = o;

@@ -102,3 +102,28 @@ def test_short_convolution(taps, channels, shift, lens):
         assert (out[at:at + n].double() - want).abs().max() <= 1e-5
         assert torch.equal(states[i + 1, 8:].view(taps - 1, channels), x[n:].float())
         at += n
+
+
+@pytest.mark.parametrize("mode", ["gla", "delta", "mlstm", "wkv"])
+@pytest.mark.parametrize("bad", [1, 7, 18])
+def test_an_infinity_does_not_reach_earlier_tokens(mode, bad):
+    T, heads, dim = 20, 2, 64
+    step = make_step([(0, 0, [0] * T, [])])
+    size = {"mlstm": heads * (dim * dim + dim + 1), "wkv": 24 + heads * dim * dim}.get(
+        mode, heads * dim * dim)
+    args = (T, heads, dim, dim, 1, 0, torch.float32)
+    clean = run(mode, step, torch.zeros((1, size), device=DEV), *args)
+    real = globals()["rows"]
+    try:
+        def spoiled(shape, seed, *a, **k):
+            t = real(shape, seed, *a, **k)
+            if seed == 1:                 # a value of the token, in the second head
+                t[bad, 2 * heads * dim + dim + 3] = float("inf")
+            return t
+        globals()["rows"] = spoiled
+        out = run(mode, step, torch.zeros((1, size), device=DEV), *args)
+    finally:
+        globals()["rows"] = real
+    assert torch.equal(out[:bad], clean[:bad])
+    assert torch.equal(out[:, :dim], clean[:, :dim])
+    assert not torch.isfinite(out[bad, dim:]).all()
