@@ -17,6 +17,9 @@
 // tokens are staged in shared memory at a time, the next chunk's copies under way while one
 // is walked, and a chunk is walked without a barrier.
 //
+// Steps of 16 and more new tokens a sequence take the same recurrences four tokens at a time
+// (state_walk.cu); this walk serves decoding and short portions.
+//
 //   short_conv   y_t = silu(sum_j w[c, j] x_(t - taps + 1 + j)) per channel, the inputs before
 //                a step's first token from the state (zeros at a sequence's start)
 #include "common.cuh"

@@ -330,18 +330,35 @@ sample_cluster_kernel(const float* __restrict__ logits, size_t stride, int V, do
   const double ws = warp_sums[warp];
   if (target >= wb && target < wb + ws) {
     double cum = wb;
-    for (int i0 = w0; i0 < w1; i0 += 32) {
-      const int i = i0 + lane;
-      const double w = i < w1 ? weight_of(row[i], best.v, inv_t) : 0.0;
-      double incl = w;
+    // 128 ids at a time, four neighbours a lane, whose loads and exponentials run side by side
+    // (32 at a time the walk was a third of the kernel: 8 rows of 151,936, 39 -> WALK_AFTER us)
+    for (int i0 = w0; i0 < w1; i0 += 128) {
+      const int i = i0 + 4 * lane;
+      double w[4], incl = 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        w[q] = i + q < w1 ? weight_of(row[i + q], best.v, inv_t) : 0.0;
+        incl += w[q];
+      }
+      const bool any = incl > 0.0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const double v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
-      const unsigned hit = __ballot_sync(0xffffffffu, w > 0.0 && target < cum + incl);
+      double before_lane = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (lane == 0) before_lane = 0.0;
+      const unsigned hit = __ballot_sync(0xffffffffu, any && target < cum + incl);
       if (hit) {
-        if (lane == 0) found = i0 + __ffs(hit) - 1;
+        if (lane == __ffs(hit) - 1) {
+          double c = cum + before_lane;
+          int at = -1;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {      // the last one with a weight if rounding leaves none
+            if (w[q] > 0.0 && (at < 0 || !(target < c))) at = i + q, c += w[q];
+          }
+          found = at;
+        }
         break;
       }
       cum += __shfl_sync(0xffffffffu, incl, 31);
