@@ -40,7 +40,6 @@ class CacheStorage:
         self.pools: List[torch.Tensor] = []
         self.tables: List[torch.Tensor] = []
         self.tables_host: List[torch.Tensor] = []
-        self.tables_copied, self.tables_in_flight = torch.cuda.Event(), False
         self.lines: Dict[int, CacheLine] = {}
         self.value_pools: Dict[int, torch.Tensor] = {}   # of groups whose value rows differ in size
         for g, plan in enumerate(plans):
@@ -60,7 +59,9 @@ class CacheStorage:
                              dtype, device)
             table = alloc(guards, f"page table of group {g}", (max_slots, plan.max_pages),
                           torch.int32, device)
-            host = torch.zeros((max_slots, plan.max_pages), dtype=torch.int32).pin_memory()
+            # pageable on purpose: the copy to the device then reads it before returning, so the
+            # host may change it again at once
+            host = torch.zeros((max_slots, plan.max_pages), dtype=torch.int32)
             self.pools.append(pool)
             self.tables.append(table)
             self.tables_host.append(host)
@@ -89,12 +90,9 @@ class CacheStorage:
                 + sum(2 * s.numel() * s.element_size() for s in self.states.values()))
 
     def map_pages(self, new_entries: List[List[Tuple[int, int, int]]]) -> None:
-        """Writes the new table entries of ``CacheBook.reserve`` to the device tables: copies from
-        pinned memory, which the host does not wait for (a copy that it waits for would keep the
-        launches of a step from going out while the step before still runs)."""
-        if self.tables_in_flight and any(new_entries):
-            self.tables_copied.synchronize()   # the last copies must have read the host tables
-            self.tables_in_flight = False
+        """Writes the new table entries of ``CacheBook.reserve`` to the device tables, in the order of
+        the stream. The copy stages the host's entries before it returns; waiting for its end as
+        well would keep a step's launches from going out while the step before still runs."""
         for g, entries in enumerate(new_entries):
             if not entries:
                 continue
@@ -103,9 +101,6 @@ class CacheStorage:
             host.numpy()[where[:, 0], where[:, 1]] = where[:, 2]
             lo, hi = int(where[:, 0].min()), int(where[:, 0].max())
             self.tables[g][lo:hi + 1].copy_(host[lo:hi + 1], non_blocking=True)
-            self.tables_in_flight = True
-        if self.tables_in_flight:
-            self.tables_copied.record()
 
     def table_faults(self, book: CacheBook) -> List[str]:
         """Compares the page tables on the device with the bookkeeping: every entry that a

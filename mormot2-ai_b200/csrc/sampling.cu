@@ -331,7 +331,7 @@ sample_cluster_kernel(const float* __restrict__ logits, size_t stride, int V, do
   if (target >= wb && target < wb + ws) {
     double cum = wb;
     // 128 ids at a time, four neighbours a lane, whose loads and exponentials run side by side
-    // (32 at a time the walk was a third of the kernel: 8 rows of 151,936, 39 -> WALK_AFTER us)
+    // (32 at a time the walk was a third of the kernel: 8 rows of 151,936, 39 -> 32 us)
     for (int i0 = w0; i0 < w1; i0 += 128) {
       const int i = i0 + 4 * lane;
       double w[4], incl = 0.0;
