@@ -315,8 +315,9 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
         const float zb = sc[2 * (4 * w + s)], zd = sc[2 * (4 * w + s) + 1];
         dec = s < have ? expf(-expf(par0) * sw_softplus(zd + par1)) : 1.f;
         beta = s < have ? 1.0f / (1.0f + expf(-zb)) : 0.f;
-        fq = g.q_scale / sqrtf(ssq + g.unit_eps);
-        fk = 1.0f / sqrtf(ssk + g.unit_eps);
+        // by choice: the zeros in a missing token's place have no unit length where unit_eps is 0
+        fq = s < have ? g.q_scale / sqrtf(ssq + g.unit_eps) : 0.f;
+        fk = s < have ? 1.0f / sqrtf(ssk + g.unit_eps) : 0.f;
       } else {
         dec = __shfl_sync(0xffffffffu, a_tok, 4 * w + s);
         beta = __shfl_sync(0xffffffffu, b_tok, 4 * w + s);

@@ -127,3 +127,27 @@ def test_an_infinity_does_not_reach_earlier_tokens(mode, bad):
     assert torch.equal(out[:bad], clean[:bad])
     assert torch.equal(out[:, :dim], clean[:, :dim])
     assert not torch.isfinite(out[bad, dim:]).all()
+
+
+# groups that a sequence does not fill, and no floor under the length that keys are divided by
+@pytest.mark.parametrize("lens", [[17], [3, 50], [18, 1, 2], [16, 35]])
+@pytest.mark.parametrize("group", [1, 2])
+def test_delta_without_a_floor_under_the_keys_length(monkeypatch, lens, group):
+    T, heads, dim, vdim = sum(lens), 4, 64, 32
+    qkw, vw = heads // group * dim, heads * vdim
+    z = rows((T, 2 * qkw + 2 * vw + 2 * heads), 1)
+    step = make_step([(i, 5, [0] * n, []) for i, n in enumerate(lens)])
+    start = rows((len(lens), heads * dim * vdim), 2, 0.3)
+    got = []
+    for fours in (False, True):
+        monkeypatch.setattr(K, "walks_by_fours", lambda *a: fours)
+        out, state = torch.empty((T, vw), device=DEV), start.clone()
+        K.linear_state_scan("delta", z, [0, qkw, 2 * qkw], group, z, 2 * qkw + vw,
+                            rows((vdim,), 4, 0.1, 1.0), 1e-6, state, step, out, heads, dim, vdim,
+                            scalars=z, beta_col=2 * qkw + 2 * vw, rate_col=2 * qkw + 2 * vw + heads,
+                            a_log=rows((heads,), 5), dt_bias=rows((heads,), 6, mean=-2.0))
+        got.append((out, state))
+    (want, state), (out, state4) = got
+    # as above: float32 sums in another order
+    assert (out - want).norm() <= 2e-5 * want.norm()
+    assert (state4 - state).norm() <= 2e-6 * state.norm()
