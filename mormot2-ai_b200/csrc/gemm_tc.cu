@@ -34,10 +34,12 @@ MB_DEFINE_LAST_ERROR
 
 static thread_local int g_last_launches = 0;
 static thread_local int g_last_splits = 1;
+static thread_local int g_last_part = 0;
 // of the last mb_gemm_tc of this thread: the splits of K (with `defer` and more than one the partial
 // sums [splits][M][N] were left in the workspace for the caller's next kernel to add) + 256 x the
-// kernels that it launched (2 when K was split and the sums were added up here)
-MB_EXPORT int mb_gemm_tc_last() { return g_last_splits | g_last_launches << 8; }
+// kernels that it launched (2 when K was split and the sums were added up here) + 65,536 x the
+// blocks of 64 values of K that one sum of an accumulator runs over at most
+MB_EXPORT int mb_gemm_tc_last() { return g_last_splits | g_last_launches << 8 | g_last_part << 16; }
 
 // TC_SWIGLU and TC_GEGLU: the weight's rows alternate gate and up and the output is
 // act(gate) * up with act = SiLU or the tanh form of GELU. In these two modes nothing is split,
@@ -484,10 +486,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // warps read the 128 accumulator lanes that landed in its own tensor memory.
 //   full[s]      in rank 0: both CTAs' TMA loads complete their bytes there
 //   empty[s]     in both:   a multicast commit of rank 0's MMA thread frees the stage in both
-//   acc_full[b]  in both:   multicast commit after a tile's last MMA
+//   acc_full[b]  in both:   multicast commit after a tile's (or a part's) last MMA
 //   acc_empty[b] in rank 0: the eight epilogue warps of the pair arrive (rank 1's from afar)
 // The tile's width BN (a multiple of 16 up to 256) is chosen so that the last round of tiles
 // leaves few pairs idle.
+// `kb_per_part`: where it is less than kb_per_split (at most one tile a pair then), no sum runs
+// over more K blocks than that. Part 0 is summed in the first accumulator, the later ones in the
+// others in turn, and the epilogue warps add those to the first, in K's order: the same sums, bit for
+// bit, as partial sums that go through memory, without their traffic. Narrow tiles have room for
+// three or four accumulators, so that a part is added up while the next ones are summed.
 #define TC2_A_HALF (128 * TC_BK * 2)  // one CTA's 128 token rows of a stage
 #define TC2_COLS 256                  // tensor-memory columns of one accumulator
 #define TC2_STAGING (4 * 4096)        // 32 rows x 128 bytes of output for each epilogue warp
@@ -496,6 +503,9 @@ template <int BN> struct Tc2Cfg {
   static constexpr int STAGE = TC2_A_HALF + B_HALF;
   static constexpr int STAGES = (200 * 1024) / STAGE > 8 ? 8 : (200 * 1024) / STAGE;
   static constexpr int SMEM = 1024 + STAGES * STAGE + 1024 + TC2_STAGING;
+  // accumulators where K goes in parts, and the columns from one to the next
+  static constexpr int PARTS = BN <= 128 ? 4 : (BN <= 160 ? 3 : 2);
+  static constexpr int PART_COLS = BN <= 128 ? 128 : (BN <= 160 ? 160 : 256);
 };
 
 // Tile `i` of tiles_m x tiles_n in bands of `band` row tiles: a band's tiles run column after
@@ -507,11 +517,37 @@ __device__ __forceinline__ int2 banded_tile(int i, int tiles_m, int tiles_n, int
   return make_int2(first + r % rows, r / rows);
 }
 
+// This warp's lanes of tensor memory: columns sum .. sum + cols - 1 += more .. (cols: a multiple
+// of 16), 64 columns at a time.
+__device__ __forceinline__ void tmem_add(uint32_t sum, uint32_t more, int cols) {
+  int c = 0;
+#pragma unroll 1
+  for (; c + 64 <= cols; c += 64) {
+    float v[64], m[64];
+    tmem_ld64(sum + c, v);
+    tmem_ld64(more + c, m);
+#pragma unroll
+    for (int j = 0; j < 64; ++j) v[j] += m[j];
+#pragma unroll
+    for (int j = 0; j < 64; j += 16) tmem_st16(sum + c + j, v + j);
+  }
+#pragma unroll 1
+  for (; c < cols; c += 16) {
+    float v[16], m[16];
+    tmem_ld16(sum + c, v);
+    tmem_ld16(more + c, m);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] += m[j];
+    tmem_st16(sum + c, v);
+  }
+  tmem_wait_st();
+}
+
 template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     void* __restrict__ C, int c_dtype, long long ldc, int M, int N, int K,
-                    int kb_per_split, int mode_act, float* __restrict__ partial,
+                    int kb_per_split, int kb_per_part, int mode_act, float* __restrict__ partial,
                     long long partial_stride, long long partial_ld, int tiles_m, int tiles_n,
                     int band, int num_tiles, int* __restrict__ error) {
   const int mode = mode_act & 255, act = mode_act >> 8;
@@ -523,8 +559,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const uint32_t sA = base, sB = base + STAGES * TC2_A_HALF;
   const uint32_t bars = sB + STAGES * Cfg::B_HALF;
   const uint32_t full0 = bars, empty0 = bars + 8 * STAGES;
-  const uint32_t acc_full0 = bars + 16 * STAGES, acc_empty0 = acc_full0 + 16;
-  const uint32_t slot = acc_empty0 + 16;
+  const uint32_t acc_full0 = bars + 16 * STAGES, acc_empty0 = acc_full0 + 32;
+  const uint32_t slot = acc_empty0 + 32;
   volatile uint32_t* slot_ptr = (volatile uint32_t*)(smem_raw + (slot - raw));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -532,13 +568,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int nkb_total = (K + TC_BK - 1) / TC_BK;
   const int tiles_mn = tiles_m * tiles_n;
+  const bool in_parts = kb_per_part < kb_per_split;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < 4; ++b) {
       mbar_init(acc_full0 + 8 * b, 1);
       mbar_init(acc_empty0 + 8 * b, 8);
     }
@@ -592,22 +629,27 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       for (int w = pair; w < num_tiles; w += pairs, ++it) {
         const int kb0 = (w / tiles_mn) * kb_per_split;
         const int nkb = min(kb_per_split, nkb_total - kb0);
-        const int b = it & 1;
-        mbar_wait(acc_empty0 + 8 * b, ((it >> 1) & 1) ^ 1, error, 16);
-        tc_fence_after_sync();
-        const uint32_t acc = tmem + b * TC2_COLS;
-        for (int i = 0; i < nkb; ++i) {
-          mbar_wait(full0 + 8 * s, ph, error, 12);
+        for (int i0 = 0, part = 0; i0 < nkb; i0 += kb_per_part, ++part) {
+          // whole sums: the tiles take turns in two accumulators; parts: see above
+          const int b = !in_parts ? it & 1 : part ? 1 + (part - 1) % (Cfg::PARTS - 1) : 0;
+          const int use = !in_parts ? it >> 1 : part ? (part - 1) / (Cfg::PARTS - 1) : 0;
+          mbar_wait(acc_empty0 + 8 * b, (use & 1) ^ 1, error, 16);
           tc_fence_after_sync();
-          const uint64_t da = umma_desc_k128(sA + s * TC2_A_HALF);
-          const uint64_t db = umma_desc_k128(sB + s * Cfg::B_HALF);
+          const uint32_t acc = tmem + b * (in_parts ? Cfg::PART_COLS : TC2_COLS);
+          const int end = min(nkb, i0 + kb_per_part);
+          for (int i = i0; i < end; ++i) {
+            mbar_wait(full0 + 8 * s, ph, error, 12);
+            tc_fence_after_sync();
+            const uint64_t da = umma_desc_k128(sA + s * TC2_A_HALF);
+            const uint64_t db = umma_desc_k128(sB + s * Cfg::B_HALF);
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k)
-            umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (i | k) != 0);
-          umma_commit_pair(empty0 + 8 * s, 3);
-          if (++s == STAGES) { s = 0; ph ^= 1; }
+            for (int k = 0; k < TC_BK / 16; ++k)
+              umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, i > i0 || k > 0);
+            umma_commit_pair(empty0 + 8 * s, 3);
+            if (++s == STAGES) { s = 0; ph ^= 1; }
+          }
+          umma_commit_pair(acc_full0 + 8 * b, 3);
         }
-        umma_commit_pair(acc_full0 + 8 * b, 3);
       }
     }
   } else {
@@ -619,9 +661,26 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int2 mn = banded_tile(w % tiles_mn, tiles_m, tiles_n, band);
       const int n0 = mn.y * BN;
       const int a = mn.x * 256 + (int)rank * 128 + lane_row;
-      const int b = it & 1;
+      const int b = in_parts ? 0 : it & 1;
       mbar_wait(acc_full0 + 8 * b, (it >> 1) & 1, error, 13);
       tc_fence_after_sync();
+      if (in_parts) {
+        const uint32_t sum = tmem + ((uint32_t)(q * 32) << 16);
+        const int nkb = min(kb_per_split, nkb_total - z * kb_per_split);
+        const int cols = min(BN, (N - n0 + 15) & ~15);
+        for (int i0 = kb_per_part, part = 0; i0 < nkb; i0 += kb_per_part, ++part) {
+          const int p = 1 + part % (Cfg::PARTS - 1);
+          mbar_wait(acc_full0 + 8 * p, (part / (Cfg::PARTS - 1)) & 1, error, 13);
+          tc_fence_after_sync();
+          tmem_add(sum, sum + p * Cfg::PART_COLS, cols);
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            if (rank == 0) mbar_arrive(acc_empty0 + 8 * p);
+            else mbar_arrive_cluster(cluster_addr_of(acc_empty0 + 8 * p, 0));
+          }
+        }
+      }
       const uint32_t taddr = tmem + b * TC2_COLS + ((uint32_t)(q * 32) << 16);
       float* part = partial ? partial + z * partial_stride : nullptr;
       if (staged) {
@@ -728,8 +787,8 @@ static int pair_band(int tiles_m, int K) {
 
 template <int BN>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, int c_dtype,
-                       long long ldc, int M, int N, int K, int kb_per_split, int mode,
-                       float* partial, int tiles_m, int tiles_n, int splits, int pairs,
+                       long long ldc, int M, int N, int K, int kb_per_split, int kb_per_part,
+                       int mode, float* partial, int tiles_m, int tiles_n, int splits, int pairs,
                        int* error, cudaStream_t s) {
   static bool configured = false;
   if (!configured) {
@@ -744,8 +803,8 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, 
   const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
   const int band = pair_band(tiles_m, K);
   mb_launch_pair(gemm_tc_pair_kernel<BN>, dim3(grid), dim3(TC_THREADS), Tc2Cfg<BN>::SMEM, s, tmA,
-                 tmB, C, c_dtype, ldc, M, N, K, kb_per_split, mode, partial, (long long)M * N,
-                 (mode & 255) >= TC_SWIGLU ? limit_bits() : (long long)N, tiles_m, tiles_n, band,
+                 tmB, C, c_dtype, ldc, M, N, K, kb_per_split, kb_per_part, mode, partial,
+                 (long long)M * N, (mode & 255) >= TC_SWIGLU ? limit_bits() : (long long)N, tiles_m, tiles_n, band,
                  num_tiles, error);
   cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) MB_FAIL("mb_gemm_tc (pairs): %s", cudaGetErrorString(le));
@@ -767,13 +826,22 @@ static int pair_tile_width(int N, int tiles_m, int pairs) {
   return best;
 }
 
-// Whether K cut into `splits` pays where a kernel of its own adds the sums up: a tile's K step
-// takes (w + 40) * 1.4 ns; the sums are written, read and added into the output at about 10 TB/s
-// (they lie in L2), after 2 us for the kernel (measured with the products' sizes of 1,024 to
-// 5,120 columns and 160 to 4,096 tokens).
-static bool split_pays(int nkb, int splits, int width, long long outputs) {
-  const double saved = (nkb - (nkb + splits - 1) / splits) * (width + 40) * 1.4e-3;
-  return saved > 2.0 + outputs * 4.0 * (2 * splits + 2) / 1e7;
+// Whether K's parts are summed one after the other by the pair that has the tile, or side by
+// side by several pairs and added up by a kernel of its own; the result is the same, so the rule
+// only weighs times. A tile's K step takes (w + 40) * 1.4 ns and a part's way into the first
+// accumulator 0.3 us; sums that go through memory are written, read and added into the output at
+// about 8 TB/s (they lie in L2; 3 where rows are no whole pieces of 16 bytes), after 1 us for the
+// kernel. 2,048 tokens, 2,048 x 2,048, three parts: 20.0 us in a row, 32.7 through memory (18.1
+// with one sum over all of K, whose error is larger); 512 tokens, 4,096 x 2,048: 13.7 and 20.7
+// (12.7); 256 tokens, 4,096 x 12,288, five parts: 44.2 and 37.1. What the rule takes is within
+// 4 per cent of the better one for 129 to 8,000 tokens, 512 to 6,144 outputs and K of 512 to
+// 12,288 (one size of 240: 17).
+static bool parts_in_row(int nkb, int splits, int tiles, int pairs, int width, int M, int N) {
+  const double step = (width + 40) * 1.4e-3, rate = N % 4 == 0 ? 8e6 : 3e6;
+  const int rounds = (tiles * splits + pairs - 1) / pairs;
+  return nkb * step + (splits - 1) * 0.3 <
+         rounds * ((nkb + splits - 1) / splits) * step + 1.0 +
+             (double)M * N * 4.0 * (2 * splits + 2) / rate;
 }
 
 // C[M, N] = (or +=) the sum over the splits, added in split order
@@ -964,10 +1032,11 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     p.smem += 4 * 4096;  // the epilogue warps' staging rows
     const int tiles = ((rowsA + TC_BM - 1) / TC_BM) * ((rowsB + bn - 1) / bn);
     if (workspace && epilogue < TC_SWIGLU && tiles < sms && nkb >= 8) {
-      // as many splits as fill the device once: each more costs a second round and one more pass
-      // over the output by whoever adds the sums up (4,096 x 4,096, 128 tokens: 9 splits 14.6 us,
-      // 16 splits 21.6; 4,096 x 12,288: 30.7 and 35.0)
-      int want = sms / tiles;
+      // up to two rounds' worth: the shorter the sums of one accumulator, the smaller their error
+      int want = (2 * sms + tiles - 1) / tiles;
+      // sums that stay pending are read once more by their consumer, a full pass over the
+      // output per split: then only as many splits as fill the device once
+      if (defer && want > sms / tiles) want = sms / tiles;
       if (defer && want > TC_MAX_SPLITS) want = TC_MAX_SPLITS;
       if (want > nkb / 4) want = nkb / 4;
       const long long per = (long long)M * N;
@@ -987,20 +1056,21 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     const int tiles = tiles_m * tiles_n;
     p.splits = 1;
     if (workspace && epilogue < TC_SWIGLU && tiles < pairs && nkb >= 8) {
-      // as many splits as fill the pairs once: more give a second round and their sums one more
-      // pass over the output each (4,096 x 12,288, 1,024 tokens: none 77 us, 3 splits 108; 2,048 x
-      // 2,048, 2,048 tokens: none 23, 3 splits 48; 4,096 x 12,288, 160 tokens: none 46, 2 splits 30)
-      int want = pairs / tiles;
+      int want = (2 * pairs + tiles - 1) / tiles;
+      if (defer && want > pairs / tiles) want = pairs / tiles;   // as above
       if (defer && want > TC_MAX_SPLITS) want = TC_MAX_SPLITS;
       if (want > nkb / 4) want = nkb / 4;
       const long long per = (long long)M * N;
       if (want > workspace_floats / per) want = (int)(workspace_floats / per);
-      // sums added up here: only where that costs less than the shorter K loops save
-      while (!defer && want > 1 && !split_pays(nkb, want, bn, per)) --want;
       if (want > 1) p.splits = want;
     }
     p.kb_per_split = (nkb + p.splits - 1) / p.splits;
     p.splits = (nkb + p.kb_per_split - 1) / p.kb_per_split;
+    const int kb_per_part = p.kb_per_split;
+    if (!defer && p.splits > 1 && parts_in_row(nkb, p.splits, tiles, pairs, bn, M, N)) {
+      p.splits = 1;
+      p.kb_per_split = nkb;
+    }
     CUtensorMap tmA, tmB;
     if (!mb_make_map_bf16(&tmA, A, M, K, lda, 128, "mb_gemm_tc input")) return -1;
     if (!mb_make_map_bf16(&tmB, W, N, K, K, bn / 2, "mb_gemm_tc weight")) return -1;
@@ -1010,8 +1080,9 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     switch (bn) {
 #define PAIR(W_)                                                                                \
   case W_:                                                                                      \
-    rc = launch_pair<W_>(tmA, tmB, C, c_dtype, (long long)ldc, M, N, K, p.kb_per_split, mode,   \
-                         partial, tiles_m, tiles_n, p.splits, pairs, error, s);                 \
+    rc = launch_pair<W_>(tmA, tmB, C, c_dtype, (long long)ldc, M, N, K, p.kb_per_split,         \
+                         kb_per_part, mode, partial, tiles_m, tiles_n, p.splits, pairs, error,  \
+                         s);                                                                    \
     break
       PAIR(256); PAIR(240); PAIR(224); PAIR(208); PAIR(192); PAIR(176); PAIR(160); PAIR(144);
       PAIR(128);
@@ -1021,6 +1092,7 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
     if (rc) return rc;
     g_last_launches = (p.splits > 1 && !defer) ? 2 : 1;
     g_last_splits = p.splits;
+    g_last_part = kb_per_part;
     if (p.splits > 1 && !defer)
       return reduce_splits(workspace, p.splits, C, c_dtype, ldc, M, N, epilogue, s);
     return 0;
@@ -1049,6 +1121,7 @@ MB_EXPORT int mb_gemm_tc(const void* A, int lda, const void* W, void* C, int c_d
   if (rc) return rc;
   g_last_launches = (p.splits > 1 && !defer) ? 2 : 1;
   g_last_splits = p.splits;
+  g_last_part = p.kb_per_split;
   if (p.splits > 1 && !defer)
     return reduce_splits(workspace, p.splits, C, c_dtype, ldc, M, N, epilogue, s);
   return 0;

@@ -179,6 +179,59 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 64 consecutive float32 columns of this thread's TMEM lane: four loads in flight, one wait.
+// The loaded registers pass through the wait (and through empty statements after it) so that
+// no use of them can be scheduled before it.
+#define TMEM_LD16(R, OFF)                                                                        \
+  asm volatile(                                                                                  \
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32"                                                   \
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"         \
+      : "=r"(R[0]), "=r"(R[1]), "=r"(R[2]), "=r"(R[3]), "=r"(R[4]), "=r"(R[5]), "=r"(R[6]),      \
+        "=r"(R[7]), "=r"(R[8]), "=r"(R[9]), "=r"(R[10]), "=r"(R[11]), "=r"(R[12]), "=r"(R[13]),  \
+        "=r"(R[14]), "=r"(R[15])                                                                 \
+      : "r"(taddr + OFF))
+#define TMEM_HOLD16(TEXT, R)                                                                     \
+  asm volatile(TEXT                                                                              \
+               : "+r"(R[0]), "+r"(R[1]), "+r"(R[2]), "+r"(R[3]), "+r"(R[4]), "+r"(R[5]),         \
+                 "+r"(R[6]), "+r"(R[7]), "+r"(R[8]), "+r"(R[9]), "+r"(R[10]), "+r"(R[11]),       \
+                 "+r"(R[12]), "+r"(R[13]), "+r"(R[14]), "+r"(R[15])                              \
+               :                                                                                 \
+               : "memory")
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float* v) {
+  uint32_t a[16], b[16], c[16], d[16];
+  TMEM_LD16(a, 0);
+  TMEM_LD16(b, 16);
+  TMEM_LD16(c, 32);
+  TMEM_LD16(d, 48);
+  TMEM_HOLD16("tcgen05.wait::ld.sync.aligned;", a);
+  TMEM_HOLD16("", b);
+  TMEM_HOLD16("", c);
+  TMEM_HOLD16("", d);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    v[i] = __uint_as_float(a[i]);
+    v[16 + i] = __uint_as_float(b[i]);
+    v[32 + i] = __uint_as_float(c[i]);
+    v[48 + i] = __uint_as_float(d[i]);
+  }
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+      ::"r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])),
+        "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
+        "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
+        "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])),
+        "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------- CTA pairs
 // Two CTAs of a cluster (ranks 0 and 1) work on one MMA tile of 256 rows: each holds its 128
 // rows of the first operand and half of the second one's rows in its own shared memory at the

@@ -1402,7 +1402,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, add: bool,
           _ptr(error), sms, _stream())
     # the split of K adds one kernel that sums the partial products
     last = _functions["mb_gemm_tc"][1].mb_gemm_tc_last()
-    Launches.count += (last >> 8) - 1
+    Launches.count += (last >> 8 & 255) - 1
     return last & 255
 
 
