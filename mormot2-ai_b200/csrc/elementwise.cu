@@ -214,13 +214,36 @@ rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ partial, int
   MB_TRACE_END(2);
 }
 
-// 1,024 rows and more of at most 1,024 values (a multiple of 4): a warp a row, row after row, the next row's
-// loads under way while this one is normed; no barrier, and the weights are read once a warp. A
-// block a row spends most of such a row's time on its two barriers and on being placed: 60,865 rows
-// of 1,024: 88 -> 57 us (375 MB), 1,728 rows 3.7 -> 2.9; rows of 2,048 take too many registers (114 us
-// with a block a row, 118 with a warp).
+// N values a lane (4 or 8): each summed over the warp, then the N sums added up. The order is that
+// of block_sum over a block of 8 warps whose warp i holds value i (zeros where N is 4): lanes 16
+// apart first, then 8, 4, 2 and 1, and the warps' sums four, two and one apart. The first rounds
+// halve what a lane keeps.
+template <int N> __device__ __forceinline__ float sum_of_warp_sums(float* v, int lane) {
+  int o = 16;
+#pragma unroll
+  for (int n = N / 2; n > 0; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+#pragma unroll
+  for (o = 16; o > 16 / N; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// 1,024 rows and more of at most 1,024 values (a multiple of 4): a warp a row, row after row, the
+// next row's loads under way while this one is normed; no barrier, and the weights are read once a
+// warp. A block a row spends most of such a row's time on its two barriers and on being placed:
+// 60,865 rows of 1,024: 88 -> 57 us (375 MB), 1,728 rows 3.7 -> 2.9; rows of 2,048 take too many
+// registers (114 us with a block a row, 118 with a warp). The squares are added up in the order of
+// a block a row, so that a row's values do not depend on how many rows there are.
 template <typename TO, int VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 rmsnorm_rows_kernel(const float* __restrict__ x, const void* __restrict__ w, int w_bf16, float eps,
                     TO* __restrict__ y, const int* __restrict__ rows, int R, int H) {
   const int lane = threadIdx.x & 31, step = gridDim.x * 8;
@@ -246,14 +269,14 @@ rmsnorm_rows_kernel(const float* __restrict__ x, const void* __restrict__ w, int
   if (r < R) ask(r);
   for (; r < R; r += step) {
     float4 v[VEC];
-    float sum = 0.f;
+    float sums[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; ++i) v[i] = next[i];
     if (r + step < R) ask(r + step);
 #pragma unroll
     for (int i = 0; i < VEC; ++i)
-      sum = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, sum))));
-    const float inv = 1.0f / sqrtf(warp_sum(sum) / (float)H + eps);
+      sums[i] = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, v[i].w * v[i].w)));
+    const float inv = 1.0f / sqrtf(sum_of_warp_sums<VEC>(sums, lane) / (float)H + eps);
     TO* yr = y + (size_t)r * H;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {

@@ -25,3 +25,18 @@ def test_many_short_rows(R, H, w_dtype, y_dtype, gather):
     # a rounding of the stored type on every value, and float32 sums
     tol = 2.0 ** -8 if y_dtype == "bfloat16" else 2e-6
     assert ((y.double() - want).abs() <= tol * want.abs() + 1e-6).all()
+
+
+# the same sums in the same order whichever form the number of rows takes, so the same values
+@pytest.mark.parametrize("H", [4, 260, 512, 516, 1000, 1024])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_a_rows_values_do_not_depend_on_how_many_there_are(H, dtype):
+    gen = torch.Generator().manual_seed(H)
+    R, dt = 2100, getattr(torch, dtype)
+    x = (torch.randn((R, H), generator=gen) * torch.rand((R, 1), generator=gen).exp()).to(DEV)
+    w = torch.randn((H,), generator=gen).to(dt).to(DEV)
+    got, want = torch.empty((R, H), dtype=dt, device=DEV), torch.empty((R, H), dtype=dt, device=DEV)
+    K.rmsnorm(x, w, 1e-6, got, None, R, None)
+    for r in range(0, R, 700):
+        K.rmsnorm(x[r:r + 700], w, 1e-6, want[r:r + 700], None, 700, None)
+    assert torch.equal(got, want)
