@@ -134,7 +134,6 @@ __host__ __device__ constexpr size_t decode_room(int dim, int vd, int VB) {
 // pages of this split (every `splits`-th page of the sequence) into shared memory, a whole K
 // tile and a whole V tile per page (16 KB each for heads of 128) by bulk asynchronous copies,
 // three pages ahead. Warps 0-3 take 16 keys of every page each.
-#define DEC_SORT ((DEC_WARPS + 1) * 32)   // most tokens of a step whose CTAs are ordered by length
 template <int DB, int VB, bool EXACT, bool CAP>
 __global__ void __launch_bounds__((DEC_WARPS + 1) * 32, 2)
 attn_decode_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restrict__ kpool,
@@ -145,8 +144,7 @@ attn_decode_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restr
                    float* __restrict__ part_ml, bf16* __restrict__ out, int out_stride,
                    int in_clusters, int* __restrict__ error, const float* __restrict__ sink,
                    float cap_log2, const bf16* __restrict__ gate, int gate_stride, int gate_dim,
-                   const float* __restrict__ slopes, int keep_first, int dim_rt, int vd_rt,
-                   int by_length) {
+                   const float* __restrict__ slopes, int keep_first, int dim_rt, int vd_rt) {
   constexpr int CH = DB / 32;  // 32-dim chunks of q·k
   constexpr int OB = VB / 64;  // 64-dim blocks of p·v
   const int dim = EXACT ? DB : dim_rt, vd = EXACT ? VB : vd_rt;
@@ -160,25 +158,7 @@ attn_decode_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restr
   const uint32_t bars = tiles + (uint32_t)decode_room(dim, vd, VB);
   const uint32_t full0 = bars, empty0 = bars + 8 * DEC_STAGES;
 
-  const int s = blockIdx.x, S = gridDim.x;
-  int t = blockIdx.z;
-  if (by_length) {
-    // More CTAs than run at once: the longest sequences must not be the last to start. CTAs start in
-    // the order of blockIdx.z, so z takes the z-th longest sequence, which every CTA finds by itself
-    // (64 sequences of 300 to 2,303 positions, 8 KV heads, two layers of the 8B shape and the head: a step 566 -> 537 us).
-    __shared__ int all_pos[DEC_SORT], chosen;
-    const int n = gridDim.z, i = threadIdx.x;
-    if (i < n) all_pos[i] = tok_pos[i];
-    __syncthreads();
-    if (i < n) {
-      const int mine = all_pos[i];
-      int before = 0;
-      for (int j = 0; j < n; ++j) before += all_pos[j] > mine || (all_pos[j] == mine && j < i);
-      if (before == (int)blockIdx.z) chosen = i;
-    }
-    __syncthreads();
-    t = chosen;
-  }
+  const int s = blockIdx.x, S = gridDim.x, t = blockIdx.z;
   const int G = nh / nkv, subs = (G + 15) / 16;
   const int g = blockIdx.y / subs, sub = blockIdx.y % subs;
   const int h0 = g * G + sub * 16;
@@ -518,8 +498,6 @@ static int decode_launch(const void* q, int q_stride, void* out, int out_stride,
   const float scale_log2 = softcap > 0.f ? 2.f * log2e * scale / softcap : scale * log2e;
   const float cap_log2 = softcap * log2e;
   dim3 grid(splits, nkv * subs, T), mgrid(T, nh);
-  // two CTAs an SM run at once; fewer than that all start together
-  const int by_length = T > 1 && T <= DEC_SORT && (long long)splits * nkv * subs * T > 2 * 148;
 #define GO(D_, V_, X_, CAP_)                                                                   \
   {                                                                                            \
     const int smem = (int)decode_room(hd, vd, V_) + 64;                                        \
@@ -537,14 +515,13 @@ static int decode_launch(const void* q, int q_stride, void* out, int out_stride,
                          (const bf16*)vpool, page_table, max_pages, ring_pages, tok_slot,      \
                          tok_pos, nh, nkv, window, scale_log2, part_o, part_ml, (bf16*)out,    \
                          out_stride, 1, error, sink, cap_log2, (const bf16*)gate, gate_stride, \
-                         gate_dim, slopes, keep_first, hd, vd, by_length);                     \
+                         gate_dim, slopes, keep_first, hd, vd);                                \
     } else {                                                                                   \
       mb_launch(attn_decode_kernel<D_, V_, X_, CAP_>, grid, dim3((DEC_WARPS + 1) * 32), smem, s, \
                 (const bf16*)q, q_stride, (const bf16*)kpool, (const bf16*)vpool, page_table,  \
                 max_pages, ring_pages, tok_slot, tok_pos, nh, nkv, window, scale_log2, part_o, \
                 part_ml, (bf16*)out, out_stride, in_clusters, error, sink, cap_log2,           \
-                (const bf16*)gate, gate_stride, gate_dim, slopes, keep_first, hd, vd,          \
-                by_length);                                                                    \
+                (const bf16*)gate, gate_stride, gate_dim, slopes, keep_first, hd, vd);         \
       if (!in_clusters)                                                                        \
         mb_launch(attn_merge_kernel, mgrid, dim3(vd), 0, s, (const float*)part_o,              \
                   (const float*)part_ml, splits, (bf16*)out, out_stride, nh,                   \

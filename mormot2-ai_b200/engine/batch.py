@@ -35,6 +35,7 @@ class StepContext:
     seq_past: torch.Tensor      # int32 [B] positions held before this pass
     want_rows: torch.Tensor     # int32 [n_want] packed rows whose logits are wanted
     n_want: int
+    entry_slots: torch.Tensor   # int32 [B] seq_slot in the order in which the caller gave them
     max_new: int                # most new tokens of one sequence
     max_len: int                # longest sequence after this pass
     decode: bool                # every sequence brings exactly one token
@@ -55,7 +56,7 @@ class StepBuffers:
 
     def __init__(self, max_tokens: int, max_seqs: int, device: torch.device, guards=None):
         self.max_tokens, self.max_seqs = max_tokens, max_seqs
-        self.size = 5 * max_tokens + 3 * max_seqs + 1
+        self.size = 5 * max_tokens + 4 * max_seqs + 1
         self.host = torch.zeros(self.size, dtype=torch.int32).pin_memory()
         self.host_np = self.host.numpy()      # the same pinned memory, for vectorised filling
         from ..cache.guards import alloc
@@ -64,8 +65,11 @@ class StepBuffers:
         self.in_flight = False
         self.views = {}
 
-    def fill(self, seqs: Sequence[Tuple[int, int, Sequence[int], Sequence[int]]]) -> StepContext:
-        """``seqs = [(slot, past, tokens, want)]``; ``want`` are places among ``tokens``."""
+    def fill(self, seqs: Sequence[Tuple[int, int, Sequence[int], Sequence[int]]],
+             longest_first: bool = False) -> StepContext:
+        """``seqs = [(slot, past, tokens, want)]``; ``want`` are places among ``tokens``.
+        ``longest_first``: a pass of one token a sequence packs the longest first; its wanted
+        rows stay in the order of ``seqs``."""
         B = len(seqs)
         T = sum(len(s[2]) for s in seqs)
         n_want = sum(len(s[3]) for s in seqs)
@@ -78,8 +82,25 @@ class StepBuffers:
         o_slot, o_start, o_past, o_want = 4 * T, 4 * T + B, 4 * T + 2 * B + 1, 4 * T + 3 * B + 1
         n_new = [len(s[2]) for s in seqs]
         total = 4 * T + 3 * B + 1 + n_want
-        if T <= 64:
-            # a decode step or a few tokens: plain lists are quicker than array slices
+        o_entry = o_slot
+        if T == B and min(n_new) == 1:
+            # a decode step: every list is a column of ``seqs``
+            slots, past, ids = [s[0] for s in seqs], [s[1] for s in seqs], [s[2][0] for s in seqs]
+            rows, entries = range(B), []
+            if longest_first and past != sorted(past, reverse=True):
+                entries = slots             # in their own order, behind all else
+                o_entry, total = total, total + B
+                order = sorted(range(B), key=past.__getitem__, reverse=True)
+                slots, past, ids = ([c[i] for i in order] for c in (slots, past, ids))
+                rows = [0] * B              # where a sequence went
+                for row, i in enumerate(order):
+                    rows[i] = row
+            wants = rows if n_want == B == sum(map(bool, (s[3] for s in seqs))) else [
+                row for row, s in zip(rows, seqs) for _ in s[3]]
+            self.host_np[:total] = [*ids, *range(B), *past, *slots, *slots, *range(B + 1), *past,
+                                    *wants, *entries]
+        elif T <= 64:
+            # a few tokens: plain lists are quicker than array slices
             ids: List[int] = []
             seq: List[int] = []
             pos: List[int] = []
@@ -117,17 +138,18 @@ class StepBuffers:
         self.copied.record()
         self.in_flight = True
         # the device views depend on the counts only: made once per shape of step
-        views = self.views.get((T, B, n_want))
+        views = self.views.get((T, B, n_want, o_entry))
         if views is None:
             d = self.dev
             views = (d[o_ids:o_ids + T], d[o_seq:o_seq + T], d[o_pos:o_pos + T],
                      d[o_tslot:o_tslot + T], d[o_slot:o_slot + B], d[o_start:o_start + B + 1],
                      d[o_past:o_past + B], d[o_want:o_want + n_want])
+            views += (views[4] if o_entry == o_slot else d[o_entry:o_entry + B],)
             if len(self.views) < 4096:
-                self.views[(T, B, n_want)] = views
+                self.views[(T, B, n_want, o_entry)] = views
         return StepContext(
             T=T, B=B, tok_ids=views[0], tok_seq=views[1], tok_pos=views[2], tok_slot=views[3],
             seq_slot=views[4], seq_start=views[5], seq_past=views[6], want_rows=views[7],
-            n_want=n_want, max_new=max(n_new),
+            n_want=n_want, entry_slots=views[8], max_new=max(n_new),
             max_len=max(s[1] + len(s[2]) for s in seqs), decode=max(n_new) == 1,
             host_new=n_new, host_past=[s[1] for s in seqs], host_slots=[s[0] for s in seqs])

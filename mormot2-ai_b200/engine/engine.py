@@ -99,6 +99,12 @@ class Engine:
         self.graphs: "OrderedDict[Tuple[int, int], _DecodeGraph]" = OrderedDict()
         self.graph_pool = None                           # one memory pool for all of them
         self.last_h2d_bytes = 0                          # index bytes copied for the last step
+        # The sequences from which on a decode step packs the longest first: with more CTAs of the
+        # attention (one a sequence and KV head at least) than run at once, two a multiprocessor,
+        # they start in the order of the rows, and the long ones must not be the last to start (64
+        # sequences of 300 to 2,303 positions, two layers of the 8B shape and the head: 566 -> 537 us).
+        heads = max((n.kv_heads for n in self.model.line_needs.values()), default=0)
+        self.sort_from = 2 * rt.sms // heads + 1 if heads else 1 << 30
 
     # ------------------------------------------------------------------ making one
     @classmethod
@@ -285,9 +291,12 @@ class Engine:
             self.cache.save_states(touched)
         try:
             for seqs, dest in passes:
-                ctx = self.buffers.fill(seqs)
+                # (``on_state`` is shown the rows as the entries come)
+                ctx = self.buffers.fill(seqs, len(seqs) >= self.sort_from and self.on_state is None)
                 self.last_h2d_bytes += 4 * (4 * ctx.T + 3 * ctx.B + 1 + ctx.n_want)
-                self.last_slots = ctx.seq_slot
+                if ctx.entry_slots is not ctx.seq_slot:
+                    self.last_h2d_bytes += 4 * ctx.B
+                self.last_slots = ctx.entry_slots
                 logits = self._forward(ctx)
                 self.passes += 1
                 if logits is not None:
