@@ -10,6 +10,7 @@ pages are this library's own.
 """
 from __future__ import annotations
 
+import gc
 from collections import OrderedDict
 from dataclasses import dataclass
 from typing import Callable, Dict, List, Optional, Sequence, Tuple
@@ -360,13 +361,20 @@ class Engine:
         """Captures a decode pass. All graphs allocate from one memory pool: one graph runs
         at a time and each is complete in itself (its inputs are the index buffers, the page
         tables and the cache, which lie outside the pool), so the activations of one may lie
-        where those of another lay."""
+        where those of another lay. Python's collector rests meanwhile: what an earlier engine
+        left (pinned buffers with copies behind them) may not be freed under a capture."""
         graph = torch.cuda.CUDAGraph()
         if self.graph_pool is None:
             self.graph_pool = torch.cuda.graph_pool_handle()
         before = K.Launches.count
-        with torch.cuda.graph(graph, pool=self.graph_pool):
-            logits = self.model.forward(ctx, self.cache)
+        collecting = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.graph(graph, pool=self.graph_pool):
+                logits = self.model.forward(ctx, self.cache)
+        finally:
+            if collecting:
+                gc.enable()
         launches = K.Launches.count - before
         K.Launches.count = before                         # capturing launched nothing
         return _DecodeGraph(graph, logits, launches)
