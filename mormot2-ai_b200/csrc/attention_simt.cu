@@ -289,8 +289,9 @@ attention_few_kernel(const AttArgs<T> a, int splits, int chunks) {
       float mx = s;
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float m_new = fmaxf(mine, mx), corr = expf(mine - m_new);
-      const float p = key < cnt ? expf(s - m_new) : 0.f;
+      // a warp's keys so far may all have the score -infinity: they weigh nothing (not 0 / 0)
+      const float m_new = fmaxf(mine, mx), corr = m_new == -INFINITY ? 1.f : expf(mine - m_new);
+      const float p = s == -INFINITY ? 0.f : expf(s - m_new);
       float sum = p;
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

@@ -120,3 +120,37 @@ def test_decode_takes_sequences_by_length(count, splits):
     K.attention_simt(q.float(), nh * hd, want, step, line32, nh, nkv, hd, 0, 0.125)
     # probabilities and outputs rounded to bfloat16, 2^-9 each
     assert ((got.float() - want).norm(dim=1) <= 1e-2 * want.norm(dim=1)).all()
+
+
+# the keys of a whole tile of one warp overflow to -infinity: they weigh nothing, with a sink or none
+@pytest.mark.parametrize("new", [1, 40])
+@pytest.mark.parametrize("first, count", [(0, 16), (16, 16), (32, 64), (0, 127)])
+@pytest.mark.parametrize("sink", [None, 0.5])
+def test_scores_of_minus_infinity(new, first, count, sink):
+    nh, nkv, hd, n = 2, 1, 64, 128
+    rng = np.random.default_rng(first)
+    line = make_line(1, n, nkv, hd, torch.float32)
+    k, v = (torch.tensor(rng.standard_normal((n, nkv, hd)), dtype=torch.float32) for _ in range(2))
+    q = torch.tensor(rng.standard_normal((new, nh * hd)), dtype=torch.float32)
+    k[:, 0, 0], q[:, 0::hd] = 0.0, 1e20
+    k[first:first + count, 0, 0] = -1e20
+    fill_line(line, 0, k, v)
+    sinks = None if sink is None else torch.full((nh,), sink, device=DEV)
+    step = make_step([(0, n - new, [0] * new, [])])
+    out = torch.empty((new, nh * hd), device=DEV)
+    K.attention_simt(q.to(DEV), nh * hd, out, step, line, nh, nkv, hd, 0, 0.125, sink=sinks)
+    ok = [i for i in range(n) if not first <= i < first + count]
+    for row, pos in enumerate(range(n - new, n)):
+        at = [i for i in ok if i <= pos]
+        qd, kd, vd = q[row].view(nh, hd).double(), k[at, 0].double(), v[at, 0].double()
+        s = qd @ kd.t() * 0.125
+        if sinks is not None:
+            s = torch.cat([s, torch.full((nh, 1), sink, dtype=torch.float64)], 1)
+            vd = torch.cat([vd, torch.zeros((1, hd), dtype=torch.float64)])
+        got = out[row].view(nh, hd).double().cpu()
+        if s.shape[1] == 0:                 # nothing to weigh: 0 / 0
+            assert torch.isnan(got).all()
+            continue
+        want = torch.softmax(s, 1) @ vd
+        # float32 sums of at most 128 terms; the product with 1e20 leaves q·k of the others whole
+        assert (got - want).norm() <= 4e-6 * want.norm() + 1e-12
