@@ -403,9 +403,12 @@ static int launch_few(const AttArgs<T>& a, int tokens, int sms, cudaStream_t s) 
   const dim3 grid(tokens * splits, a.nkv * chunks);
 #define GO(R_, W_)                                                                             \
   {                                                                                            \
-    if (smem > 48 * 1024)                                                                      \
-      cudaFuncSetAttribute(attention_few_kernel<T, R_, W_>,                                    \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
+    if (smem > 48 * 1024) { /* heads of 256 and eight to a KV head: 53 KB */                   \
+      static unsigned long long allowed = 0;                                                   \
+      const cudaError_t e =                                                                    \
+          mb_allow_smem((const void*)attention_few_kernel<T, R_, W_>, 56 * 1024, &allowed);    \
+      if (e != cudaSuccess) MB_FAIL("mb_attention_simt: %s", cudaGetErrorString(e));           \
+    }                                                                                          \
     mb_launch_clusters(attention_few_kernel<T, R_, W_>, grid, dim3(ATF_WARPS * 32), smem, s,   \
                        splits, a, splits, chunks);                                             \
   }
@@ -420,9 +423,10 @@ static int launch_few(const AttArgs<T>& a, int tokens, int sms, cudaStream_t s) 
 // 64 new tokens of one sequence and one head per CTA, a page of 64 keys at a time through shared
 // memory: it is float32 multiply-adds that bound it, and a tile of 64 x 64 scores gives each of
 // 256 threads 4 x 4 of them (every value read from shared memory serves four multiply-adds) and
-// 4 x 8 values of the output (128 threads with twice the rows take 385 us where these take 335: too few warps). Rows of q and k keep their order in shared memory (pitch hd + 4: a
-// warp's 16 keys lie on different banks) and are read four values along the head at a time. K and
-// V take turns in one tile, so that two CTAs fit an SM and one computes while the other loads.
+// 4 x 8 values of the output (128 threads with twice the rows take 385 us where these take 335: too
+// few warps). Rows of q and k keep their order in shared memory (pitch hd + 4: a warp's 16 keys lie
+// on different banks) and are read four values along the head at a time. K and V take turns in one
+// tile, so that two CTAs fit an SM and one computes while the other loads.
 // Before, a warp walked a (token, head) alone: 1,728 tokens of three prompts (16 heads on 8 of
 // 128 values, float32) took 1,907 us; now 335 (17 TFLOP/s).
 #define ATM_ROWS 64
@@ -600,14 +604,11 @@ template <typename T>
 static int launch_many(const AttArgs<T>& a, int B, int max_new, cudaStream_t s) {
   const int pitch = a.hd + 4, kv_pitch = pitch > a.vd ? pitch : a.vd;
   const size_t smem = (size_t)ATM_ROWS * (pitch + kv_pitch + ATM_PITCH) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {      // heads of 128: 85 KB
-    cudaFuncSetAttribute(attention_many_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         88 * 1024);
-    configured = true;
-  }
-  mb_launch(attention_many_kernel<T>, dim3(a.nh, (max_new + ATM_ROWS - 1) / ATM_ROWS, B), dim3(ATM_THREADS),
-            smem, s, a);
+  static unsigned long long allowed = 0;      // heads of 128: 85 KB
+  const cudaError_t e = mb_allow_smem((const void*)attention_many_kernel<T>, 88 * 1024, &allowed);
+  if (e != cudaSuccess) MB_FAIL("mb_attention_simt: %s", cudaGetErrorString(e));
+  mb_launch(attention_many_kernel<T>, dim3(a.nh, (max_new + ATM_ROWS - 1) / ATM_ROWS, B),
+            dim3(ATM_THREADS), smem, s, a);
   MB_CHECK_LAUNCH("mb_attention_simt");
 }
 

@@ -59,6 +59,19 @@ static cudaError_t mb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// Lets `kernel` take up to `bytes` of dynamic shared memory on the current device, once for each
+// device of the process (`done`: a bit a device, from zero).
+static inline cudaError_t mb_allow_smem(const void* kernel, int bytes, unsigned long long* done) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = device < 64 ? 1ull << device : 0;
+  if (__atomic_load_n(done, __ATOMIC_ACQUIRE) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) __atomic_fetch_or(done, bit, __ATOMIC_RELEASE);
+  return e;
+}
+
 // The same with the CTAs of the grid's x direction in clusters of `cluster_x` (which divides it).
 template <typename... KArgs, typename... Args>
 static cudaError_t mb_launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -386,19 +386,9 @@ gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ 
   cluster.sync();      // nobody leaves while its sums are still read
 }
 
-static int sm_count() {
-  static const int n = [] {
-    int device = 0, count = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-    return count;
-  }();
-  return n;
-}
-
 template <typename TA, typename TW>
 static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, int ldc, int M, int N,
-                  int K, int epi, cudaStream_t s) {
+                  int K, int epi, int sms, cudaStream_t s) {
   // few rows, and every row piece of 4 values a whole aligned load
   const int a_align = sizeof(TA) == 4 ? 15 : 7, w_align = sizeof(TW) == 4 ? 15 : 7;
   if (M <= FEW_MAX && K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A & a_align) == 0 &&
@@ -428,7 +418,7 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
     const int vec_w = K % 4 == 0 && ((uintptr_t)W & w_align) == 0;
     // splits of K, at least 128 values each: what a multiprocessor has to do in units of one whole
     // tile, where fewer than three CTAs take as long as three
-    const int tiles = tiles_n * tiles_m, sms = sm_count();
+    const int tiles = tiles_n * tiles_m;
     int splits = 1;
     double best = 1e30;
     for (int n = 1; n <= 8 && (n == 1 || K >= 128 * n); ++n) {
@@ -458,10 +448,10 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
 }
 
 // C[M, N] (row stride ldc) = A[M, K] (row stride lda) · W[N, K]ᵀ. For EPI_ADD, C must be
-// float32. For the SwiGLU epilogues, W is [2N, K].
+// float32. For the SwiGLU epilogues, W is [2N, K]. `sms`: the number of SMs of the device.
 MB_EXPORT int mb_gemm_simt(const void* A, int a_dtype, int lda, const void* W, int w_dtype,
                            void* C, int c_dtype, int ldc, int M, int N, int K, int epilogue,
-                           void* stream) {
+                           int sms, void* stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) MB_FAIL("mb_gemm_simt: K = %d", K);
   if (epilogue < 0 || epilogue > 3) MB_FAIL("mb_gemm_simt: epilogue %d", epilogue);
@@ -470,8 +460,8 @@ MB_EXPORT int mb_gemm_simt(const void* A, int a_dtype, int lda, const void* W, i
   typedef __nv_bfloat16 bf;
   const int c_bf16 = c_dtype == MB_BF16;
   if (a_dtype == MB_F32 && w_dtype == MB_F32)
-    return launch<float, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, s);
-  if (a_dtype == MB_F32) return launch<float, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, s);
-  if (w_dtype == MB_F32) return launch<bf, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, s);
-  return launch<bf, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, s);
+    return launch<float, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
+  if (a_dtype == MB_F32) return launch<float, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
+  if (w_dtype == MB_F32) return launch<bf, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
+  return launch<bf, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
 }

@@ -468,13 +468,13 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
 // out[t, h, :] for the new tokens of B sequences. q [T, nh * (dim + rot_dim)] with its rotated
 // parts turned; kv [R, nh * (dim + vd)]: the gathered rows' keys of all heads, then their values;
 // rot [R, 64]; gate (may be null) [T, >= nh * vd]. `error`: a device word that receives 9..19 if
-// a wait in the kernel ran out.
+// a wait in the kernel ran out. `sms`: the number of SMs of the device.
 MB_EXPORT int mb_latent_prefill_tc(const void* q, int q_stride, const void* kv, int kv_stride,
                                    const void* rot, int R, void* out, int out_stride,
                                    const int* seq_start, const int* seq_past, int B, int T,
                                    int max_new, int nh, int dim, int rot_dim, int vd, int window,
                                    float scale, int* error, const void* gate, int gate_stride,
-                                   void* stream) {
+                                   int sms, void* stream) {
   if (B <= 0 || max_new <= 0) return 0;
   const char* who = "mb_latent_prefill_tc";
   if ((dim != 64 && dim != 128) || (vd != 64 && vd != 128) || rot_dim < 0 || rot_dim > 64 || rot_dim % 8)
@@ -491,12 +491,6 @@ MB_EXPORT int mb_latent_prefill_tc(const void* q, int q_stride, const void* kv, 
   if (!mb_make_map_bf16(&tmKV, kv, R, (long long)nh * (dim + vd), kv_stride, MB_PAGE, who)) return -1;
   if (!mb_make_map_bf16(&tmR, rot, R, 64, 64, MB_PAGE, who)) return -1;
   dim3 grid(nh, row_tiles, B);
-  static const int sms = [] {
-    int device = 0, n = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
-    return n;
-  }();
   const int apart = window <= 0 && (long long)nh * row_tiles * B <= sms;
 #define GO(DH_, VH_)                                                                           \
   {                                                                                            \

@@ -942,12 +942,10 @@ MB_EXPORT int mb_sample_filtered(const float* logits, long long stride, int rows
     const bool held = share <= SAMPLE_HELD;
     auto* kernel = held ? sample_filtered_cluster_kernel<true> : sample_filtered_cluster_kernel<false>;
     const size_t smem = held ? (size_t)share * sizeof(float) : 0;
-    static bool configured = false;
-    if (!configured) {
-      cudaFuncSetAttribute(sample_filtered_cluster_kernel<true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_HELD * (int)sizeof(float));
-      configured = true;
-    }
+    static unsigned long long allowed = 0;
+    const cudaError_t e = mb_allow_smem((const void*)sample_filtered_cluster_kernel<true>,
+                                        SAMPLE_HELD * (int)sizeof(float), &allowed);
+    if (e != cudaSuccess) MB_FAIL("mb_sample_filtered: %s", cudaGetErrorString(e));
     mb_launch_clusters(kernel, dim3(rows * SAMPLE_CTAS),
                        dim3(SAMPLE_CL_THREADS), smem, (cudaStream_t)stream, SAMPLE_CTAS, logits,
                        (size_t)stride, V, 1.0 / temperature, top_k, top_p, min_p, state_index,

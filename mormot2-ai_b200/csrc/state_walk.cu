@@ -654,12 +654,10 @@ MB_EXPORT int mb_state_walk(const WalkArgs* args, int sms, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
 #define GO(M_, R_)                                                                             \
   {                                                                                            \
-    static bool configured = false;                                                            \
-    if (!configured) {                                                                         \
-      cudaFuncSetAttribute(state_walk_kernel<M_, R_>,                                          \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);           \
-      configured = true;                                                                       \
-    }                                                                                          \
+    static unsigned long long allowed = 0;                                                     \
+    const cudaError_t e =                                                                      \
+        mb_allow_smem((const void*)state_walk_kernel<M_, R_>, 224 * 1024, &allowed);           \
+    if (e != cudaSuccess) MB_FAIL("mb_state_walk: %s", cudaGetErrorString(e));                 \
     mb_launch(state_walk_kernel<M_, R_>, grid, dim3(threads + 8 * CT), smem, s, g, P, CW, CT); \
   }
 #define GOR(M_) if (R == 8) GO(M_, 8) else GO(M_, 16)

@@ -55,7 +55,7 @@ def _sms_of(device: int) -> int:
 
 def _sms() -> int:
     """How many multiprocessors the current device has."""
-    return _sms_of(torch.cuda.current_device())
+    return _sms_of(torch._C._cuda_getDevice())
 
 
 def require_gpu() -> None:
@@ -1029,11 +1029,11 @@ def latent_prefill_tc(q: torch.Tensor, kv: torch.Tensor, rot: torch.Tensor, out:
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1)
     _call("latent_tc", "mb_latent_prefill_tc",
           [_vp, _i, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp,
-           _vp, _i, _vp],
+           _vp, _i, _i, _vp],
           _ptr(q), q.stride(0), _ptr(kv), kv.stride(0), _ptr(rot), kv.shape[0], _ptr(out),
           out.stride(0), _ptr(step.seq_start), _ptr(step.seq_past), step.B, T, step.max_new, nh,
           dim, rot_dim, vd, window, float(scale), _ptr(error), _ptr(gate),
-          gate.stride(0) if gate is not None else 0, _stream())
+          gate.stride(0) if gate is not None else 0, _sms(), _stream())
 
 
 # ------------------------------------------------------------------------------ routed experts
@@ -1306,9 +1306,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int =
     assert c.shape[0] == M and a.stride(1) == 1 and c.stride(1) == 1
     _contig(w, "the weight")
     _call("gemm_simt", "mb_gemm_simt",
-          [_vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp],
+          [_vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
           _ptr(a), code_of(a.dtype), a.stride(0), _ptr(w), code_of(w.dtype), _ptr(c),
-          code_of(c.dtype), c.stride(0), M, N, K, epilogue, _stream())
+          code_of(c.dtype), c.stride(0), M, N, K, epilogue, _sms(), _stream())
 
 
 # ------------------------------------------------------------------------------ attention
