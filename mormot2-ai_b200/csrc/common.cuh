@@ -35,9 +35,14 @@ static thread_local char g_mb_error[512];
 // Programmatic dependent launch: a kernel launched through mb_launch may be scheduled while the
 // kernel before it in the stream is still draining; it must call mb_grid_wait() before it
 // touches global memory (the wait returns when the kernels before have completed and their
-// writes are visible). Every kernel that is launched this way waits at its very top, on every
-// path, so that completion stays transitive along a chain of kernels. mb_grid_launch_next()
-// lets the next kernel's CTAs be placed as soon as all CTAs of this one have started.
+// writes are visible). Every kernel that is launched this way waits on every path before it lets
+// its successor start, so that completion stays transitive along a chain of kernels: whatever the
+// kernels before the one before wrote is settled when a kernel begins. Ahead of its wait a
+// kernel may read such settled memory only, and says so: the weights of products in the decode form
+// and of norms, a step's index arrays, pages of the cache that the step does not write. A weight
+// that the kernel just before it writes must not be handed to these; products in float32 read
+// theirs early only if the caller says that it is settled. mb_grid_launch_next() lets the next
+// kernel's CTAs be placed as soon as all CTAs of this one have started.
 __device__ __forceinline__ void mb_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mb_grid_launch_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

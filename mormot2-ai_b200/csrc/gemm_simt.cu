@@ -146,7 +146,8 @@ __device__ __forceinline__ float sum32_by_lane(float* v, int lane) {
 template <typename TA, typename TW, int EPI>
 __global__ void __launch_bounds__(256, 2)
 gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
-                     void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K, int KW) {
+                     void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K, int KW,
+                     int settled) {
   constexpr bool GLU = EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_PAIRS;
   constexpr int FEATS = GLU ? 2 : 4;  // output features of a warp
   __shared__ float part[8][32];
@@ -169,9 +170,11 @@ gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
     for (int j = 0; j < 4; ++j)
       next[j] = k < K ? load4_once<TW>(wr[j] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  ask(k_first);      // weights depend on no earlier kernel
+  // the first chunk ahead of the wait, where the kernel before does not write the weight
+  if (settled) ask(k_first);
   mb_grid_wait();
   mb_grid_launch_next();
+  if (!settled) ask(k_first);
   for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
     float acc[4 * FEW_ROWS];
 #pragma unroll
@@ -388,7 +391,7 @@ gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ 
 
 template <typename TA, typename TW>
 static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, int ldc, int M, int N,
-                  int K, int epi, int sms, cudaStream_t s) {
+                  int K, int epi, int settled, int sms, cudaStream_t s) {
   // few rows, and every row piece of 4 values a whole aligned load
   const int a_align = sizeof(TA) == 4 ? 15 : 7, w_align = sizeof(TW) == 4 ? 15 : 7;
   if (M <= FEW_MAX && K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A & a_align) == 0 &&
@@ -402,7 +405,7 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
     const int blocks = (groups + 8 / kw - 1) / (8 / kw);
 #define FEW(E)                                                                                \
   mb_launch(gemm_few_rows_kernel<TA, TW, E>, dim3(blocks), dim3(256), 0, s, (const TA*)A, lda, \
-            (const TW*)W, C, c_bf16, ldc, M, N, K, kw)
+            (const TW*)W, C, c_bf16, ldc, M, N, K, kw, settled)
     if (epi == EPI_STORE) FEW(EPI_STORE);
     else if (epi == EPI_ADD) FEW(EPI_ADD);
     else if (epi == EPI_SWIGLU) FEW(EPI_SWIGLU);
@@ -448,10 +451,12 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
 }
 
 // C[M, N] (row stride ldc) = A[M, K] (row stride lda) · W[N, K]ᵀ. For EPI_ADD, C must be
-// float32. For the SwiGLU epilogues, W is [2N, K]. `sms`: the number of SMs of the device.
+// float32. For the SwiGLU epilogues, W is [2N, K]. `settled`: W was not written by the kernel just
+// before in the stream, so that reading it need not wait for that kernel. `sms`: the number of SMs
+// of the device.
 MB_EXPORT int mb_gemm_simt(const void* A, int a_dtype, int lda, const void* W, int w_dtype,
                            void* C, int c_dtype, int ldc, int M, int N, int K, int epilogue,
-                           int sms, void* stream) {
+                           int settled, int sms, void* stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) MB_FAIL("mb_gemm_simt: K = %d", K);
   if (epilogue < 0 || epilogue > 3) MB_FAIL("mb_gemm_simt: epilogue %d", epilogue);
@@ -460,8 +465,8 @@ MB_EXPORT int mb_gemm_simt(const void* A, int a_dtype, int lda, const void* W, i
   typedef __nv_bfloat16 bf;
   const int c_bf16 = c_dtype == MB_BF16;
   if (a_dtype == MB_F32 && w_dtype == MB_F32)
-    return launch<float, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
-  if (a_dtype == MB_F32) return launch<float, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
-  if (w_dtype == MB_F32) return launch<bf, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
-  return launch<bf, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, sms, s);
+    return launch<float, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, settled, sms, s);
+  if (a_dtype == MB_F32) return launch<float, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, settled, sms, s);
+  if (w_dtype == MB_F32) return launch<bf, float>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, settled, sms, s);
+  return launch<bf, bf>(A, lda, W, C, c_bf16, ldc, M, N, K, epilogue, settled, sms, s);
 }

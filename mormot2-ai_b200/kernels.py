@@ -1296,9 +1296,12 @@ def attention_diff_prefill_tc(q: torch.Tensor, out: torch.Tensor, step, line, nh
 
 
 # ------------------------------------------------------------------------------ products
-def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPI_STORE) -> None:
+def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPI_STORE,
+              settled: bool = False) -> None:
     """c = a · wᵀ (store), c += a · wᵀ (add, float32 c), or SwiGLU over w = [gate; up]
-    (EPI_SWIGLU) or over a w whose rows alternate gate, up (EPI_SWIGLU_PAIRS)."""
+    (EPI_SWIGLU) or over a w whose rows alternate gate, up (EPI_SWIGLU_PAIRS). ``settled``: w is a
+    bound weight, which the kernel just before in the stream does not write, and may be read
+    before that kernel has ended."""
     M, K = a.shape
     N = c.shape[1]
     assert w.shape[1] == K
@@ -1306,9 +1309,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int =
     assert c.shape[0] == M and a.stride(1) == 1 and c.stride(1) == 1
     _contig(w, "the weight")
     _call("gemm_simt", "mb_gemm_simt",
-          [_vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
+          [_vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
           _ptr(a), code_of(a.dtype), a.stride(0), _ptr(w), code_of(w.dtype), _ptr(c),
-          code_of(c.dtype), c.stride(0), M, N, K, epilogue, _sms(), _stream())
+          code_of(c.dtype), c.stride(0), M, N, K, epilogue, int(settled), _sms(), _stream())
 
 
 # ------------------------------------------------------------------------------ attention

@@ -80,12 +80,13 @@ class Linear:
             raise KernelError("a gated epilogue with a bias or another activation than SiLU "
                               "needs bfloat16 operands on 16-byte boundaries")
         if add_into is not None:
-            K.gemm_simt(a, self.weight, add_into, K.EPI_ADD)
+            K.gemm_simt(a, self.weight, add_into, K.EPI_ADD, settled=True)
             return add_into
         if self.unary is not None:
             z = torch.empty_like(out)
-            K.gemm_simt(a, self.weight, z, K.EPI_STORE)
+            K.gemm_simt(a, self.weight, z, K.EPI_STORE, settled=True)
             K.unary_act(z, out, self.unary)
             return out
-        K.gemm_simt(a, self.weight, out, K.EPI_SWIGLU_PAIRS if self.swiglu else K.EPI_STORE)
+        K.gemm_simt(a, self.weight, out, K.EPI_SWIGLU_PAIRS if self.swiglu else K.EPI_STORE,
+                    settled=True)
         return out
