@@ -233,6 +233,38 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// v[i] summed over the warp's lanes, value i's sum in lane i: every round halves what a lane keeps.
+__device__ __forceinline__ float sum32_by_lane(float* v, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+
+// Two float32 values side by side in 64 bits, and arithmetic on both at once (each half is rounded
+// as a single value would be)
+typedef unsigned long long f32_pair;
+__device__ __forceinline__ f32_pair pair_of(float a, float b) {
+  f32_pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float pair_half(f32_pair v, int h) {
+  return __uint_as_float((unsigned)(v >> (32 * h)));
+}
+__device__ __forceinline__ void pair_fma(f32_pair& s, f32_pair a, f32_pair b) {   // s += a b
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void pair_mul(f32_pair& s, f32_pair a) {
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(s) : "l"(a));
+}
+
 // The sum over the split sums of one element: p[0] + p[stride] + ... (parts of them), added in
 // that order, with up to eight loads in flight at once (a loop of dependent loads would wait a
 // trip to memory for each).

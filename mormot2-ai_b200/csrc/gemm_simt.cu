@@ -129,20 +129,6 @@ template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __
 #define FEW_ROWS 8   // rows of A in one pass
 #define FEW_MAX 16   // the most rows that take this kernel
 
-// v[i] summed over the warp's lanes, value i's sum in lane i: every round halves what a lane keeps.
-__device__ __forceinline__ float sum32_by_lane(float* v, int lane) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  return v[0];
-}
-
 template <typename TA, typename TW, int EPI>
 __global__ void __launch_bounds__(256, 2)
 gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
@@ -253,16 +239,6 @@ __device__ __forceinline__ float4 row_piece(const T* __restrict__ base, bool row
   return v;
 }
 
-__device__ __forceinline__ void fma_pair(unsigned long long& s, unsigned long long a,
-                                         unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long twice(float v) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-  return r;
-}
-
 template <typename TA, typename TW, int EPI>
 __global__ void __launch_bounds__(64, 4)
 gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
@@ -280,7 +256,7 @@ gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ 
   const int lr = tid / PER, lk = 4 * (tid % PER);
   const int ty = tid >> 4, tx = tid & 15;
   // rows 16 g + 4 ty + (0 .. 3), two a pair; columns 64 h + 4 tx + (0 .. 3)
-  unsigned long long acc[8][8];
+  f32_pair acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -332,11 +308,12 @@ gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ 
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float4 bq = b[j >> 2];
-        const unsigned long long bb = twice((j & 3) == 0 ? bq.x : ((j & 3) == 1 ? bq.y : ((j & 3) == 2 ? bq.z : bq.w)));
+        const float bj = (j & 3) == 0 ? bq.x : ((j & 3) == 1 ? bq.y : ((j & 3) == 2 ? bq.z : bq.w));
+        const f32_pair bb = pair_of(bj, bj);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-          fma_pair(acc[2 * g][j], a[g].x, bb);
-          fma_pair(acc[2 * g + 1][j], a[g].y, bb);
+          pair_fma(acc[2 * g][j], a[g].x, bb);
+          pair_fma(acc[2 * g + 1][j], a[g].y, bb);
         }
       }
     }
@@ -346,7 +323,6 @@ gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ 
       cur ^= 1;
     }
   }
-  auto half = [](unsigned long long v, int h) { return __uint_as_float((unsigned)(v >> (32 * h))); };
   // four neighbouring columns of a row
   auto finish = [&](int gm, int gn, float4 v) {
     if (gm >= M) return;
@@ -369,8 +345,9 @@ gemm_many_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ 
     const int row = 16 * (i >> 2) + 4 * ty + (i & 3);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const unsigned long long* p = acc[i >> 1] + 4 * h;
-      const float4 v = make_float4(half(p[0], i & 1), half(p[1], i & 1), half(p[2], i & 1), half(p[3], i & 1));
+      const f32_pair* p = acc[i >> 1] + 4 * h;
+      const float4 v = make_float4(pair_half(p[0], i & 1), pair_half(p[1], i & 1),
+                                   pair_half(p[2], i & 1), pair_half(p[3], i & 1));
       if (splits == 1) finish(m0 + row, n0 + 64 * h + 4 * tx, v);
       else *(float4*)(sm + row * LN + 64 * h + 4 * tx) = v;
     }

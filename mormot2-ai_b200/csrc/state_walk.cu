@@ -83,36 +83,7 @@ template <int BYTES> __device__ __forceinline__ void sw_copy(float* dst, const f
 __device__ __forceinline__ void sw_prep_sync(int threads) {
   asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
-typedef unsigned long long sw_pair;     // two neighbouring rows' values
-__device__ __forceinline__ void sw_fma(sw_pair& s, sw_pair a, sw_pair b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ void sw_mul(sw_pair& s, sw_pair a) {
-  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(s) : "l"(a));
-}
-__device__ __forceinline__ sw_pair sw_both(float a, float b) {
-  sw_pair r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float sw_added(sw_pair v) {
-  return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
-}
-__device__ __forceinline__ float sw_half(sw_pair v, int h) { return __uint_as_float((unsigned)(v >> (32 * h))); }
-
-// v[i] summed over the warp's lanes, value i's sum in lane i
-__device__ __forceinline__ float sw_sum32(float* v, int lane) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  return v[0];
-}
+__device__ __forceinline__ float sw_added(f32_pair v) { return pair_half(v, 0) + pair_half(v, 1); }
 
 // Shared memory: three buffers [q | k | decays (gla, wkv)] of 16 x DP + 16 x CW of v + 16 x 2
 // logits; two of coefficients; two of 16 x CW outputs. mlstm: block z = NS has the one column of
@@ -302,7 +273,7 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
           }
         }
       }
-      const float sum = sw_sum32(sums, lane);
+      const float sum = sum32_by_lane(sums, lane);
       const int t = (lane >> 2) & 3, s = lane & 3;
       const float qk = __shfl_sync(0xffffffffu, sum, t * (t + 1) / 2 + min(s, t));
       if (CHANNEL) {
@@ -404,14 +375,14 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
   const int j = 2 * (threadIdx.x / P), p = threadIdx.x % P, hc = P >> 1;
   const bool second = p & hc;
   const int mine = j + (second ? 1 : 0), pl = p & (hc - 1), my_t = pl & 3;
-  sw_pair S[2][R / 2];
+  f32_pair S[2][R / 2];
 #pragma unroll
   for (int c = 0; c < 2; ++c)
 #pragma unroll
     for (int r = 0; r < R / 2; ++r) {
       const int i = p * R + 2 * r;
       const bool own = j + c < cw;
-      S[c][r] = sw_both(own && i < D ? Sg[(size_t)i * s_row + j + c] : 0.f,
+      S[c][r] = pair_of(own && i < D ? Sg[(size_t)i * s_row + j + c] : 0.f,
                         own && i + 1 < D ? Sg[(size_t)(i + 1) * s_row + j + c] : 0.f);
     }
   __syncthreads();
@@ -446,7 +417,7 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
         if (MODE == WALK_MLSTM) em = co[SW_EM + my_t];
       }
       const float4 nn = *(const float4*)(co + SW_N + 4 * my_t);
-      sw_pair rd[4][2], pd[4][2];
+      f32_pair rd[4][2], pd[4][2];
 #pragma unroll
       for (int t = 0; t < 4; ++t) rd[t][0] = rd[t][1] = pd[t][0] = pd[t][1] = 0ull;
 #pragma unroll
@@ -456,15 +427,15 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
           const ulonglong2 q = *(const ulonglong2*)(qb + t * DP + 2 * r);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            sw_fma(rd[t][c], S[c][r], q.x);
-            sw_fma(rd[t][c], S[c][r + 1], q.y);
+            pair_fma(rd[t][c], S[c][r], q.x);
+            pair_fma(rd[t][c], S[c][r + 1], q.y);
           }
           if (MODE == WALK_DELTA) {
             const ulonglong2 k = *(const ulonglong2*)(kb + t * DP + 2 * r);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-              sw_fma(pd[t][c], S[c][r], k.x);
-              sw_fma(pd[t][c], S[c][r + 1], k.y);
+              pair_fma(pd[t][c], S[c][r], k.x);
+              pair_fma(pd[t][c], S[c][r + 1], k.y);
             }
           }
         }
@@ -494,23 +465,23 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
 #pragma unroll
         for (int t = 0; t < 4; ++t) other[t] = __shfl_xor_sync(0xffffffffu, x[t], hc);
       }
-      sw_pair xp[4][2];
+      f32_pair xp[4][2];
       {
         const float h[4] = {CHANNEL ? 1.f : h4.x, CHANNEL ? 1.f : h4.y, CHANNEL ? 1.f : h4.z,
                             CHANNEL ? 1.f : h4.w};
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const float a = h[t] * (second ? other[t] : x[t]), b = h[t] * (second ? x[t] : other[t]);
-          xp[t][0] = sw_both(a, a);
-          xp[t][1] = sw_both(b, b);
+          xp[t][0] = pair_of(a, a);
+          xp[t][1] = pair_of(b, b);
         }
       }
       if (!CHANNEL) {
-        const sw_pair A = sw_both(A1, A1);
+        const f32_pair A = pair_of(A1, A1);
 #pragma unroll
         for (int r = 0; r < R / 2; ++r) {
-          sw_mul(S[0][r], A);
-          sw_mul(S[1][r], A);
+          pair_mul(S[0][r], A);
+          pair_mul(S[1][r], A);
         }
       } else {
         const float* ab = kb + CT * DP;
@@ -519,8 +490,8 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
           const ulonglong2 a = *(const ulonglong2*)(ab + 2 * r);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            sw_mul(S[c][r], a.x);
-            sw_mul(S[c][r + 1], a.y);
+            pair_mul(S[c][r], a.x);
+            pair_mul(S[c][r + 1], a.y);
           }
         }
       }
@@ -531,8 +502,8 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
           const ulonglong2 k = *(const ulonglong2*)(kb + t * DP + 2 * r);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            sw_fma(S[c][r], k.x, xp[t][c]);
-            sw_fma(S[c][r + 1], k.y, xp[t][c]);
+            pair_fma(S[c][r], k.x, xp[t][c]);
+            pair_fma(S[c][r + 1], k.y, xp[t][c]);
           }
         }
       // the outputs, a token a lane (a column's two lanes, P = 4, have two each)
@@ -559,7 +530,7 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int i = p * R + r;
-      if (j + c < cw && i < D) Sg[(size_t)i * s_row + j + c] = sw_half(S[c][r >> 1], r & 1);
+      if (j + c < cw && i < D) Sg[(size_t)i * s_row + j + c] = pair_half(S[c][r >> 1], r & 1);
     }
 }
 
