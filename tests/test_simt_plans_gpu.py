@@ -40,3 +40,18 @@ def test_swiglu(M, N, Kd, pairs):
     K.gemm_simt(a, w, out, K.EPI_SWIGLU_PAIRS if pairs else K.EPI_SWIGLU)
     # float32 sums of up to 2,048 terms: the error grows with their root
     assert (out.double() - want).norm() <= 5e-6 * want.norm()
+
+
+# a weight that the library's kernel just before writes: read only after that kernel has ended
+@pytest.mark.parametrize("M", [1, 16, 40])
+def test_a_weight_of_the_kernel_before(M):
+    N, Kd, inner = 512, 1024, 2048
+    left, right, a = whole((N, inner), 7, 1), whole((Kd, inner), 8, 1), whole((M, Kd), 9, 2)
+    w, out = torch.empty((N, Kd), device=DEV), torch.empty((M, N), device=DEV)
+    exact = a.double() @ (left.double() @ right.double().t()).t()      # whole numbers below 2^24
+    assert exact.abs().max() < 2 ** 24
+    for _ in range(10):
+        w.zero_()
+        K.gemm_simt(left, right, w)
+        K.gemm_simt(a, w, out)
+        assert torch.equal(out.double(), exact)
