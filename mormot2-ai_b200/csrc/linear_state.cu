@@ -17,8 +17,9 @@
 // tokens are staged in shared memory at a time, the next chunk's copies under way while one
 // is walked, and a chunk is walked without a barrier.
 //
-// Steps of 16 and more new tokens a sequence take the same recurrences four tokens at a time
-// (state_walk.cu); this walk serves decoding and short portions.
+// Steps that bring many new tokens take the same recurrences four tokens at a time
+// (state_walk.cu); this walk serves decoding, short portions and steps of which most sequences
+// decode.
 //
 //   short_conv   y_t = silu(sum_j w[c, j] x_(t - taps + 1 + j)) per channel, the inputs before
 //                a step's first token from the state (zeros at a sequence's start)
@@ -65,7 +66,9 @@ __global__ void short_conv_kernel(const float* __restrict__ in, int ld, int col0
 
 // The same for four neighbouring channels a thread and a run of tokens, whose inputs pass through
 // registers: every input is read once, 16 bytes at a time (the kernel above reads it once for every
-// tap, and weights that lie `taps` apart): 2,048 tokens of 4,096 channels, four taps: 65 -> 19 us.
+// tap, and weights that lie `taps` apart): 2,048 tokens of 4,096 channels, four taps: 59 -> 18 us
+// with the kernel for the state. A run is walked by one thread, so a step has to be large enough for
+// it (see mb_short_conv).
 #define SC_RUN 16
 template <int TAPS>
 __global__ void __launch_bounds__(128)
@@ -166,14 +169,21 @@ MB_EXPORT int mb_short_conv(const float* in, int ld, int col0, const float* w, i
   const bool four = taps == 4 && C % 4 == 0 && ld % 4 == 0 && col0 % 4 == 0 && ldo % 4 == 0 &&
                     state_stride % 4 == 0 && state_off % 4 == 0 &&
                     (((uintptr_t)in | (uintptr_t)state | (uintptr_t)out) & 15) == 0;
-  if (four)
-    mb_launch(short_conv4_kernel<4>, dim3((T + SC_RUN - 1) / SC_RUN, (C + 511) / 512), dim3(128), 0, s,
-              in, ld, col0, w, C, (const float*)state, (size_t)state_stride, (size_t)state_off, tok_seq,
-              seq_start, seq_slot, out, ldo, T);
+  // A run of 16 tokens takes 8.5 us whatever there is to do, and up to 7 more where every token
+  // begins a sequence (slot and state are then fetched one after the other); a block a token takes
+  // 4 us and 6.5 for every million values. Both with the kernel for the state, a block a token |
+  // runs: 8 decoding sequences of 4,096 channels 4.1 | 8.8, 64 of them 6.9 | 16.1; one prompt of
+  // 128 tokens 6.7 | 8.8, 256: 10.2 | 8.8, 2,048: 59 | 18; 64 prompts of 4: 12.1 | 16.3, of 8: 18.9 |
+  // 17.8, 300 tokens beside 63 decoding ones 15.2 | 21.9, 1,000 beside 63: 34 | 22.
+  const bool runs = four && (long long)T * C >= (B > 4 ? 2ll << 20 : 1ll << 20);
+  if (runs)
+    mb_launch(short_conv4_kernel<4>, dim3((T + SC_RUN - 1) / SC_RUN, (C + 511) / 512), dim3(128), 0,
+              s, in, ld, col0, w, C, (const float*)state, (size_t)state_stride, (size_t)state_off,
+              tok_seq, seq_start, seq_slot, out, ldo, T);
   else
-  mb_launch(short_conv_kernel, dim3(T, by), dim3(256), 0, s, in, ld, col0, w, taps, C,
-            (const float*)state, (size_t)state_stride, (size_t)state_off, tok_seq, seq_start,
-            seq_slot, out, ldo);
+    mb_launch(short_conv_kernel, dim3(T, by), dim3(256), 0, s, in, ld, col0, w, taps, C,
+              (const float*)state, (size_t)state_stride, (size_t)state_off, tok_seq, seq_start,
+              seq_slot, out, ldo);
   if (taps > 1)
     mb_launch(short_conv_state_kernel, dim3(B, by), dim3(256), 0, s, in, ld, col0, taps, C, state,
               (size_t)state_stride, (size_t)state_off, seq_start, seq_slot);

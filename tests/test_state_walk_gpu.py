@@ -151,3 +151,21 @@ def test_delta_without_a_floor_under_the_keys_length(monkeypatch, lens, group):
     # as above: float32 sums in another order
     assert (out - want).norm() <= 2e-5 * want.norm()
     assert (state4 - state).norm() <= 2e-6 * state.norm()
+
+
+# a block a token and runs of 16 tokens, whichever the step's size takes, give the same values
+@pytest.mark.parametrize("lens", [[600], [300, 1, 2, 270], [1] * 20 + [1100]])
+def test_convolutions_values_do_not_depend_on_the_steps_size(lens):
+    channels, T = 2048, sum(lens)
+    z, w = rows((T, channels), 1), rows((channels, 4), 2)
+    states = rows((len(lens), 3 * channels), 3)
+    after = states.clone()
+    out, alone = torch.empty((T, channels), device=DEV), torch.empty((T, channels), device=DEV)
+    K.short_conv(z, 0, w, after, make_step([(i, 9, [0] * n, []) for i, n in enumerate(lens)]), out)
+    at = 0
+    for i, n in enumerate(lens):          # parts of at most 64 tokens: far below a run's work
+        for a in range(at, at + n, 64):
+            m = min(64, at + n - a)
+            K.short_conv(z[a:a + m], 0, w, states, make_step([(i, 9, [0] * m, [])]), alone[a:a + m])
+        at += n
+    assert torch.equal(out, alone) and torch.equal(after, states)
