@@ -6,7 +6,7 @@
 // step's tokens of its sequence in order, sixteen at a time staged in shared memory; a thread
 // owns one value column of the head's matrix state, which is kept in shared memory.
 //
-// wkv and mlstm of steps of 16 and more new tokens a sequence run in state_walk.cu.
+// wkv and mlstm of steps that bring many new tokens run in state_walk.cu.
 //
 //   token_shift   [h[t] ; h[t-1] - h[t]], from which every blend h + (h' - h) mu_s is projected
 //                 by one product; h[-1] of a sequence is kept in the state (zeros at first)

@@ -14,12 +14,14 @@
 // products, never as quotients). Walked token by token a state element costs four instructions a
 // token and every token ends in a chain of shuffles that the next one waits for; by fours it is
 // two and a quarter to three, and one chain for four tokens. N, M and the factors are small
-// products of keys and queries alone: four warps of the block prepare the next 16 tokens (and copy
-// in the 16 after them) while the others walk these. A thread owns 16 rows of one column of the
-// state in registers, P lanes share a column. What bounds it: the issue slots and the chain of the
-// walking warps; a block takes as few columns as leave it one walking warp a scheduler while the
-// step has few (sequence, head) pairs, so that one prompt spreads over the device. All of it
-// float32. One prompt of 2,048 tokens, 16 heads of 128 x 128: delta 936 -> 366 us, gated linear
+// products of keys and queries alone: CT / 4 warps of the block (a group each) prepare the next
+// chunk of CT tokens (32, or 16 where shared memory does not allow it) and copy in the chunk after
+// it while the others walk this one. A walking thread has 8 or 16 rows of two neighbouring columns
+// of the state in registers, P lanes share a pair of columns. What bounds it: the chain of a group
+// in the walking warps, of which a scheduler has one (of its three warps; issue slots 0.44 busy, the
+// preparing warps wait at the chunk's barrier, the walking ones for fixed latencies and shared
+// memory); a block takes as few columns as leave it one walking warp a scheduler while the step
+// has few (sequence, head) pairs, so that one prompt spreads over the device. All of it float32. One prompt of 2,048 tokens, 16 heads of 128 x 128: delta 936 -> 366 us, gated linear
 // attention 960 -> 365; 8 heads of 128 x 128, mlstm: 1,660 -> 298; 32 heads of 64 x 64, wkv: 870 ->
 // 258. Tried on the way: one column a thread (delta 424: reads of shared memory, 512 bytes each
 // whatever lanes share, bound it).
@@ -67,6 +69,8 @@ struct WalkArgs {
   float q_scale, inv_tau, unit_eps, cap, eps;
 };
 
+static_assert(sizeof(WalkArgs) == 264, "as kernels.py packs it");
+
 __device__ __forceinline__ float sw_log_sigmoid(float x) {
   return fminf(x, 0.f) - log1pf(expf(-fabsf(x)));
 }
@@ -85,9 +89,9 @@ __device__ __forceinline__ void sw_prep_sync(int threads) {
 }
 __device__ __forceinline__ float sw_added(f32_pair v) { return pair_half(v, 0) + pair_half(v, 1); }
 
-// Shared memory: three buffers [q | k | decays (gla, wkv)] of 16 x DP + 16 x CW of v + 16 x 2
-// logits; two of coefficients; two of 16 x CW outputs. mlstm: block z = NS has the one column of
-// the normalizer.
+// Shared memory: three buffers [q | k | decays (gla, wkv)] of CT x DP + CT x CW of v + CT x 2
+// logits; two of coefficients; two of CT x CW outputs. mlstm: the block behind the slices of the
+// columns has the one column of the normalizer.
 template <int MODE, int R>   // R: rows of a walking thread
 __global__ void __launch_bounds__(128 + SW_MOST_CT * 8, 1)
 state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
@@ -169,7 +173,7 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
       float* qb = sw_smem + (ci % 3) * BUF + 4 * w * DP;      // this warp's group
       float* kb = qb + CT * DP;
       float* vb = sw_smem + (ci % 3) * BUF + NV * CT * DP;
-      const float* sc = vb + CT * CW;                      // [16][2]
+      const float* sc = vb + CT * CW;                      // [CT][2]
       float* co = coefs + ((ci & 1) * warps + w) * SW_COEF;
       const int cn = min(CT, n - ci * CT), have = min(4, cn - 4 * w);
       // tokens behind the sequence's last: zeros, so that what an older chunk left has no part
@@ -597,21 +601,26 @@ static size_t walk_smem(int mode, int P, int R, int CW, int CT) {
 MB_EXPORT int mb_state_walk(const WalkArgs* args, int sms, void* stream) {
   WalkArgs g = *args;
   if (g.T <= 0 || g.B <= 0) return 0;
-  if (g.D <= 0 || g.D > 256 || g.DV <= 0 || g.DV > 1024)
-    MB_FAIL("mb_state_walk: heads of %d x %d values (at most 256 x 1024)", g.D, g.DV);
+  if (g.D <= 0 || g.D > 256 || g.DV <= 0 || g.DV > (g.mode == WALK_MLSTM ? 512 : 1024))
+    MB_FAIL("mb_state_walk: heads of %d x %d values (at most 256 x 1024, mlstm 256 x 512)", g.D, g.DV);
   if (g.group <= 0 || g.H % g.group) MB_FAIL("mb_state_walk: %d heads in groups of %d", g.H, g.group);
   if (g.mode < 0 || g.mode > 3) MB_FAIL("mb_state_walk: mode %d", g.mode);
-  // Rows of a walking thread: 16 read least from shared memory and serve a step whose blocks fill
-  // the device; 8 (twice the lanes a column) shorten a group's chain where they do not, as long as
-  // chunks of 32 tokens still fit (one prompt of 2,048, us with 8 and 16: delta, 16 heads of 128 x
-  // 128: 366, 489; four prompts of up to 900, mlstm, 8 heads of 128 x 128: 240, 170).
-  int R = (long long)g.B * g.H * g.DV * walk_lanes(g.D, 16) < (long long)sms * 150 ? 8 : 16;
-  if (R == 8 && walk_smem(g.mode, walk_lanes(g.D, 8), 8, 2 * 128 / walk_lanes(g.D, 8), 32) > 200 * 1024) R = 16;
+  // blocks of a step with R rows a walking thread and so many walking threads a block
+  const auto blocks = [&](int R, int threads) {
+    const int cw = 2 * threads / walk_lanes(g.D, R);
+    return (long long)g.B * g.H * ((g.DV + cw - 1) / cw + (g.mode == WALK_MLSTM ? 1 : 0));
+  };
+  // Rows of a walking thread: 8 (twice the lanes a column) shorten a group's chain and serve a step
+  // whose blocks all run at once (one fits a multiprocessor), as long as chunks of 32 tokens fit; 16
+  // read least from shared memory and have half the blocks. 500 tokens a prompt, us with 8 | 16:
+  // delta, 16 heads of 128 x 128, one prompt 101 | 133, two 198 | 142, four 394 | 281; mlstm, 8 heads
+  // of 128 x 128, two 89 | 94, three 172 | 101, four 174 | 191 (of 111 to 900 tokens 240 | 170); wkv,
+  // 32 heads of 64 x 64, two 85 | 93, three 162 | 107.
+  const int P8 = walk_lanes(g.D, 8);
+  const int R = blocks(8, 128) <= sms && walk_smem(g.mode, P8, 8, 2 * 128 / P8, 32) <= 200 * 1024 ? 8 : 16;
   const int P = walk_lanes(g.D, R);
-  // walking threads of a block (of which one fits a multiprocessor): 128, or 64 where even twice as
-  // many blocks all run at once
-  int threads = 128;
-  if ((long long)g.B * g.H * ((g.DV * P / 2 + threads - 1) / threads) * 2 <= sms) threads = 64;
+  // walking threads of a block: 128, or 64 where even twice as many blocks all run at once
+  const int threads = blocks(R, 64) <= sms ? 64 : 128;
   const int CW = 2 * threads / P, slices = (g.DV + CW - 1) / CW;
   const int CT = walk_smem(g.mode, P, R, CW, 32) <= 200 * 1024 ? 32 : 16;
   g.vec = g.D % 4 == 0 && g.DV % 4 == 0 && CW % 4 == 0 && g.ldq % 4 == 0 && g.ldk % 4 == 0 &&

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import struct
 from typing import Optional
 
 import torch
@@ -643,26 +644,32 @@ def tanh_rows(x: torch.Tensor, out: torch.Tensor) -> None:
           _ptr(out), code_of(out.dtype), x.shape[0], x.shape[1], _stream())
 
 
-class _WalkArgs(_c.Structure):
-    """``WalkArgs`` of csrc/state_walk.cu."""
-    _fields_ = ([(n, _vp) for n in ("q", "k", "v", "a", "s0", "s1", "gate", "abias", "u", "p0", "p1",
-                                    "normw", "state", "seq_start", "seq_slot", "h", "out", "raw")]
-                + [(n, _ll) for n in ("state_stride", "state_off", "head_stride")]
-                + [(n, _i) for n in ("ldq", "ldk", "ldv", "lda", "lds", "ldg", "group", "mode",
-                                     "gate_kind", "norm_stride", "T", "B", "H", "D", "DV", "W",
-                                     "out_bf16", "h_bf16", "vec")]
-                + [(n, _f) for n in ("q_scale", "inv_tau", "unit_eps", "cap", "eps")])
-
-
+# ``WalkArgs`` of csrc/state_walk.cu: 18 addresses, 3 strides, 19 whole numbers, 5 factors
+_WALK_ARGS = struct.Struct("18P3q19i5f")
 WALK_GLA, WALK_DELTA, WALK_MLSTM, WALK_WKV = 0, 1, 2, 3
-# new tokens of a step's longest sequence from which on the recurrences go four tokens at a time
-WALK_TOKENS = 16
 
 
-def walks_by_fours(step, dim: int) -> bool:
-    """Whether a step goes through csrc/state_walk.cu: with fewer tokens a sequence its chunks of
-    16 are mostly empty and the walk token by token is as quick."""
-    return step.max_new >= WALK_TOKENS and dim <= 256
+def walks_by_fours(step, dim: int, mode: int = WALK_DELTA, heads: int = 8) -> bool:
+    """Whether a step goes through csrc/state_walk.cu, four tokens at a time, or token by token. By
+    fours a (sequence, head) takes longer before its first token and less for each, and short
+    values need two kernels (wkv, mlstm) where token by token they need one (3 us of the
+    host's time): it takes enough tokens of the longest sequence, and enough of all, since one
+    long prompt must not draw many decoding sequences along. Measured with heads of 64 x 64 to
+    128 x 128, us token by token | by fours: delta rule, 16 heads, one prompt of 16: 14.7 | 11.5,
+    of 8: 11.3 | 9.9, 32 prompts of 16: 160 | 135, one of 64 (128) beside 63 decoding sequences
+    202 | 206 (240 | 229); matrix memory, 8 heads, one prompt of 24: 22.7 | 13.2, eight of 64 (80
+    would be even) 52 | 55, one of 64 (128) beside 63: 104 | 130 (177 | 142); decaying state, 32
+    heads, one prompt of 32 (48): 13.9 | 13.7 (19.3 | 16.4), 32 prompts of 32: 90 | 81, one of 128
+    (300) beside 63: 93 | 104 (152 | 135)."""
+    n, T, B = step.max_new, step.T, step.B
+    if dim > 256:
+        return False
+    if mode in (WALK_GLA, WALK_DELTA):
+        return n >= 16 and (T >= 8 * B or n >= 2 * B)
+    if mode == WALK_WKV:
+        return n >= 48 and (T >= 24 * B or n >= 4 * B)
+    # the matrix memory: the more (sequence, head) pairs, the sooner token by token fills the device
+    return n >= max(24, min(1.5 * B * heads, 80)) and (T >= 24 * B or n >= 2 * B)
 
 
 def _at(t: torch.Tensor, col: int) -> int:
@@ -670,13 +677,17 @@ def _at(t: torch.Tensor, col: int) -> int:
     return _ptr(t) + 4 * int(col)
 
 
-def _state_walk(step, state, out, heads, dim, vdim, raw, **args) -> None:
-    a = _WalkArgs(state=_ptr(state), state_stride=state.stride(0), seq_start=_ptr(step.seq_start),
-                  seq_slot=_ptr(step.seq_slot), out=_ptr(out), raw=_ptr(raw), T=out.shape[0],
-                  B=step.B, H=heads, D=dim, DV=vdim, out_bf16=int(out.dtype == torch.bfloat16),
-                  group=args.pop("group", 1), **args)
-    _call("state_walk", "mb_state_walk", [_c.POINTER(_WalkArgs), _i, _vp], _c.byref(a), _sms(),
-          _stream(), launches=2)
+def _state_walk(step, state, out, heads, dim, vdim, raw, *, mode, q, k, v, gate, normw, eps, ldq,
+                ldk, ldv, ldg, head_stride, group=1, a=0, s0=0, s1=0, abias=0, u=0, p0=0, p1=0, h=0,
+                state_off=0, lda=0, lds=0, gate_kind=0, norm_stride=0, width=0, h_bf16=0,
+                q_scale=1.0, inv_tau=1.0, unit_eps=0.0, cap=0.0) -> None:
+    args = _WALK_ARGS.pack(
+        q, k, v, a, s0, s1, gate, abias, u, p0, p1, normw, _ptr(state), _ptr(step.seq_start),
+        _ptr(step.seq_slot), h, _ptr(out), _ptr(raw), state.stride(0), state_off, head_stride,
+        ldq, ldk, ldv, lda, lds, ldg, group, mode, gate_kind, norm_stride, out.shape[0], step.B,
+        heads, dim, vdim, width, out.dtype == torch.bfloat16, h_bf16, 0,
+        q_scale, inv_tau, unit_eps, cap, eps)
+    _call("state_walk", "mb_state_walk", [_c.c_char_p, _i, _vp], args, _sms(), _stream(), launches=2)
 
 
 def wkv_scan(r, k, v, lw, g, w0, u, normw, eps: float, state: torch.Tensor,
@@ -697,12 +708,12 @@ def wkv_scan(r, k, v, lw, g, w0, u, normw, eps: float, state: torch.Tensor,
     # where a step has few (sequence, head) pairs a head's columns are dealt over several
     # blocks, which leave their outputs here for the kernel that norms and gates them
     raw = torch.empty((T, heads * dim), dtype=torch.float32, device=out.device)
-    if walks_by_fours(step, dim):
+    if walks_by_fours(step, dim, WALK_WKV, heads):
         _state_walk(step, state, out, heads, dim, dim, raw, mode=WALK_WKV, q=_ptr(r), k=_ptr(k),
                     v=_ptr(v), a=_ptr(lw), gate=_ptr(g), ldq=ld, ldk=ld, ldv=ld, lda=ld, ldg=ld,
                     abias=_ptr(w0), u=_ptr(u), normw=_ptr(normw), norm_stride=dim, eps=float(eps),
                     q_scale=1.0, state_off=h.shape[1], head_stride=dim * dim, h=_ptr(h),
-                    h_bf16=int(h.dtype == torch.bfloat16), W=h.shape[1])
+                    h_bf16=h.dtype == torch.bfloat16, width=h.shape[1])
         return
     _call("recurrent", "mb_wkv_scan",
           [_vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _f, _vp, _ll, _ll, _vp, _i, _i, _vp, _vp,
@@ -729,7 +740,7 @@ def mlstm_scan(z: torch.Tensor, cols, bi, bf, cap: float, q_scale: float, normw,
     _contig(out, "out")
     assert out.shape == (T, heads * vdim) and state.dtype == torch.float32
     assert state.stride(1) == 1 and state.shape[1] >= heads * (dim * vdim + dim + 1)
-    if walks_by_fours(step, dim):
+    if walks_by_fours(step, dim, WALK_MLSTM, heads):
         # the outputs, their denominators and the running maxima after the step
         raw = torch.empty((T * heads * (vdim + 1) + step.B * heads,), dtype=torch.float32,
                           device=out.device)
@@ -861,7 +872,7 @@ def linear_state_scan(mode: str, qkv: torch.Tensor, cols, group: int, gate: torc
     # blocks, which leave their outputs here for the kernel that norms and gates them
     sliced = step.B * heads < 96 and vdim > 32
     raw = torch.empty((T, heads * vdim), dtype=f32, device=out.device)
-    if walks_by_fours(step, dim):
+    if walks_by_fours(step, dim, WALK_GLA if mode == "gla" else WALK_DELTA, heads):
         ld, at = qkv.stride(0), lambda i: _at(qkv, cols[i])
         more = (dict(mode=WALK_GLA, a=_at(decay_logits, decay_col), lda=decay_logits.stride(0),
                      abias=_ptr(decay_bias), inv_tau=float(inv_tau)) if mode == "gla" else

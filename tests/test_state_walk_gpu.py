@@ -153,6 +153,23 @@ def test_delta_without_a_floor_under_the_keys_length(monkeypatch, lens, group):
     assert (state4 - state).norm() <= 2e-6 * state.norm()
 
 
+# GLA and the delta rule, the matrix memory, the decaying state: steps on both sides of the rule's edges
+@pytest.mark.parametrize("lens, by", [
+    ([16], (True, False, False)), ([24], (True, True, False)), ([48], (True, True, True)),
+    ([16] * 8, (True, False, False)), ([80] * 8, (True, True, True)), ([47, 48], (True, True, True)),
+    ([23, 23], (True, False, False)), ([47] * 4, (True, False, False)), ([48] * 4, (True, True, True)),
+    ([16] + [1] * 15, (False, False, False)), ([32] + [1] * 15, (True, False, False)),
+    ([64] + [1] * 15, (True, False, True)), ([80] + [1] * 15, (True, True, True)),
+    ([128] + [1] * 63, (True, True, False)), ([256] + [1] * 63, (True, True, True)),
+    ([127] + [1] * 63, (False, False, False))])
+def test_rule_of_the_walk(lens, by):
+    step = make_step([(i, 0, [0] * n, []) for i, n in enumerate(lens)])
+    modes = (K.WALK_GLA, K.WALK_MLSTM, K.WALK_WKV)
+    assert tuple(K.walks_by_fours(step, 64, m, 8) for m in modes) == by
+    assert K.walks_by_fours(step, 64, K.WALK_DELTA, 8) == by[0]
+    assert not any(K.walks_by_fours(step, 257, m, 8) for m in modes)
+
+
 # a block a token and runs of 16 tokens, whichever the step's size takes, give the same values
 @pytest.mark.parametrize("lens", [[600], [300, 1, 2, 270], [1] * 20 + [1100]])
 def test_convolutions_values_do_not_depend_on_the_steps_size(lens):
