@@ -153,6 +153,99 @@ def test_delta_without_a_floor_under_the_keys_length(monkeypatch, lens, group):
     assert (state4 - state).norm() <= 2e-6 * state.norm()
 
 
+def plain(mode, start, lens, heads, dim, vdim, group, T):
+    """``run`` token after token in float64: outputs [T, heads * vdim] and the sequences' states,
+    without wkv's input row."""
+    qkw, vw = heads // group * dim, heads * vdim
+    z = rows((T, 2 * qkw + 2 * vw + 2 * heads), 1)
+    z[:, :2 * qkw] *= dim ** -0.25
+    z = z.double().cpu()
+    f = lambda *a: rows(*a).double().cpu()
+    head = lambda c, n, per: z[:, c:c + n].reshape(T, -1, per).repeat_interleave(heads * per // n, 1)
+    q, k = head(0, qkw, dim), head(qkw, qkw, dim)
+    v, gate = head(2 * qkw, vw, vdim), head(2 * qkw + vw, vw, vdim)
+    s0, s1 = z[:, 2 * qkw + 2 * vw:].reshape(T, 2, heads).unbind(1)
+    w0, w1 = f((heads,), 2), f((heads,), 3, 1.0, 4.0 if mode == "mlstm" else -2.0)
+    if mode == "gla":
+        a = torch.sigmoid(f((T, heads * dim + 3), 6)[:, 3:] + f((heads * dim,), 7)) ** (1 / 16)
+        q = q * dim ** -0.5
+    elif mode == "wkv":
+        a = torch.exp(-torch.exp(f((T, vw), 6) + f((vw,), 7, 1.0, -2.0)))
+        u = f((vw,), 8).view(heads, dim, 1)
+    elif mode == "delta":
+        q = q / (q.square().sum(-1, keepdim=True) + 1e-6).sqrt() * dim ** -0.5
+        k = k / (k.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+        a = torch.exp(-torch.exp(w0) * torch.nn.functional.softplus(s1 + w1))
+        beta = torch.sigmoid(s0)
+    else:
+        q = q * dim ** -0.5
+        gi = 15 * torch.tanh((s0 + w0) / 15)
+        gf = torch.nn.functional.logsigmoid(15 * torch.tanh((s1 + w1) / 15))
+    out, states, t = torch.empty((T, heads, vdim), dtype=torch.float64), [], 0
+    for b, n in enumerate(lens):
+        S = start[b].double().cpu()
+        if mode == "mlstm":
+            S = S[:heads * (dim * vdim + dim + 1)].view(heads, -1)
+            S, nrm, m = S[:, :dim * vdim].view(heads, dim, vdim), S[:, -dim - 1:-1], S[:, -1]
+        else:
+            S = S[24 if mode == "wkv" else 0:][:heads * dim * vdim].view(heads, dim, vdim)
+        for t in range(t, t + n):
+            kv = k[t][:, :, None] * v[t][:, None, :]
+            if mode == "mlstm":
+                top = torch.maximum(gf[t] + m, gi[t])
+                keep, new, m = torch.exp(gf[t] + m - top), torch.exp(gi[t] - top), top
+                S = keep[:, None, None] * S + new[:, None, None] * kv
+                nrm = keep[:, None] * nrm + new[:, None] * k[t]
+                den = torch.maximum((nrm * q[t]).sum(1).abs(), torch.exp(-m)) + 1e-6
+                o = torch.einsum("hdv,hd->hv", S, q[t]) / den[:, None]
+            elif mode == "wkv":
+                o = torch.einsum("hdv,hd->hv", S + u * kv, q[t])
+                S = a[t].view(heads, dim, 1) * S + kv
+            elif mode == "gla":
+                S = a[t].view(heads, dim, 1) * S + kv
+                o = torch.einsum("hdv,hd->hv", S, q[t])
+            else:
+                S = a[t].view(heads, 1, 1) * S
+                new = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+                S = S + k[t][:, :, None] * new[:, None, :]
+                o = torch.einsum("hdv,hd->hv", S, q[t])
+            out[t] = o / (o.square().mean(1, keepdim=True) + 1e-6).sqrt()
+        t += 1
+        states.append(torch.cat([S.reshape(heads, -1), nrm, m[:, None]], 1).view(-1)
+                      if mode == "mlstm" else S.reshape(-1))
+    per_head = mode in ("mlstm", "wkv")
+    normw = f((vw if per_head else vdim,), 4, 0.1, 1.0).view(-1, vdim)
+    gate = torch.sigmoid(gate) * (1 if mode == "mlstm" else gate)
+    return (out * normw * gate).view(T, -1), torch.stack(states)
+
+
+# from states that are not zero; the last lengths leave a group with one, two and three tokens
+@pytest.mark.parametrize("mode", ["gla", "delta", "mlstm", "wkv"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("fours", [True, False])
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (36, 20)])
+def test_recurrences_in_float64(monkeypatch, mode, dtype, fours, dim, vdim):
+    lens, heads, group = [40, 17, 1, 22, 3], 4, 1 if mode in ("mlstm", "wkv") else 2
+    vdim = dim if mode == "wkv" else vdim
+    T = sum(lens)
+    size = {"mlstm": heads * (dim * vdim + dim + 1), "wkv": 24 + heads * dim * dim}.get(
+        mode, heads * dim * vdim)
+    start = rows((len(lens), size), 9, 0.3)
+    want, states = plain(mode, start, lens, heads, dim, vdim, group, T)
+    monkeypatch.setattr(K, "walks_by_fours", lambda *a: fours)
+    state, step = start.clone(), make_step([(i, 5, [0] * n, []) for i, n in enumerate(lens)])
+    out = run(mode, step, state, T, heads, dim, vdim, group, 0, dtype).double().cpu()
+    # float32 sums over the head, the tokens and the root mean square; bfloat16: the stored
+    # output's rounding, 2^-9 of every value
+    tol = 2e-5 if dtype == torch.float32 else 2.0 ** -8
+    assert (out - want).norm() <= tol * want.norm()
+    got = state.double().cpu()[:, 24 if mode == "wkv" else 0:]
+    assert (got - states).norm() <= 1e-6 * states.norm() + (0 if mode != "mlstm" else 1e-6)
+    if mode == "wkv":      # the last input row of every sequence, as it came
+        last = rows((T, 24), 5).to(dtype).float()[torch.tensor(lens).cumsum(0) - 1]
+        assert torch.equal(state[:, :24], last)
+
+
 # GLA and the delta rule, the matrix memory, the decaying state: steps on both sides of the rule's edges
 @pytest.mark.parametrize("lens, by", [
     ([16], (True, False, False)), ([24], (True, True, False)), ([48], (True, True, True)),
