@@ -21,6 +21,11 @@ namespace cg = cooperative_groups;
 MB_DEFINE_LAST_ERROR
 
 #define ATT_WARPS 4
+// From so many new tokens on a sequence goes in tiles: 16 fill a quarter of a tile of 64; with fewer
+// the tile costs more than reading the keys once per token. Each sequence by itself: a tile with
+// one token in it walks the token's keys in a row on one CTA a head (63 sequences of 2,000
+// positions beside a prompt of 16: 2,700 us with tiles for all, 225 with both kernels).
+#define ATT_MANY 16
 #define ATT_MAX_D 8  // head sizes up to 32 * 8
 
 template <typename T, bool VEC>
@@ -192,14 +197,23 @@ __device__ __forceinline__ float att_gate(const AttArgs<T>& a, int t, int h, int
 // p.v, and a key's row serves all heads of its group. Before, a warp walked a (token, head) alone,
 // with 32 lanes in 32 different rows: a decode step of 8 sequences of 200 to 1,500 positions (16
 // heads on 8 of 128 values, float32, 55 MB) took 744 us; now 25 (2.2 TB/s).
+// `per_seq` > 0: a step in which other sequences bring many tokens (for the kernel below); the
+// clusters then stand for the first per_seq tokens of every sequence and leave those alone.
 #define ATF_WARPS 4
 #define ATF_KEYS 16
 
 template <typename T, int RT, bool WHOLE>   // WHOLE: hd = vd = 128
 __global__ void __launch_bounds__(ATF_WARPS * 32)
-attention_few_kernel(const AttArgs<T> a, int splits, int chunks) {
+attention_few_kernel(const AttArgs<T> a, int splits, int chunks, int per_seq) {
   mb_grid_wait();
   mb_grid_launch_next();
+  int t = blockIdx.x / splits;
+  const int split = blockIdx.x - t * splits;
+  if (per_seq > 0) {
+    const int b = t / per_seq, n_new = a.seq_start[b + 1] - a.seq_start[b];
+    if (n_new >= ATT_MANY || t - b * per_seq >= n_new) return;      // the whole cluster
+    t = a.seq_start[b] + t - b * per_seq;
+  }
   extern __shared__ __align__(16) float sm[];
   const int hd = WHOLE ? 128 : a.hd, vd = WHOLE ? 128 : a.vd;
   constexpr int ND = WHOLE ? 1 : 2;
@@ -211,7 +225,6 @@ attention_few_kernel(const AttArgs<T> a, int splits, int chunks) {
   float* bml = bo + RT * vd;
   size_t* rows = (size_t*)(bml + RT * 2);            // [warps][16]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x / splits, split = blockIdx.x - t * splits;
   const int g = blockIdx.y / chunks, R = a.nh / a.nkv;
   const int h0 = g * R + (blockIdx.y - g * chunks) * RT, heads = min(RT, (g + 1) * R - h0);
   const int pos = a.tok_pos[t], slot = a.seq_slot[a.tok_seq[t]];
@@ -390,7 +403,7 @@ attention_few_kernel(const AttArgs<T> a, int splits, int chunks) {
 }
 
 template <typename T>
-static int launch_few(const AttArgs<T>& a, int tokens, int sms, cudaStream_t s) {
+static int launch_few(const AttArgs<T>& a, int tokens, int per_seq, int sms, cudaStream_t s) {
   const int R = a.nh / a.nkv, RT = R > 4 ? 8 : (R > 2 ? 4 : R), chunks = (R + RT - 1) / RT;
   const bool whole = a.hd == 128 && a.vd == 128;
   // about four CTAs an SM, at most the eight of a portable cluster; it depends on nothing that
@@ -410,7 +423,7 @@ static int launch_few(const AttArgs<T>& a, int tokens, int sms, cudaStream_t s) 
       if (e != cudaSuccess) MB_FAIL("mb_attention_simt: %s", cudaGetErrorString(e));           \
     }                                                                                          \
     mb_launch_clusters(attention_few_kernel<T, R_, W_>, grid, dim3(ATF_WARPS * 32), smem, s,   \
-                       splits, a, splits, chunks);                                             \
+                       splits, a, splits, chunks, per_seq);                                             \
   }
 #define GOW(R_) if (whole) GO(R_, true) else GO(R_, false)
   if (RT == 1) GOW(1) else if (RT == 2) GOW(2) else if (RT == 4) GOW(4) else GOW(8)
@@ -421,12 +434,13 @@ static int launch_few(const AttArgs<T>& a, int tokens, int sms, cudaStream_t s) 
 
 // ---------------------------------------------------------------------------- many new tokens
 // 64 new tokens of one sequence and one head per CTA, a page of 64 keys at a time through shared
-// memory: it is float32 multiply-adds that bound it, and a tile of 64 x 64 scores gives each of
-// 256 threads 4 x 4 of them (every value read from shared memory serves four multiply-adds) and
-// 4 x 8 values of the output (128 threads with twice the rows take 385 us where these take 335: too
-// few warps). Rows of q and k keep their order in shared memory (pitch hd + 4: a warp's 16 keys lie
-// on different banks) and are read four values along the head at a time. K and V take turns in one
-// tile, so that two CTAs fit an SM and one computes while the other loads.
+// memory: a tile of 64 x 64 scores gives each of 256 threads 4 x 4 of them (every value read from
+// shared memory serves four multiply-adds) and 4 x 8 values of the output (128 threads with twice
+// the rows take 385 us where these take 335: too few warps). Rows of q and k keep their order in
+// shared memory (pitch hd + 4: a warp's 16 keys lie on different banks) and are read four values
+// along the head at a time. K and V take turns in one tile, so that two CTAs fit an SM and one
+// computes while the other loads. The reads of shared memory bound it (issue slots 0.51 busy, the
+// pipe of the multiply-adds 0.24; warps wait for operands first of all).
 // Before, a warp walked a (token, head) alone: 1,728 tokens of three prompts (16 heads on 8 of
 // 128 values, float32) took 1,907 us; now 335 (17 TFLOP/s).
 #define ATM_ROWS 64
@@ -436,7 +450,7 @@ static int launch_few(const AttArgs<T>& a, int tokens, int sms, cudaStream_t s) 
 
 template <typename T>
 __global__ void __launch_bounds__(ATM_THREADS, 2)
-attention_many_kernel(const AttArgs<T> a) {
+attention_many_kernel(const AttArgs<T> a, int fewest) {   // fewest: new tokens of a sequence
   mb_grid_wait();
   mb_grid_launch_next();
   extern __shared__ __align__(16) float sm[];
@@ -447,7 +461,7 @@ attention_many_kernel(const AttArgs<T> a) {
   const int h = blockIdx.x, g = h / (a.nh / a.nkv), b = blockIdx.z;
   const int t0 = a.seq_start[b], n_new = a.seq_start[b + 1] - t0;
   const int tiles = (n_new + ATM_ROWS - 1) / ATM_ROWS;
-  if ((int)blockIdx.y >= tiles) return;
+  if ((int)blockIdx.y >= tiles || n_new < fewest) return;
   const int r0 = (tiles - 1 - blockIdx.y) * ATM_ROWS;   // the tiles that see the most keys first
   const int cnt = min(ATM_ROWS, n_new - r0);
   const int slot = a.seq_slot[b], p0 = a.tok_pos[t0 + r0];   // row r stands at position p0 + r
@@ -601,14 +615,14 @@ attention_many_kernel(const AttArgs<T> a) {
 }
 
 template <typename T>
-static int launch_many(const AttArgs<T>& a, int B, int max_new, cudaStream_t s) {
+static int launch_many(const AttArgs<T>& a, int B, int max_new, int fewest, cudaStream_t s) {
   const int pitch = a.hd + 4, kv_pitch = pitch > a.vd ? pitch : a.vd;
   const size_t smem = (size_t)ATM_ROWS * (pitch + kv_pitch + ATM_PITCH) * sizeof(float);
   static unsigned long long allowed = 0;      // heads of 128: 85 KB
   const cudaError_t e = mb_allow_smem((const void*)attention_many_kernel<T>, 88 * 1024, &allowed);
   if (e != cudaSuccess) MB_FAIL("mb_attention_simt: %s", cudaGetErrorString(e));
   mb_launch(attention_many_kernel<T>, dim3(a.nh, (max_new + ATM_ROWS - 1) / ATM_ROWS, B),
-            dim3(ATM_THREADS), smem, s, a);
+            dim3(ATM_THREADS), smem, s, a, fewest);
   MB_CHECK_LAUNCH("mb_attention_simt");
 }
 
@@ -621,12 +635,13 @@ static int launch_many(const AttArgs<T>& a, int B, int max_new, cudaStream_t s) 
 // `gate_dim` > 0, its value d by sigmoid(gate[t * gate_stride + h * gate_dim + d]). `slopes`:
 // float32 [nh] or null: slopes[h] * (query's position - key's position) is taken off every
 // score of head h after the cap. `keep_first` > 0: with a window, the first keep_first
-// positions of a sequence stay visible to every later one.
+// positions of a sequence stay visible to every later one. `few_new`: the most new tokens of a
+// sequence that brings fewer than ATT_MANY of them (0: there is none).
 MB_EXPORT int mb_attention_simt(const void* q, int q_stride, void* out, int out_stride,
                                 const void* kpool, const void* vpool, int dtype,
                                 const int* page_table, int max_pages, int ring_pages,
                                 const int* tok_seq, const int* tok_pos, const int* seq_slot,
-                                const int* seq_start, int B, int max_new,
+                                const int* seq_start, int B, int max_new, int few_new,
                                 int T, int nh, int nkv, int hd, int window, float scale,
                                 int vd, const float* sink, float softcap, const void* gate,
                                 int gate_stride, int gate_dim, const float* slopes, int keep_first,
@@ -645,9 +660,9 @@ MB_EXPORT int mb_attention_simt(const void* q, int q_stride, void* out, int out_
   const bool vec = hd % 4 == 0 && vd % 4 == 0 && q_stride % 4 == 0 && out_stride % 4 == 0 &&
                    (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kpool | (uintptr_t)vpool) & four) == 0;
   if (vec && hd <= 256) {
-    // 16 new tokens of a sequence fill a quarter of a tile of 64; with fewer the tile costs more
-    // than reading the keys once per token
-    const bool many = max_new >= 16 && hd <= 128 && vd <= 128 && B <= 65535;
+    const bool many = max_new >= ATT_MANY && hd <= 128 && vd <= 128 && B <= 65535;
+    const bool mixed = many && few_new > 0;
+    if (mixed && few_new >= ATT_MANY) MB_FAIL("mb_attention_simt: %d are not few new tokens", few_new);
 #define GOA(T_)                                                                               \
   {                                                                                           \
     const AttArgs<T_> a = {(const T_*)q, (T_*)out, (const T_*)kpool, (const T_*)vpool,        \
@@ -655,7 +670,9 @@ MB_EXPORT int mb_attention_simt(const void* q, int q_stride, void* out, int out_
                            (const T_*)gate, q_stride, out_stride, max_pages, ring_pages, nh,  \
                            nkv, hd, vd, window, gate_stride, gate_dim, keep_first, scale,     \
                            softcap};                                                          \
-    return many ? launch_many<T_>(a, B, max_new, s) : launch_few<T_>(a, T, sms, s);           \
+    if (mixed && launch_few<T_>(a, B * few_new, few_new, sms, s)) return -1;                  \
+    return many ? launch_many<T_>(a, B, max_new, mixed ? ATT_MANY : 0, s)                     \
+                : launch_few<T_>(a, T, 0, sms, s);                                            \
   }
     if (dtype == MB_F32) GOA(float) else GOA(__nv_bfloat16)
 #undef GOA

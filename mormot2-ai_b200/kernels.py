@@ -1326,6 +1326,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int =
 
 
 # ------------------------------------------------------------------------------ attention
+ATTENTION_MANY = 16      # ATT_MANY of csrc/attention_simt.cu
+
+
 def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, step, line, nh, nkv, hd,
                    window: int, scale: float, vd: int = 0,
                    sink: Optional[torch.Tensor] = None, softcap: float = 0.0,
@@ -1346,15 +1349,18 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, step, line
     assert slopes is None or (slopes.dtype == torch.float32 and slopes.numel() == nh)
     assert gate is None or gate.dtype == out.dtype
     assert keep_first == 0 or line.ring_pages == 0
+    # sequences that bring few tokens beside one that brings many (see the file)
+    few = max((n for n in step.host_new if n < ATTENTION_MANY), default=0) if (
+        step.max_new >= ATTENTION_MANY and step.B > 1 and max(hd, vd) <= 128) else 0
     _call("attention_simt", "mb_attention_simt",
           [_vp, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
-           _i, _f, _i, _vp, _f, _vp, _i, _i, _vp, _i, _i, _vp],
+           _i, _i, _f, _i, _vp, _f, _vp, _i, _i, _vp, _i, _i, _vp],
           _ptr(q), q_stride, _ptr(out), out.stride(0), _ptr(line.k), _ptr(line.v),
           code_of(out.dtype), _ptr(line.page_table), line.max_pages, line.ring_pages,
           _ptr(step.tok_seq), _ptr(step.tok_pos), _ptr(step.seq_slot), _ptr(step.seq_start), step.B,
-          step.max_new, T, nh, nkv, hd,
+          step.max_new, few, T, nh, nkv, hd,
           window, float(scale), vd or hd, _ptr(sink), float(softcap), _ptr(gate), gate_stride,
-          int(gate_dim), _ptr(slopes), int(keep_first), _sms(), _stream())
+          int(gate_dim), _ptr(slopes), int(keep_first), _sms(), _stream(), launches=2 if few else 1)
 
 
 # ------------------------------------------------------------------------------ sampling

@@ -32,7 +32,8 @@ def reference(q, k, v, pos, window, keep, scale, sink, cap, slopes, gate):
 
 
 # (new tokens, positions held): 15 | 16 is where the form changes, 64 and 65 the tile's edges
-STEPS = [[(1, 0), (1, 63), (1, 700)], [(15, 50), (3, 0)], [(16, 0), (1, 130), (65, 64)], [(129, 300)]]
+STEPS = [[(1, 0), (1, 63), (1, 700)], [(15, 50), (3, 0)], [(16, 0), (1, 130), (65, 64)], [(129, 300)],
+         [(2, 700), (20, 3), (15, 64), (1, 0), (16, 1)]]      # each sequence by its own tokens
 SIZES = [(4, 2, 128, 128), (8, 1, 64, 64), (5, 5, 20, 12), (12, 2, 100, 128), (2, 1, 256, 196)]
 
 
