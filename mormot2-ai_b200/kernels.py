@@ -652,24 +652,24 @@ WALK_GLA, WALK_DELTA, WALK_MLSTM, WALK_WKV = 0, 1, 2, 3
 def walks_by_fours(step, dim: int, mode: int = WALK_DELTA, heads: int = 8) -> bool:
     """Whether a step goes through csrc/state_walk.cu, four tokens at a time, or token by token. By
     fours a (sequence, head) takes longer before its first token and less for each, and short
-    values need two kernels (wkv, mlstm) where token by token they need one (3 us of the
-    host's time): it takes enough tokens of the longest sequence, and enough of all, since one
-    long prompt must not draw many decoding sequences along. Measured with heads of 64 x 64 to
-    128 x 128, us token by token | by fours: delta rule, 16 heads, one prompt of 16: 14.7 | 11.5,
-    of 8: 11.3 | 9.9, 32 prompts of 16: 160 | 135, one of 64 (128) beside 63 decoding sequences
-    202 | 206 (240 | 229); matrix memory, 8 heads, one prompt of 24: 22.7 | 13.2, eight of 64 (80
-    would be even) 52 | 55, one of 64 (128) beside 63: 104 | 130 (177 | 142); decaying state, 32
-    heads, one prompt of 32 (48): 13.9 | 13.7 (19.3 | 16.4), 32 prompts of 32: 90 | 81, one of 128
-    (300) beside 63: 93 | 104 (152 | 135)."""
+    values need two kernels (wkv, mlstm) where token by token they need one: it takes enough tokens
+    of the longest sequence, and enough of all, since one long prompt must not draw many decoding
+    sequences along. Measured with heads of 64 x 64 to 128 x 128, us token by token | by fours:
+    delta rule, 16 heads, one prompt of 16: 14.7 | 11.5, 32 prompts of 16: 160 | 135, one of 64
+    (128) beside 63 decoding sequences 202 | 206 (240 | 229); matrix memory, 8 heads, eight prompts
+    of 64 (80 would be even) 52 | 55, one of 64 (128) beside 63: 104 | 130 (177 | 142); decaying
+    state, 32 heads, 32 prompts of 32: 90 | 81, one of 128 (300) beside 63: 93 | 104 (152 | 135).
+    A single short prompt is bound by the host, whom the second kernel costs 3 us: a whole mixer
+    over 30 tokens of the matrix memory (4 heads) 58 | 61, over 60 of the decaying state 114 | 115."""
     n, T, B = step.max_new, step.T, step.B
     if dim > 256:
         return False
     if mode in (WALK_GLA, WALK_DELTA):
         return n >= 16 and (T >= 8 * B or n >= 2 * B)
     if mode == WALK_WKV:
-        return n >= 48 and (T >= 24 * B or n >= 4 * B)
+        return n >= (96 if B < 16 else 48) and (T >= 48 * B or n >= 4 * B)
     # the matrix memory: the more (sequence, head) pairs, the sooner token by token fills the device
-    return n >= max(24, min(1.5 * B * heads, 80)) and (T >= 24 * B or n >= 2 * B)
+    return n >= max(48, min(1.5 * B * heads, 80)) and (T >= 24 * B or n >= 2 * B)
 
 
 def _at(t: torch.Tensor, col: int) -> int:
