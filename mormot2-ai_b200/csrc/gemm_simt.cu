@@ -206,19 +206,20 @@ gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
 }
 
 // ---------------------------------------------------------------------------- many rows
-// The same product for many rows, bound by float32 multiply-adds and, close behind, by reads of
-// shared memory: a 16-byte read of a warp takes four cycles whatever its lanes share, so a thread
-// has 16 x 8 results (six reads per 128 multiply-adds; 8 x 8 would need as many cycles for the one
-// as for the other). Multiply-adds go two rows an instruction (`fma.rn.f32x2`, each half rounded
-// like a single one), which leaves issue slots for the reads. Blocks are small (64 threads, 64 x
-// 128 results, four to a multiprocessor), K goes in steps of 8 through two buffers with the next
-// step's global loads under way; where tiles are few or would leave a last round half empty, K is
-// dealt out over a cluster whose CTAs add their sums up through shared memory, in K's order.
-// Epilogues: store, residual add, and SwiGLU over weight rows that alternate gate and up (NW = 2 N
-// weight rows, neighbouring columns pair up). 1,728 rows, 6,144 x 1,024 (SwiGLU): 639 us
-// with 128 x 128 tiles, 8 x 8 results a thread -> 519 (42 TFLOP/s); 1,024 x 2,048: 247 -> 216,
-// with 400 rows 246 -> 68. Lanes of a row-wise load that stand in 32 rows cost a tenth of it: a
-// row's LK values lie with neighbouring lanes.
+// The same product for many rows, bound by the latencies of multiply-adds and of shared memory
+// with the 7.6 warps a multiprocessor that the registers leave (the multiply-adds' pipe is 0.57
+// busy). Reads of shared memory come close behind: a 16-byte read of a warp takes four cycles
+// whatever its lanes share, so a thread has 16 x 8 results (six reads per 128 multiply-adds; 8 x 8
+// would need as many cycles for the one as for the other). Multiply-adds go two rows an
+// instruction (`fma.rn.f32x2`, each half rounded like a single one), which leaves issue slots for
+// the reads. Blocks are small (64 threads, 64 x 128 results, four to a multiprocessor), K goes in
+// steps of 8 through two buffers with the next step's global loads under way; where tiles are few
+// or would leave a last round half empty, K is dealt out over a cluster whose CTAs add their sums
+// up through shared memory, in K's order. Epilogues: store, residual add, and SwiGLU over weight
+// rows that alternate gate and up (NW = 2 N weight rows, neighbouring columns pair up). 1,728
+// rows, 6,144 x 1,024 (SwiGLU): 639 us with 128 x 128 tiles, 8 x 8 results a thread -> 519 (42
+// TFLOP/s); 1,024 x 2,048: 247 -> 216, with 400 rows 246 -> 68. Lanes of a row-wise load that
+// stand in 32 rows cost a tenth of it: a row's LK values lie with neighbouring lanes.
 #define LM 64
 #define LN 128
 #define LK 8

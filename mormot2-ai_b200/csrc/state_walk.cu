@@ -18,12 +18,13 @@
 // chunk of CT tokens (32, or 16 where shared memory does not allow it) and copy in the chunk after
 // it while the others walk this one. A walking thread has 8 or 16 rows of two neighbouring columns
 // of the state in registers, P lanes share a pair of columns. What bounds it: the chain of a group
-// in the walking warps, of which a scheduler has one (of its three warps; issue slots 0.44 busy, the
-// preparing warps wait at the chunk's barrier, the walking ones for fixed latencies and shared
+// in the walking warps, of which a scheduler has one (of its three warps; issue slots 0.44 busy,
+// the preparing warps wait at the chunk's barrier, the walking ones for fixed latencies and shared
 // memory); a block takes as few columns as leave it one walking warp a scheduler while the step
-// has few (sequence, head) pairs, so that one prompt spreads over the device. All of it float32. One prompt of 2,048 tokens, 16 heads of 128 x 128: delta 936 -> 366 us, gated linear
-// attention 960 -> 365; 8 heads of 128 x 128, mlstm: 1,660 -> 298; 32 heads of 64 x 64, wkv: 870 ->
-// 258. Tried on the way: one column a thread (delta 424: reads of shared memory, 512 bytes each
+// has few (sequence, head) pairs, so that one prompt spreads over the device. All of it float32.
+// One prompt of 2,048 tokens, 16 heads of 128 x 128: delta 936 -> 366 us, gated linear attention
+// 960 -> 365; 8 heads of 128 x 128, mlstm: 1,660 -> 298; 32 heads of 64 x 64, wkv: 870 -> 258.
+// Tried on the way: one column a thread (delta 424: reads of shared memory, 512 bytes each
 // whatever lanes share, bound it).
 #include "common.cuh"
 
