@@ -250,9 +250,10 @@ def test_recurrences_in_float64(monkeypatch, mode, dtype, fours, dim, vdim):
 @pytest.mark.parametrize("lens, by", [
     ([16], (True, False, False)), ([47], (True, False, False)), ([48], (True, True, False)),
     ([96], (True, True, True)), ([16] * 8, (True, False, False)), ([79] * 8, (True, False, False)),
-    ([96] * 8, (True, True, True)), ([48] * 16, (True, False, True)), ([47, 48], (True, True, False)), ([47] * 4, (True, False, False)),
+    ([96] * 8, (True, True, True)), ([48] * 16, (True, False, True)),
+    ([47, 48], (True, True, False)), ([47] * 4, (True, False, False)),
     ([16] + [1] * 15, (False, False, False)), ([32] + [1] * 15, (True, False, False)),
-    ([80] + [1] * 15, (True, True, False)), ([96] + [1] * 15, (True, True, True)),
+    ([80] + [1] * 15, (True, True, True)), ([96] + [1] * 15, (True, True, True)),
     ([128] + [1] * 63, (True, True, False)), ([256] + [1] * 63, (True, True, True)),
     ([127] + [1] * 63, (False, False, False))])
 def test_rule_of_the_walk(lens, by):
