@@ -42,6 +42,7 @@ SOURCES = {
     "elementwise": "elementwise.cu",
     "rope": "rope.cu",
     "gemm_simt": "gemm_simt.cu",
+    "gemm_split": "gemm_split.cu",
     "attention_simt": "attention_simt.cu",
     "sampling": "sampling.cu",
     "gemm_tc": "gemm_tc.cu",
@@ -64,6 +65,7 @@ HEADERS = ["common.cuh"]
 EXTRA_HEADERS = {"gemm_tc": ["tc_common.cuh"],
                  "attention_mma": ["attention_mma.cuh", "mma_common.cuh", "tc_common.cuh", "no_alloc.h"],
                  "attention_diff": ["attention_mma.cuh", "mma_common.cuh", "tc_common.cuh"],
+                 "gemm_split": ["attention_tc.cuh", "tc_common.cuh"],
                  "attention_tc": ["attention_tc.cuh", "tc_common.cuh"],
                  "attention_diff_tc": ["attention_tc.cuh", "tc_common.cuh"],
                  "latent": ["mma_common.cuh", "mma_tile.cuh"],

@@ -1,7 +1,7 @@
 // y = x · Wᵀ for a weight [N, K] and any M, N, K and any mix of float32 / bfloat16 operands,
 // with float32 multiply-adds on the CUDA cores (no tensor-core or reduced-precision mode):
-// the matrix product of the true 32-bit path, and the fallback for sizes that the
-// tensor-core kernels refuse. The role of the reference's `gemm8` and `linear8`
+// the matrix product of the true 32-bit path for few rows, and the fallback for sizes that the
+// tensor-core kernels refuse (gemm_split.cu has the 32-bit path's products of many rows). The role of the reference's `gemm8` and `linear8`
 // (tools/cuda/linear.cu:418-463, :517-606 of the reference project), without its
 // quantized formats.
 //
@@ -206,7 +206,8 @@ gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
 }
 
 // ---------------------------------------------------------------------------- many rows
-// The same product for many rows, bound by the latencies of multiply-adds and of shared memory
+// The same product for many rows where an operand is bfloat16 or K is short (float32 operands
+// otherwise go through gemm_split.cu), bound by the latencies of multiply-adds and of shared memory
 // with the 7.6 warps a multiprocessor that the registers leave (the multiply-adds' pipe is 0.57
 // busy). Reads of shared memory come close behind: a 16-byte read of a warp takes four cycles
 // whatever its lanes share, so a thread has 16 x 8 results (six reads per 128 multiply-adds; 8 x 8

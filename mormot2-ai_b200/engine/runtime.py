@@ -111,7 +111,7 @@ class Runtime:
         """The kernel libraries that a model of this runtime needs: those of every model and
         what its ``parts`` name (``Part.libraries``); without ``parts``, all of the built-in
         attention's."""
-        libs = ["elementwise", "gemm_simt"]
+        libs = ["elementwise", "gemm_simt", "gemm_split"]
         if self.fast_kernels:
             libs.append("gemm_tc")
         if parts is None:

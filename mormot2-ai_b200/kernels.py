@@ -74,6 +74,7 @@ class Launches:
 
 
 CLASS_OF = {"mb_gemm_tc": "products", "mb_gemm_simt": "products",
+            "mb_gemm_split": "products",
             "mb_attention_simt": "attention", "mb_attention_decode": "attention",
             "mb_attention_decode_clusters": "attention", "mb_attention_prefill": "attention",
             "mb_attention_prefill_tc": "attention", "mb_rmsnorm": "norms",
@@ -1307,22 +1308,46 @@ def attention_diff_prefill_tc(q: torch.Tensor, out: torch.Tensor, step, line, nh
 
 
 # ------------------------------------------------------------------------------ products
+# Up to so many rows a float32 product streams its weight through fma, and up to so many values of K
+# the tensor cores' form is no quicker: it is two kernels and a scratch tensor, 3 us more of the host
+# (17 rows, 64 x 64 back to back: 10.3 us with fma, 11 to 17; 17 rows, 128 x 128: 17.4 and 16.4; 24
+# rows, 1,024 x 2,048: 41 and 19.5).
+SPLIT_ROWS, SPLIT_K = 16, 64
+
+
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPI_STORE,
-              settled: bool = False) -> None:
+              settled: bool = False, error: Optional[torch.Tensor] = None) -> None:
     """c = a · wᵀ (store), c += a · wᵀ (add, float32 c), or SwiGLU over w = [gate; up]
     (EPI_SWIGLU) or over a w whose rows alternate gate, up (EPI_SWIGLU_PAIRS). ``settled``: w is a
     bound weight, which the kernel just before in the stream does not write, and may be read
-    before that kernel has ended."""
+    before that kernel has ended. ``error``: int32 device word for a wait that gave up (the form of
+    many float32 rows waits for its own copies and products)."""
     M, K = a.shape
     N = c.shape[1]
     assert w.shape[1] == K
     assert w.shape[0] == (2 * N if epilogue in (EPI_SWIGLU, EPI_SWIGLU_PAIRS) else N)
     assert c.shape[0] == M and a.stride(1) == 1 and c.stride(1) == 1
     _contig(w, "the weight")
+    if (M > SPLIT_ROWS and K > SPLIT_K and a.dtype == w.dtype == torch.float32 and epilogue != EPI_SWIGLU
+            and not (epilogue == EPI_ADD and c.dtype != torch.float32)):
+        gemm_split(a, w, c, epilogue, error)
+        return
     _call("gemm_simt", "mb_gemm_simt",
           [_vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
           _ptr(a), code_of(a.dtype), a.stride(0), _ptr(w), code_of(w.dtype), _ptr(c),
           code_of(c.dtype), c.stride(0), M, N, K, epilogue, int(settled), _sms(), _stream())
+
+
+def gemm_split(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPI_STORE,
+               error: Optional[torch.Tensor] = None, cols: int = 0, splits: int = 0) -> None:
+    """``gemm_simt`` of float32 operands on the tensor cores, every value in three bfloat16 parts
+    (``csrc/gemm_split.cu``). ``cols`` and ``splits``: 0, or a tile's rows of a and K's parts."""
+    M, Kd = a.shape
+    scratch = torch.empty(6 * M * (-(-Kd // 8) * 8), dtype=torch.uint8, device=a.device)
+    _call("gemm_split", "mb_gemm_split",
+          [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _ll, _vp, _vp],
+          _ptr(a), a.stride(0), _ptr(w), _ptr(c), code_of(c.dtype), c.stride(0), M, c.shape[1], Kd,
+          epilogue, _sms(), cols, splits, _ptr(scratch), scratch.numel(), _ptr(error), _stream(), launches=2)
 
 
 # ------------------------------------------------------------------------------ attention

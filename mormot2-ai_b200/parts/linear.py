@@ -2,8 +2,9 @@
 with the epilogue fused: store, add into the float32 residual, or SwiGLU over gate and up.
 
 The kernel is chosen by the operand types and sizes: the tensor-core kernels for bfloat16
-operands whose sizes they take, else the float32 multiply-add kernel, which takes every size
-and every mix of types (a weight stored in 32 bits stays so and is multiplied in 32 bits).
+operands whose sizes they take, else the float32 products: multiply-adds for few rows and for
+mixed types, the tensor cores with every value cut into three exact bfloat16 parts for more rows
+of float32 (a weight stored in 32 bits stays so, and its products are those of 32 bits).
 """
 from __future__ import annotations
 
@@ -80,13 +81,15 @@ class Linear:
             raise KernelError("a gated epilogue with a bias or another activation than SiLU "
                               "needs bfloat16 operands on 16-byte boundaries")
         if add_into is not None:
-            K.gemm_simt(a, self.weight, add_into, K.EPI_ADD, settled=True)
+            K.gemm_simt(a, self.weight, add_into, K.EPI_ADD, settled=True,
+                        error=self.rt.error_word)
             return add_into
         if self.unary is not None:
             z = torch.empty_like(out)
-            K.gemm_simt(a, self.weight, z, K.EPI_STORE, settled=True)
+            K.gemm_simt(a, self.weight, z, K.EPI_STORE, settled=True,
+                        error=self.rt.error_word)
             K.unary_act(z, out, self.unary)
             return out
         K.gemm_simt(a, self.weight, out, K.EPI_SWIGLU_PAIRS if self.swiglu else K.EPI_STORE,
-                    settled=True)
+                    settled=True, error=self.rt.error_word)
         return out

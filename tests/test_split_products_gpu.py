@@ -1,0 +1,90 @@
+"""Float32 products of more than 16 rows, whose values are cut into three bfloat16 parts: every tile
+width and share of K, rows that are no whole tiles, bases off the 16-byte boundaries, infinities and
+NaNs, and the error against float64 beside that of a chain of float32 multiply-adds."""
+import pytest
+import torch
+
+from mormot2_ai_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def drawn(shape, seed, whole=False):
+    gen = torch.Generator().manual_seed(seed)
+    x = torch.randint(-3, 4, shape, generator=gen).float() if whole else torch.randn(shape, generator=gen)
+    return x.to(DEV)
+
+
+# whole numbers: every sum is exact. Tiles of 16, 96 (four stages of the weight), 112 (three) and 128
+# (two) rows; K shared by 1, 2, 5 and 8 CTAs, with ragged last stages
+@pytest.mark.parametrize("cols, splits", [(16, 1), (16, 8), (96, 1), (96, 2), (112, 1), (112, 5), (128, 1), (128, 3)])
+@pytest.mark.parametrize("M, N, Kd", [(17, 5, 1028), (129, 130, 1095), (300, 384, 1056)])
+def test_plans(cols, splits, M, N, Kd):
+    a, w = drawn((M, Kd), 1, True), drawn((2 * N, Kd), 2, True)
+    error = torch.zeros(1, dtype=torch.int32, device=DEV)
+    exact = a.double() @ w.double().t()
+    out = torch.empty((M, 2 * N), device=DEV)
+    K.gemm_split(a, w, out, K.EPI_STORE, error, cols, splits)
+    assert torch.equal(out.double(), exact)
+    K.gemm_split(a, w, out, K.EPI_ADD, error, cols, splits)
+    assert torch.equal(out.double(), 2 * exact)
+    a, w = a * 0.05, w * 0.25
+    z = a.double() @ w.double().t()
+    want = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
+    for dtype, bound in ((torch.float32, 2e-6), (torch.bfloat16, 4e-3)):    # half a unit of the last place
+        out = torch.empty((M, N), dtype=dtype, device=DEV)
+        K.gemm_split(a, w, out, K.EPI_SWIGLU_PAIRS, error, cols, splits)
+        assert (out.double() - want).norm() <= bound * want.norm()
+    assert int(error) == 0
+
+
+# tiles in several rounds of the device's CTAs
+def test_many_tiles():
+    a, w = drawn((1000, 96), 3, True), drawn((6000, 96), 4, True)
+    out = torch.empty((1000, 6000), device=DEV)
+    K.gemm_simt(a, w, out)
+    assert torch.equal(out, a @ w.t())
+
+
+@pytest.mark.parametrize("shift_a, shift_w, ld", [(1, 0, 200), (0, 1, 200), (0, 0, 203), (3, 2, 201)])
+def test_rows_off_the_boundaries(shift_a, shift_w, ld):
+    M, N, Kd = 70, 140, 200
+    a = drawn((M * ld + 8,), 5, True)[shift_a:shift_a + M * ld].view(M, ld)[:, :Kd]
+    w = drawn((N * Kd + 8,), 6, True)[shift_w:shift_w + N * Kd].view(N, Kd)
+    out = torch.empty((M, N + 3), device=DEV)[:, :N]
+    K.gemm_simt(a, w, out)
+    assert torch.equal(out.double(), a.double() @ w.double().t())
+
+
+# infinities, NaNs (one whose upper 16 bits are an infinity's), the largest and the smallest values
+def test_values_that_are_no_numbers():
+    M, N, Kd = 40, 130, 160
+    a, w = drawn((M, Kd), 7), drawn((N, Kd), 8)
+    a[3, 5], a[4, 7], a[5, 9] = float("inf"), float("-inf"), float("nan")
+    a.view(torch.int32)[6, 11] = 0x7F800001
+    a[7] *= 1e-38
+    a[8, :], w[:, 0] = 0.0, 1.0
+    a[8, 0] = torch.finfo(torch.float32).max
+    w[9, 20], w[10, 21] = float("inf"), float("nan")
+    out = torch.empty((M, N), device=DEV)
+    K.gemm_simt(a, w, out)
+    want = a.double() @ w.double().t()
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.isposinf(), want.isposinf()) and torch.equal(out.isneginf(), want.isneginf())
+    fine = want.isfinite()
+    rows = [m for m in range(M) if m != 7]      # 1e-38: its parts leave float32's normal range
+    assert ((out.double() - want)[rows][fine[rows]].abs() <= 1e-5 * Kd ** 0.5 * want[rows][fine[rows]].abs()
+            .clamp_min(1.0)).all()
+    assert (out.double() - want)[7][fine[7]].abs().max() <= 1e-38
+
+
+# Kd 2^-24 is what a chain of Kd multiply-adds may lose of the sum of magnitudes; four parts of it are far
+# from what is measured (1.3e-7 to 1.9e-7 of the result for 1,024 to 12,288 values)
+@pytest.mark.parametrize("Kd", [64, 1024, 12288])
+def test_error_against_float64(Kd):
+    a, w = drawn((130, Kd), 9), drawn((200, Kd), 10)
+    out = torch.empty((130, 200), device=DEV)
+    K.gemm_simt(a, w, out)
+    want = a.double() @ w.double().t()
+    assert (out.double() - want).norm() <= 4e-7 * want.norm()
