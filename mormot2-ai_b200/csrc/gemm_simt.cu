@@ -100,27 +100,39 @@ gemm_swiglu_halves_kernel(const TA* __restrict__ A, int lda, const TW* __restric
 
 // ---------------------------------------------------------------------------- few rows
 // The same product for at most 16 rows of A (a decode step): the weight streams through once, and
-// its bytes are what bounds it. A warp owns four weight rows (four output features, or two with
-// their gate and up rows) and walks K in chunks of 128 (every lane 4 consecutive values of each of
-// its rows, 16 bytes of float32, the next chunk's asked for before this one is multiplied), against
-// up to eight rows of A at a time. Its 32 sums are reduced by halves, a value a lane at the end. A
-// weight with few rows has KW warps of a block share each four rows along K, so that enough warps
-// ask for it: 1,024 x 3,072 with 8 rows of A, float32: 51 -> 7.8 us; 151,936 x
-// 1,024: 193 -> 147 us (4.2 TB/s).
-// a weight row's values are used once: they pass by the L1 cache, which keeps the rows of A
-template <typename T> __device__ __forceinline__ float4 load4_once(const T* p);
-template <> __device__ __forceinline__ float4 load4_once<float>(const float* p) {
+// its bytes are what bounds it. A warp owns four weight rows at a time (four output features, or two
+// with their gate and up rows) and walks K in chunks of 128 (every lane 4 consecutive values of each
+// of its rows, 16 bytes of float32), against up to eight rows of A. Three chunks are under way or at
+// work at a time, over the border from one group of rows to the next, and the blocks stay for the
+// whole weight, so that enough bytes are asked for at every moment; the rows of A lie in shared
+// memory where they fit (FEW_STAGED: two blocks a multiprocessor) and a warp has work enough, and come
+// four reads at a time elsewhere, with two chunks under way. The 32 sums are reduced by halves, a
+// value a lane at the end. A weight with few rows has KW warps of a block share each four rows along
+// K. Eight rows, float32, from memory, one chunk ahead and a block for every eight groups -> this
+// form: 151,936 x 1,024 163 -> 119 us (5.2 TB/s), 2 x 12,288 x 4,096 182 -> 123, 4,096 x 12,288 147 ->
+// 84, 2 x 3,072 x 1,024 27 -> 18.5, 1,024 x 3,072 18.5 -> 13.3.
+// A weight row's values are used once: they pass by the L1 cache. Predicated, zeros where not `ok`: a
+// load behind a branch would be waited for where the branch ends.
+template <typename T> __device__ __forceinline__ float4 load4_once(const T* p, bool ok);
+template <> __device__ __forceinline__ float4 load4_once<float>(const float* p, bool ok) {
   float4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(p));
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+      "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+      "@p ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}\n"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+      : "l"(p), "r"((int)ok));
   return v;
 }
-template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __nv_bfloat16* p) {
+template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __nv_bfloat16* p, bool ok) {
   uint2 raw;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];"
-               : "=r"(raw.x), "=r"(raw.y)
-               : "l"(p));
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t"
+      "@p ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];\n\t}\n"
+      : "=&r"(raw.x), "=&r"(raw.y)
+      : "l"(p), "r"((int)ok));
   const float2 lo = __bfloat1622float2(*(const __nv_bfloat162*)&raw.x);
   const float2 hi = __bfloat1622float2(*(const __nv_bfloat162*)&raw.y);
   return make_float4(lo.x, lo.y, hi.x, hi.y);
@@ -129,79 +141,124 @@ template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __
 #define FEW_ROWS 8   // rows of A in one pass
 #define FEW_MAX 16   // the most rows that take this kernel
 
-template <typename TA, typename TW, int EPI>
+#define FEW_STAGED (96 * 1024)   // bytes of A's rows that still go into shared memory
+
+template <typename TA, typename TW, int EPI, bool STAGED>
 __global__ void __launch_bounds__(256, 2)
 gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
                      void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K, int KW,
-                     int settled) {
+                     int groups, int settled) {
   constexpr bool GLU = EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_PAIRS;
   constexpr int FEATS = GLU ? 2 : 4;  // output features of a warp
+  constexpr int DEPTH = STAGED ? 3 : 2;      // chunks under way or at work
+  extern __shared__ __align__(16) float As[];      // STAGED: [min(M, 8)][K]
   __shared__ float part[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * (8 / KW) + warp / KW) * FEATS, kw = warp % KW;
-  // the warp's four weight rows; a row beyond the weight is read as its last and not stored
-  const TW* wr[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    int row;
-    if (EPI == EPI_SWIGLU) row = (j >> 1) * N + min(n0 + (j & 1), N - 1);     // g0 g1 u0 u1
-    else if (EPI == EPI_SWIGLU_PAIRS) row = 2 * min(n0 + (j >> 1), N - 1) + (j & 1);  // g0 u0 g1 u1
-    else row = min(n0 + j, N - 1);
-    wr[j] = W + (size_t)row * K;
-  }
+  const int per_block = 8 / KW, kw = warp % KW, step = gridDim.x * per_block;
   const int k_first = kw * 128 + lane * 4, k_step = KW * 128;
-  float4 next[4];
-  auto ask = [&](int k) {
+  const int chunks = (K + k_step - 1) / k_step;
+  const int g_block = blockIdx.x * per_block, g0 = g_block + warp / KW;
+  // the chunk that is asked for next: its group, place and the group's four weight rows; a row beyond
+  // the weight is read as its last and not stored
+  int ask_g, ask_k;
+  const TW* wr[4];
+  auto enter = [&](int g) {
+    ask_g = g;
+    ask_k = k_first;
+    const int n0 = g * FEATS;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      next[j] = k < K ? load4_once<TW>(wr[j] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < 4; ++j) {
+      int row;
+      if (EPI == EPI_SWIGLU) row = (j >> 1) * N + min(n0 + (j & 1), N - 1);     // g0 g1 u0 u1
+      else if (EPI == EPI_SWIGLU_PAIRS) row = 2 * min(n0 + (j >> 1), N - 1) + (j & 1);  // g0 u0 g1 u1
+      else row = min(n0 + j, N - 1);
+      wr[j] = W + (size_t)row * K;
+    }
   };
-  // the first chunk ahead of the wait, where the kernel before does not write the weight
-  if (settled) ask(k_first);
+  auto ask = [&](float4* w) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = load4_once<TW>(wr[j] + ask_k, ask_k < K && ask_g < groups);
+    ask_k += k_step;
+    if (ask_k - k_first >= chunks * k_step) enter(ask_g + step);
+  };
+  float4 w0[4], w1[4], w2[4];
+  auto begin = [&]() {
+    enter(g0);
+    ask(w0);
+    ask(w1);
+    if (DEPTH > 2) ask(w2);
+  };
+  // the first chunks ahead of the wait, where the kernel before does not write the weight
+  if (settled) begin();
   mb_grid_wait();
   mb_grid_launch_next();
-  if (!settled) ask(k_first);
+  if (!settled) begin();
   for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
+    const int rows = min(M - m0, FEW_ROWS);
+    if (m0) begin();
+    if (STAGED) {
+      if (m0) __syncthreads();
+      const int per_row = K >> 2;
+      for (int m = 0; m < rows; ++m)
+        for (int i = threadIdx.x; i < per_row; i += 256)
+          *(float4*)(As + m * K + 4 * i) = load4<TA>(A + (size_t)(m0 + m) * lda + 4 * i);
+      __syncthreads();
+    }
     float acc[4 * FEW_ROWS];
+    int g = g0, k = k_first, chunk = 0;
+    bool more = g_block < groups;      // the same for the whole block
+    auto work = [&](float4* w) {
+      if (chunk == 0) {
 #pragma unroll
-    for (int j = 0; j < 4 * FEW_ROWS; ++j) acc[j] = 0.f;
-    if (m0) ask(k_first);
-    for (int k = k_first; k < K; k += k_step) {
-      float4 w[4];
+        for (int j = 0; j < 4 * FEW_ROWS; ++j) acc[j] = 0.f;
+      }
+      if (k < K) {
+        constexpr int BATCH = STAGED ? 1 : 4;      // reads of A under way together
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = next[j];
-      ask(k + k_step);
+        for (int mb = 0; mb < FEW_ROWS; mb += BATCH) {
+          if (mb >= rows) break;  // uniform over the block
+          float4 a[BATCH];
 #pragma unroll
-      for (int m = 0; m < FEW_ROWS; ++m) {
-        if (m0 + m >= M) break;  // uniform over the warp
-        const float4 a = load4<TA>(A + (size_t)(m0 + m) * lda + k);
+          for (int i = 0; i < BATCH; ++i)
+            a[i] = STAGED ? *(const float4*)(As + mb * K + k)
+                          : load4<TA>(A + (size_t)(m0 + min(mb + i, rows - 1)) * lda + k);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float& s = acc[j * FEW_ROWS + m];
-          s = fmaf(a.x, w[j].x, fmaf(a.y, w[j].y, fmaf(a.z, w[j].z, fmaf(a.w, w[j].w, s))));
+          for (int i = 0; i < BATCH; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float& s = acc[j * FEW_ROWS + mb + i];
+              s = fmaf(a[i].x, w[j].x, fmaf(a[i].y, w[j].y, fmaf(a[i].z, w[j].z, fmaf(a[i].w, w[j].w, s))));
+            }
         }
       }
+      ask(w);
+      k += k_step;
+      if (++chunk < chunks) return;
+      // the group's end
+      float v = sum32_by_lane(acc, lane);      // lane 8 j + m: weight row j, row m0 + m of A
+      if (KW > 1) {
+        __syncthreads();      // the sums of the group before have been read
+        part[warp][lane] = v;
+        __syncthreads();
+        if (kw == 0)
+          for (int i = 1; i < KW; ++i) v += part[warp + i][lane];
+      }
+      const int j = lane >> 3, m = m0 + (lane & 7);
+      const float up = GLU ? __shfl_sync(0xffffffffu, v, (lane + (EPI == EPI_SWIGLU ? 16 : 8)) & 31) : 0.f;
+      const int f = EPI == EPI_SWIGLU_PAIRS ? j >> 1 : j, n0 = g * FEATS;
+      const bool has = EPI == EPI_SWIGLU_PAIRS ? !(j & 1) : (EPI != EPI_SWIGLU || j < 2);
+      if (kw == 0 && m < M && has && n0 + f < N)
+        put_out(C, c_bf16, (size_t)m * ldc + n0 + f, GLU ? v / (1.0f + expf(-v)) * up : v, EPI == EPI_ADD);
+      chunk = 0;
+      k = k_first;
+      g += step;
+      more = g - warp / KW < groups;
+    };
+    while (more) {
+      work(w0);
+      if (more) work(w1);
+      if (DEPTH > 2 && more) work(w2);
     }
-    float v = sum32_by_lane(acc, lane);      // lane 8 j + m: weight row j, row m0 + m of A
-    if (KW > 1) {
-      __syncthreads();      // the sums of the rows of A before have been read
-      part[warp][lane] = v;
-      __syncthreads();
-      if (kw == 0)
-        for (int i = 1; i < KW; ++i) v += part[warp + i][lane];
-    }
-    const int j = lane >> 3, m = m0 + (lane & 7);
-    const float up = GLU ? __shfl_sync(0xffffffffu, v, (lane + (EPI == EPI_SWIGLU ? 16 : 8)) & 31) : 0.f;
-    if (kw != 0 || m >= M) continue;
-    int f = j;
-    if (EPI == EPI_SWIGLU_PAIRS) {
-      if (j & 1) continue;
-      f = j >> 1;
-    }
-    if (EPI == EPI_SWIGLU && j >= 2) continue;
-    if (n0 + f >= N) continue;
-    const float out = GLU ? v / (1.0f + expf(-v)) * up : v;
-    put_out(C, c_bf16, (size_t)m * ldc + n0 + f, out, EPI == EPI_ADD);
   }
 }
 
@@ -377,19 +434,45 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
       ((uintptr_t)W & w_align) == 0) {
     const int feats = (epi == EPI_SWIGLU || epi == EPI_SWIGLU_PAIRS) ? 2 : 4;
     const int groups = (N + feats - 1) / feats;
-    // warps that share a group's K: until some 3,000 warps ask for the weight (8 rows of A;
-    // 1,024 x 2,048: 39 us with one, 6 with eight), at least 128 values of K each
+    // Warps that share a group's K: as many as leave the least to do for the busiest warp, in chunks of
+    // 128 with one more for what a group's end takes, when two blocks of eight warps a multiprocessor
+    // are all that run
+    const int room = 2 * sms;
     int kw = 1;
-    while (kw < 8 && groups * kw < 3000 && kw * 128 < K) kw *= 2;
-    const int blocks = (groups + 8 / kw - 1) / (8 / kw);
+    long long least = 1ll << 60;
+    for (int n = 1; n <= 8 && (n == 1 || (n - 1) * 128 < K); n *= 2) {
+      const long long work = (long long)((groups + (8 / n) * room - 1) / ((8 / n) * room)) *
+                             ((K + 128 * n - 1) / (128 * n) + 1);
+      if (work < least) { least = work; kw = n; }
+    }
+    const int all = (groups + 8 / kw - 1) / (8 / kw), blocks = all < room ? all : room;
+    const int rows = M < FEW_ROWS ? M : FEW_ROWS;
+    const size_t bytes = (size_t)rows * K * sizeof(float);
+    // The rows of A into shared memory where a warp has at least eight chunks: the copy costs a wait
+    // of its own. Eight rows, us with | without: 151,936 x 1,024 119 | 134 and 2 x 3,072 x 1,024 (8
+    // chunks a warp) 18.5 | 20.5, but 4,096 x 1,024 (4) 16.4 | 14.5 and 1,024 x 3,072 (3) 16.4 | 13.3.
+    const long long rounds = (groups + (8 / kw) * (long long)blocks - 1) / ((8 / kw) * (long long)blocks);
+    const bool staged = bytes <= FEW_STAGED && rounds * ((K + 128 * kw - 1) / (128 * kw)) >= 8;
+#define FEW2(E, S_)                                                                           \
+  {                                                                                           \
+    static unsigned long long allowed = 0;                                                    \
+    const cudaError_t e =                                                                     \
+        S_ ? mb_allow_smem((const void*)gemm_few_rows_kernel<TA, TW, E, S_>, FEW_STAGED, &allowed) \
+           : cudaSuccess;                                                                     \
+    if (e != cudaSuccess) MB_FAIL("mb_gemm_simt: %s", cudaGetErrorString(e));                 \
+    mb_launch(gemm_few_rows_kernel<TA, TW, E, S_>, dim3(blocks), dim3(256), S_ ? bytes : 0, s, \
+              (const TA*)A, lda, (const TW*)W, C, c_bf16, ldc, M, N, K, kw, groups, settled); \
+  }
 #define FEW(E)                                                                                \
-  mb_launch(gemm_few_rows_kernel<TA, TW, E>, dim3(blocks), dim3(256), 0, s, (const TA*)A, lda, \
-            (const TW*)W, C, c_bf16, ldc, M, N, K, kw, settled)
-    if (epi == EPI_STORE) FEW(EPI_STORE);
-    else if (epi == EPI_ADD) FEW(EPI_ADD);
-    else if (epi == EPI_SWIGLU) FEW(EPI_SWIGLU);
-    else FEW(EPI_SWIGLU_PAIRS);
+  if (staged) FEW2(E, true) else FEW2(E, false)
+    switch (epi) {
+      case EPI_STORE: FEW(EPI_STORE) break;
+      case EPI_ADD: FEW(EPI_ADD) break;
+      case EPI_SWIGLU: FEW(EPI_SWIGLU) break;
+      default: FEW(EPI_SWIGLU_PAIRS)
+    }
 #undef FEW
+#undef FEW2
     MB_CHECK_LAUNCH("mb_gemm_simt");
   }
   if (epi != EPI_SWIGLU) {
