@@ -65,6 +65,7 @@ HEADERS = ["common.cuh"]
 EXTRA_HEADERS = {"gemm_tc": ["tc_common.cuh"],
                  "attention_mma": ["attention_mma.cuh", "mma_common.cuh", "tc_common.cuh", "no_alloc.h"],
                  "attention_diff": ["attention_mma.cuh", "mma_common.cuh", "tc_common.cuh"],
+                 "state_walk": ["state_chunks.cuh", "mma_common.cuh"],
                  "gemm_split": ["attention_tc.cuh", "tc_common.cuh"],
                  "attention_tc": ["attention_tc.cuh", "tc_common.cuh"],
                  "attention_diff_tc": ["attention_tc.cuh", "tc_common.cuh"],

@@ -258,6 +258,29 @@ __device__ __forceinline__ f32_pair pair_of(float a, float b) {
 __device__ __forceinline__ float pair_half(f32_pair v, int h) {
   return __uint_as_float((unsigned)(v >> (32 * h)));
 }
+
+// A float32 value as the exact sum of three bfloat16 parts of 8 significant bits each: its upper half,
+// the upper half of what is left, and the rest. Of two neighbouring values, as they stand in memory.
+// An infinity's first part is that infinity, its others are NaN.
+struct Cut2 {
+  uint32_t hi, mid, lo;
+};
+__device__ __forceinline__ f32_pair pair_sub_upper(f32_pair v) {      // v less its upper halves
+  f32_pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r) : "l"(v & 0xffff0000ffff0000ull), "l"(0xbf800000bf800000ull), "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint32_t upper_halves(f32_pair v) {
+  return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632);
+}
+__device__ __forceinline__ Cut2 cut(float a, float b) {
+  f32_pair v;      // a NaN whose upper half alone would read as an infinity becomes the common one
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(pair_of(a, b)), "l"(0x8000000080000000ull));
+  const f32_pair r = pair_sub_upper(v), q = pair_sub_upper(r);
+  return {upper_halves(v), upper_halves(r), upper_halves(q)};
+}
+
 __device__ __forceinline__ void pair_fma(f32_pair& s, f32_pair a, f32_pair b) {   // s += a b
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
 }

@@ -44,26 +44,6 @@ constexpr int GS_A_COLS = 3 * GS_K / 2;      // tensor memory of a stage: hi, mi
 constexpr int GS_THREADS = 32 * 20;  // 8 warps cut the weight, 8 drain, 1 loads, 2 issue, 1 has no part
 constexpr int GS_SMEM = 200 * 1024;  // of the stages of x
 
-// The parts of two neighbouring values, as they stand in memory
-struct Cut2 {
-  uint32_t hi, mid, lo;
-};
-__device__ __forceinline__ f32_pair pair_sub_upper(f32_pair v) {      // v less its upper halves
-  f32_pair r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(r) : "l"(v & 0xffff0000ffff0000ull), "l"(0xbf800000bf800000ull), "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint32_t upper_halves(f32_pair v) {
-  return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632);
-}
-__device__ __forceinline__ Cut2 cut(float a, float b) {
-  f32_pair v;      // a NaN whose upper half alone would read as an infinity becomes the common one
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(pair_of(a, b)), "l"(0x8000000080000000ull));
-  const f32_pair r = pair_sub_upper(v), q = pair_sub_upper(r);
-  return {upper_halves(v), upper_halves(r), upper_halves(q)};
-}
-
 // 16 lanes x 16 columns of tensor memory: registers 4 j .. 4 j + 3 hold columns 8 j + 2 (lane % 4)
 // and the next of row lane / 4, then of row lane / 4 + 8
 __device__ __forceinline__ void tmem_st_rows16(uint32_t taddr, const uint32_t* w) {

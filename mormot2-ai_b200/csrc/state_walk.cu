@@ -10,6 +10,8 @@
 //   mlstm    x = v, A a scalar; the normalizer n is one more column whose values are one
 //   gla, wkv x = v, A per key channel; q' and k' carry the decays of the group's tokens
 //
+// Long sequences of the first two go in chunks of 32 tokens instead (state_chunks.cuh).
+//
 // (definitions of the mixers in linear_state.cu and recurrent.cu; products of decays are formed as
 // products, never as quotients). Walked token by token a state element costs four instructions a
 // token and every token ends in a chain of shuffles that the next one waits for; by fours it is
@@ -78,6 +80,8 @@ __device__ __forceinline__ float sw_log_sigmoid(float x) {
 __device__ __forceinline__ float sw_softplus(float x) {
   return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x)));
 }
+#include "state_chunks.cuh"
+
 template <int BYTES> __device__ __forceinline__ void sw_copy(float* dst, const float* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   if (BYTES == 16)
@@ -586,6 +590,19 @@ __global__ void state_walk_norm_kernel(const WalkArgs g) {
   }
 }
 
+static int launch_norm(const WalkArgs& g, cudaStream_t s) {
+  const bool vec = g.DV % 4 == 0 && g.ldg % 4 == 0 && g.norm_stride % 4 == 0 &&
+                   (((uintptr_t)g.raw | (uintptr_t)g.gate | (uintptr_t)g.normw) & 15) == 0 &&
+                   ((uintptr_t)g.out & (g.out_bf16 ? 7 : 15)) == 0;
+  const dim3 grid((g.T * g.H + 7) / 8);
+#define NORM(T_)                                                                   \
+  if (vec) mb_launch(state_walk_norm_kernel<T_, true>, grid, dim3(256), 0, s, g);  \
+  else mb_launch(state_walk_norm_kernel<T_, false>, grid, dim3(256), 0, s, g)
+  if (g.out_bf16) { NORM(__nv_bfloat16); } else { NORM(float); }
+#undef NORM
+  MB_CHECK_LAUNCH("mb_state_walk");
+}
+
 static int walk_lanes(int D, int R) {
   int p = 4;
   while (p * R < D) p *= 2;
@@ -627,9 +644,6 @@ MB_EXPORT int mb_state_walk(const WalkArgs* args, int sms, void* stream) {
   g.vec = g.D % 4 == 0 && g.DV % 4 == 0 && CW % 4 == 0 && g.ldq % 4 == 0 && g.ldk % 4 == 0 &&
           g.ldv % 4 == 0 && g.lda % 4 == 0 &&
           (((uintptr_t)g.q | (uintptr_t)g.k | (uintptr_t)g.v | (uintptr_t)g.a) & 15) == 0;
-  const bool vec_norm = g.DV % 4 == 0 && g.ldg % 4 == 0 && g.norm_stride % 4 == 0 &&
-                        (((uintptr_t)g.raw | (uintptr_t)g.gate | (uintptr_t)g.normw) & 15) == 0 &&
-                        ((uintptr_t)g.out & (g.out_bf16 ? 7 : 15)) == 0;
   const size_t smem = walk_smem(g.mode, P, R, CW, CT);
   const dim3 grid(g.B, g.H, slices + (g.mode == WALK_MLSTM ? 1 : 0));
   cudaStream_t s = (cudaStream_t)stream;
@@ -650,11 +664,61 @@ MB_EXPORT int mb_state_walk(const WalkArgs* args, int sms, void* stream) {
   }
 #undef GOR
 #undef GO
-  const int rows = g.T * g.H;
-#define NORM(T_)                                                                               \
-  if (vec_norm) mb_launch(state_walk_norm_kernel<T_, true>, dim3((rows + 7) / 8), dim3(256), 0, s, g); \
-  else mb_launch(state_walk_norm_kernel<T_, false>, dim3((rows + 7) / 8), dim3(256), 0, s, g)
-  if (g.out_bf16) { NORM(__nv_bfloat16); } else { NORM(float); }
-#undef NORM
-  MB_CHECK_LAUNCH("mb_state_walk");
+  return launch_norm(g, s);
+}
+
+// The delta rule and the matrix memory in chunks of 32 tokens (state_chunks.cuh): heads of up to 128 x
+// 1024 (mlstm 128 x 512) values, multiples of 16 both, rows on 16-byte boundaries. `scratch`:
+// `scratch_floats` floats, at least mb_state_chunks_scratch of one chunk a sequence; with less than all
+// chunks' room the chunks go in several passes. `longest`: the most new tokens of a sequence.
+MB_EXPORT long long mb_state_chunks_scratch(int mode, int B, int H, int D, int DV, int chunks) {
+  return (long long)B * H * ((long long)sc_chunk_floats(mode == WALK_DELTA, D, DV) * chunks + 2);
+}
+
+MB_EXPORT int mb_state_chunks(const WalkArgs* args, float* scratch, long long scratch_floats, int longest,
+                              void* stream) {
+  const WalkArgs g = *args;
+  if (g.T <= 0 || g.B <= 0) return 0;
+  const bool delta = g.mode == WALK_DELTA;
+  if (!delta && g.mode != WALK_MLSTM) MB_FAIL("mb_state_chunks: mode %d", g.mode);
+  if (g.D <= 0 || g.D > 128 || g.D % 16 || g.DV <= 0 || g.DV % 16 || g.DV > (delta ? 1024 : 512))
+    MB_FAIL("mb_state_chunks: heads of %d x %d values", g.D, g.DV);
+  if (g.group <= 0 || g.H % g.group) MB_FAIL("mb_state_chunks: %d heads in groups of %d", g.H, g.group);
+  if (g.ldq % 4 || g.ldk % 4 || g.ldv % 4 ||
+      (((uintptr_t)g.q | (uintptr_t)g.k | (uintptr_t)g.v | (uintptr_t)scratch) & 15))
+    MB_FAIL("mb_state_chunks: rows off the 16-byte boundaries");
+  const int all = (longest + SC_C - 1) / SC_C;
+  const long long each = (long long)g.B * g.H * sc_chunk_floats(delta, g.D, g.DV), maxima = 2ll * g.B * g.H;
+  const long long fit = (scratch_floats - maxima) / each;
+  const int per_seq = fit < all ? (int)fit : all;
+  if (all < 1 || per_seq < 1) MB_FAIL("mb_state_chunks: %lld floats of scratch are too few", scratch_floats);
+  cudaStream_t s = (cudaStream_t)stream;
+  const size_t prep_smem = (2 * SC_C * (g.D + 8) + SC_C * 33 + 2 * SC_C * 36 + 16 * 17 + 3 * SC_C +
+                            (delta ? (g.DV <= SC_V_HERE ? SC_C * (size_t)(g.DV + 8) : 0) : 2 * (size_t)per_seq)) * 4;
+  const int warps = g.D / 16, rows = delta ? 2 * SC_C : SC_C, threads = 32 * (warps < 4 ? 4 : warps);
+  const size_t walk_smem = ((size_t)warps * rows * SC_PART + SC_C * SC_PART + 3 * SC_COLS * 20) * 4;
+  if (prep_smem > 200 * 1024) MB_FAIL("mb_state_chunks: %d chunks in one pass", per_seq);
+  static unsigned long long allowed[4] = {0, 0, 0, 0};
+  const void* kernels[4] = {(const void*)state_chunk_prep_kernel<false>, (const void*)state_chunk_prep_kernel<true>,
+                            (const void*)state_chunk_walk_kernel<false>, (const void*)state_chunk_walk_kernel<true>};
+  for (int i = 0; i < 4; ++i) {
+    const cudaError_t e = mb_allow_smem(kernels[i], 200 * 1024, &allowed[i]);
+    if (e != cudaSuccess) MB_FAIL("mb_state_chunks: %s", cudaGetErrorString(e));
+  }
+  float* m[2] = {scratch + scratch_floats - maxima, scratch + scratch_floats - maxima / 2};
+  int pass = 0;
+  for (int c = 0; c < all; c += per_seq, ++pass) {
+    const int now = all - c < per_seq ? all - c : per_seq;
+    const dim3 grid((unsigned)(g.B * now), g.H), walk(g.B, g.H, g.DV / SC_COLS + (delta ? 0 : 1));
+    if (delta) {
+      mb_launch(state_chunk_prep_kernel<true>, grid, dim3(256), prep_smem, s, g, scratch, c, now,
+                (const float*)m[pass & 1], m[1 - (pass & 1)]);
+      mb_launch(state_chunk_walk_kernel<true>, walk, dim3(threads), walk_smem, s, g, (const float*)scratch, c, now);
+    } else {
+      mb_launch(state_chunk_prep_kernel<false>, grid, dim3(256), prep_smem, s, g, scratch, c, now,
+                (const float*)m[pass & 1], m[1 - (pass & 1)]);
+      mb_launch(state_chunk_walk_kernel<false>, walk, dim3(threads), walk_smem, s, g, (const float*)scratch, c, now);
+    }
+  }
+  return launch_norm(g, s);
 }

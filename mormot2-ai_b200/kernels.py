@@ -99,7 +99,7 @@ CLASS_OF = {"mb_gemm_tc": "products", "mb_gemm_simt": "products",
             "mb_norm_add": "norms", "mb_cast_rows": "norms", "mb_norm_step": "norms",
             "mb_unary_act": "activation", "mb_softcap": "activation",
             "mb_pass_input": "embedding", "mb_wide_qk_norm": "rotary", "mb_rope_store": "rotary",
-            "mb_short_conv": "recurrence", "mb_state_walk": "recurrence", "mb_linear_state_scan": "recurrence"}
+            "mb_short_conv": "recurrence", "mb_state_walk": "recurrence", "mb_state_chunks": "recurrence", "mb_linear_state_scan": "recurrence"}
 
 
 class Timing:
@@ -673,6 +673,28 @@ def walks_by_fours(step, dim: int, mode: int = WALK_DELTA, heads: int = 8) -> bo
     return n >= max(48, min(1.5 * B * heads, 80)) and (T >= 24 * B or n >= 2 * B)
 
 
+CHUNK = 32                      # SC_C of csrc/state_chunks.cuh
+CHUNK_SCRATCH = 160 << 20       # bytes of chunks' factors that a pass may take
+
+
+def walks_in_chunks(step, dim: int, vdim: int, mode: int, heads: int) -> bool:
+    """Whether a step that goes by fours goes in chunks of 32 tokens instead (csrc/state_chunks.cuh).
+    That takes a third of the time for a long sequence's tokens and 10 us before the first, and pays
+    less the more (sequence, head) pairs there are to fill the device by fours already. Measured, walk
+    and norm, us by fours | in chunks: delta rule, 16 heads of 128 x 128, one prompt of 64 / 128 / 1,000:
+    30 | 35, 41 | 39, 202 | 117; three 54 | 40, 87 | 57, 551 | 345; eight of 64 / 400 101 | 78, 464 |
+    370; 63 decoding beside 256 284 | 580. 8 heads of 64 x 128, three prompts of 64 / 128 24 | 26, 36 |
+    31, eight of 128 / 200 46 | 46, 63 | 71. Matrix memory, 8 heads of 128 x 128, one prompt of 64 / 96 /
+    1,000: 28 | 25, 30 | 27, 164 | 111; eight of 64 / 400 61 | 38, 245 | 123; 63 decoding beside 128
+    153 | 111; 4 heads of 64 x 64, one of 64 / 96 22 | 21, 26 | 24."""
+    if mode not in (WALK_DELTA, WALK_MLSTM) or dim % 16 or dim > 128 or vdim % 16:
+        return False
+    n, pairs = step.max_new, step.B * heads
+    if mode == WALK_MLSTM:
+        return n >= (64 if pairs >= 64 else 96)
+    return n >= (64 if pairs > 24 else 128) and pairs <= (48 if dim <= 64 else 128)
+
+
 def _at(t: torch.Tensor, col: int) -> int:
     """The address of column ``col`` of a float32 tensor whose rows are dense."""
     return _ptr(t) + 4 * int(col)
@@ -688,6 +710,17 @@ def _state_walk(step, state, out, heads, dim, vdim, raw, *, mode, q, k, v, gate,
         ldq, ldk, ldv, lda, lds, ldg, group, mode, gate_kind, norm_stride, out.shape[0], step.B,
         heads, dim, vdim, width, out.dtype == torch.bfloat16, h_bf16, 0,
         q_scale, inv_tau, unit_eps, cap, eps)
+    if (walks_in_chunks(step, dim, vdim, mode, heads) and ldq % 4 == 0 and ldk % 4 == 0
+            and ldv % 4 == 0 and (q | k | v) % 16 == 0):
+        chunks = -(-step.max_new // CHUNK)
+        each = 1728 + dim // 16 * 192 * (12 if mode == WALK_DELTA else 8) + (
+            CHUNK * vdim if mode == WALK_DELTA else 0)      # sc_chunk_floats of csrc/state_chunks.cuh
+        pairs = step.B * heads
+        passes = min(chunks, max(1, CHUNK_SCRATCH // (4 * pairs * each)))
+        scratch = torch.empty(pairs * (each * passes + 2), dtype=torch.float32, device=out.device)
+        _call("state_walk", "mb_state_chunks", [_c.c_char_p, _vp, _ll, _i, _vp], args, _ptr(scratch),
+              scratch.numel(), step.max_new, _stream(), launches=2 * -(-chunks // passes) + 1)
+        return
     _call("state_walk", "mb_state_walk", [_c.c_char_p, _i, _vp], args, _sms(), _stream(), launches=2)
 
 
