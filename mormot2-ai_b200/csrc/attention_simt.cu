@@ -3,7 +3,8 @@
 // or bfloat16 storage. It serves prefill and decode of the true 32-bit path and is the fallback
 // of the bfloat16 path. Sizes that are multiples of four (heads of up to 256) with rows on the
 // boundaries of four values go through two kernels: `attention_few_kernel` for a step that brings
-// few tokens a sequence and `attention_many_kernel` for tiles of 64 new tokens. For all else one
+// few tokens a sequence and `attention_many_kernel` for tiles of 64 new tokens (float32 heads of 128
+// values that see many keys: attention_split.cuh, on the tensor cores). For all else one
 // warp per (token, query head) walks the keys of the token's own sequence in tiles of 32 with an
 // online softmax (a lane has one key of the tile for q·k and four neighbouring values of every
 // key's row for p·v).
@@ -14,18 +15,13 @@
 // y = (sum p v) / (sum p) — and the tiled form of tools/cuda/ops.cu:352-540.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "attention_split.cuh"
 
 namespace cg = cooperative_groups;
 
 MB_DEFINE_LAST_ERROR
 
 #define ATT_WARPS 4
-// From so many new tokens on a sequence goes in tiles: 16 fill a quarter of a tile of 64; with fewer
-// the tile costs more than reading the keys once per token. Each sequence by itself: a tile with
-// one token in it walks the token's keys in a row on one CTA a head (63 sequences of 2,000
-// positions beside a prompt of 16: 2,700 us with tiles for all, 225 with both kernels).
-#define ATT_MANY 16
 #define ATT_MAX_D 8  // head sizes up to 32 * 8
 
 template <typename T, bool VEC>
@@ -151,41 +147,6 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
       if (i < vd) op[i] = from_f32<T>(acc[d] * inv);
     }
   }
-}
-
-// What both kernels below are given. A score s (after the scale) goes through softcap and slopes as
-// in attention_simt_kernel; `max_pages`, `ring_pages`, `keep_first`, `gate` likewise.
-template <typename T> struct AttArgs {
-  const T* q;
-  T* out;
-  const T* kpool;
-  const T* vpool;
-  const int* page_table;
-  const int* tok_seq;
-  const int* tok_pos;
-  const int* seq_slot;
-  const int* seq_start;
-  const float* sink;
-  const float* slopes;
-  const T* gate;
-  int q_stride, out_stride, max_pages, ring_pages, nh, nkv, hd, vd, window, gate_stride, gate_dim,
-      keep_first;
-  float scale, softcap;
-};
-
-template <typename T>
-__device__ __forceinline__ float att_score(const AttArgs<T>& a, float dot, float slope, int dist) {
-  float s = dot * a.scale;
-  if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
-  return s - slope * (float)dist;
-}
-
-// The factor of value i of head h in token t's output: a gate per head or per value, or none.
-template <typename T>
-__device__ __forceinline__ float att_gate(const AttArgs<T>& a, int t, int h, int i) {
-  if (!a.gate) return 1.f;
-  const size_t at = (size_t)t * a.gate_stride + (a.gate_dim > 0 ? (size_t)h * a.gate_dim + i : h);
-  return sigmoid_f32(to_f32<T>(a.gate[at]));
 }
 
 // ---------------------------------------------------------------------------- few new tokens
@@ -450,7 +411,8 @@ static int launch_few(const AttArgs<T>& a, int tokens, int per_seq, int sms, cud
 
 template <typename T>
 __global__ void __launch_bounds__(ATM_THREADS, 2)
-attention_many_kernel(const AttArgs<T> a, int fewest) {   // fewest: new tokens of a sequence
+attention_many_kernel(const AttArgs<T> a, int fewest, const int* __restrict__ redo) {
+  // fewest: new tokens of a sequence; redo: [B][tiles of 128][heads], the tiles to do (null: all)
   mb_grid_wait();
   mb_grid_launch_next();
   extern __shared__ __align__(16) float sm[];
@@ -463,6 +425,7 @@ attention_many_kernel(const AttArgs<T> a, int fewest) {   // fewest: new tokens 
   const int tiles = (n_new + ATM_ROWS - 1) / ATM_ROWS;
   if ((int)blockIdx.y >= tiles || n_new < fewest) return;
   const int r0 = (tiles - 1 - blockIdx.y) * ATM_ROWS;   // the tiles that see the most keys first
+  if (redo && !redo[((size_t)b * ((gridDim.y * ATM_ROWS + 127) / 128) + r0 / 128) * a.nh + h]) return;
   const int cnt = min(ATM_ROWS, n_new - r0);
   const int slot = a.seq_slot[b], p0 = a.tok_pos[t0 + r0];   // row r stands at position p0 + r
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -615,14 +578,14 @@ attention_many_kernel(const AttArgs<T> a, int fewest) {   // fewest: new tokens 
 }
 
 template <typename T>
-static int launch_many(const AttArgs<T>& a, int B, int max_new, int fewest, cudaStream_t s) {
+static int launch_many(const AttArgs<T>& a, int B, int max_new, int fewest, const int* redo, cudaStream_t s) {
   const int pitch = a.hd + 4, kv_pitch = pitch > a.vd ? pitch : a.vd;
   const size_t smem = (size_t)ATM_ROWS * (pitch + kv_pitch + ATM_PITCH) * sizeof(float);
   static unsigned long long allowed = 0;      // heads of 128: 85 KB
   const cudaError_t e = mb_allow_smem((const void*)attention_many_kernel<T>, 88 * 1024, &allowed);
   if (e != cudaSuccess) MB_FAIL("mb_attention_simt: %s", cudaGetErrorString(e));
   mb_launch(attention_many_kernel<T>, dim3(a.nh, (max_new + ATM_ROWS - 1) / ATM_ROWS, B),
-            dim3(ATM_THREADS), smem, s, a, fewest);
+            dim3(ATM_THREADS), smem, s, a, fewest, redo);
   MB_CHECK_LAUNCH("mb_attention_simt");
 }
 
@@ -636,7 +599,9 @@ static int launch_many(const AttArgs<T>& a, int B, int max_new, int fewest, cuda
 // float32 [nh] or null: slopes[h] * (query's position - key's position) is taken off every
 // score of head h after the cap. `keep_first` > 0: with a window, the first keep_first
 // positions of a sequence stay visible to every later one. `few_new`: the most new tokens of a
-// sequence that brings fewer than ATT_MANY of them (0: there is none).
+// sequence that brings fewer than ATT_MANY of them (0: there is none). `redo`: null, or room for an
+// int per sequence, 128 of max_new tokens (rounded up) and head: many new tokens of float32 heads of
+// 128 values then go through the tensor cores (attention_split.cuh). `error`: its waits' error word.
 MB_EXPORT int mb_attention_simt(const void* q, int q_stride, void* out, int out_stride,
                                 const void* kpool, const void* vpool, int dtype,
                                 const int* page_table, int max_pages, int ring_pages,
@@ -645,7 +610,7 @@ MB_EXPORT int mb_attention_simt(const void* q, int q_stride, void* out, int out_
                                 int T, int nh, int nkv, int hd, int window, float scale,
                                 int vd, const float* sink, float softcap, const void* gate,
                                 int gate_stride, int gate_dim, const float* slopes, int keep_first,
-                                int sms, void* stream) {
+                                int sms, int* redo, int* error, void* stream) {
   if (T <= 0) return 0;
   if (vd <= 0) vd = hd;
   if (hd <= 0 || hd > 1024 || vd > 32 * ATT_MAX_D)
@@ -671,7 +636,10 @@ MB_EXPORT int mb_attention_simt(const void* q, int q_stride, void* out, int out_
                            nkv, hd, vd, window, gate_stride, gate_dim, keep_first, scale,     \
                            softcap};                                                          \
     if (mixed && launch_few<T_>(a, B * few_new, few_new, sms, s)) return -1;                  \
-    return many ? launch_many<T_>(a, B, max_new, mixed ? ATT_MANY : 0, s)                     \
+    const int fewest = mixed ? ATT_MANY : 0;                                                  \
+    if (!many || hd != 128 || vd != 128 || sizeof(T_) != 4) redo = nullptr;                   \
+    if (redo && launch_split(a, B, max_new, fewest, redo, error, s)) return -1;               \
+    return many ? launch_many<T_>(a, B, max_new, fewest, redo, s)                             \
                 : launch_few<T_>(a, T, 0, sms, s);                                            \
   }
     if (dtype == MB_F32) GOA(float) else GOA(__nv_bfloat16)

@@ -67,6 +67,8 @@ EXTRA_HEADERS = {"gemm_tc": ["tc_common.cuh"],
                  "attention_diff": ["attention_mma.cuh", "mma_common.cuh", "tc_common.cuh"],
                  "state_walk": ["state_chunks.cuh", "mma_common.cuh"],
                  "gemm_split": ["attention_tc.cuh", "tc_common.cuh"],
+                 "attention_simt": ["attention_simt.cuh", "attention_split.cuh", "attention_tc.cuh",
+                                    "tc_common.cuh"],
                  "attention_tc": ["attention_tc.cuh", "tc_common.cuh"],
                  "attention_diff_tc": ["attention_tc.cuh", "tc_common.cuh"],
                  "latent": ["mma_common.cuh", "mma_tile.cuh"],

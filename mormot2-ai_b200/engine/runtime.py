@@ -178,4 +178,4 @@ class Runtime:
                                   gate_dim):
                 return
         K.attention_simt(q, q_stride, out, step, line, nh, nkv, hd, window, scale, vd, sink,
-                         softcap, gate, gate_stride, slopes, keep_first, gate_dim)
+                         softcap, gate, gate_stride, slopes, keep_first, gate_dim, self.error_word)

@@ -1384,7 +1384,14 @@ def gemm_split(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int 
 
 
 # ------------------------------------------------------------------------------ attention
-ATTENTION_MANY = 16      # ATT_MANY of csrc/attention_simt.cu
+ATTENTION_MANY = 16      # ATT_MANY of csrc/attention_simt.cuh
+# Many new float32 tokens of heads of 128 values go through the tensor cores where some token sees so many
+# keys: a page of 64 costs a tile there 6 us, in multiply-adds 16 to 24, but the way into and out of
+# tensor memory and the launch behind cost 12 and the host 5. Us with multiply-adds | on the tensor cores,
+# 16 heads on 8: one prompt of 64 27 | 30, of 100 40 | 37, eight of 40 after 100 56 | 46, one of 20 after
+# 1,000 280 | 99, two of 1,000 371 | 115, one of 2,048 693 | 174; a whole layer (0.6B shape) over 128
+# tokens 138 | 143, over 160 158 | 143.
+ATTENTION_SPLIT = 129
 
 
 def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, step, line, nh, nkv, hd,
@@ -1392,7 +1399,7 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, step, line
                    sink: Optional[torch.Tensor] = None, softcap: float = 0.0,
                    gate: Optional[torch.Tensor] = None, gate_stride: int = 0,
                    slopes: Optional[torch.Tensor] = None, keep_first: int = 0,
-                   gate_dim: int = 0) -> None:
+                   gate_dim: int = 0, error: Optional[torch.Tensor] = None) -> None:
     """``vd``: the size of a value row when it differs from ``hd``. ``sink``: float32 [nh],
     one more term exp(sink[h]) in the softmax denominators of head h. ``softcap`` > 0: scores
     become softcap * tanh(score / softcap). ``gate``: logits of q's type, head h of token t at
@@ -1410,15 +1417,23 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, step, line
     # sequences that bring few tokens beside one that brings many (see the file)
     few = max((n for n in step.host_new if n < ATTENTION_MANY), default=0) if (
         step.max_new >= ATTENTION_MANY and step.B > 1 and max(hd, vd) <= 128) else 0
+    redo = None
+    if (out.dtype == torch.float32 and hd == 128 and vd in (0, 128)
+            and step.max_new >= ATTENTION_MANY
+            and max(min(n + p, n + window) if window > 0 else n + p
+                    for n, p in zip(step.host_new, step.host_past) if n >= ATTENTION_MANY)
+            >= ATTENTION_SPLIT):
+        redo = torch.empty(step.B * nh * -(-step.max_new // 128), dtype=torch.int32, device=out.device)
     _call("attention_simt", "mb_attention_simt",
           [_vp, _i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
-           _i, _i, _f, _i, _vp, _f, _vp, _i, _i, _vp, _i, _i, _vp],
+           _i, _i, _f, _i, _vp, _f, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _vp],
           _ptr(q), q_stride, _ptr(out), out.stride(0), _ptr(line.k), _ptr(line.v),
           code_of(out.dtype), _ptr(line.page_table), line.max_pages, line.ring_pages,
           _ptr(step.tok_seq), _ptr(step.tok_pos), _ptr(step.seq_slot), _ptr(step.seq_start), step.B,
           step.max_new, few, T, nh, nkv, hd,
           window, float(scale), vd or hd, _ptr(sink), float(softcap), _ptr(gate), gate_stride,
-          int(gate_dim), _ptr(slopes), int(keep_first), _sms(), _stream(), launches=2 if few else 1)
+          int(gate_dim), _ptr(slopes), int(keep_first), _sms(), _ptr(redo), _ptr(error), _stream(),
+          launches=1 + (few > 0) + (redo is not None))
 
 
 # ------------------------------------------------------------------------------ sampling
