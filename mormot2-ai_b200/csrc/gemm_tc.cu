@@ -243,15 +243,6 @@ __device__ __forceinline__ void staged_rows(uint32_t taddr, uint32_t stage_w, in
     if (acc_cols == 32) {
       float* dst = mode == TC_PARTIAL ? part : (float*)C;
       const long long ld = mode == TC_PARTIAL ? partial_ld : ldc;
-      float4 old[8];
-      if (mode == TC_ADD) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = 4 * i + (lane >> 3);
-          if (pc < pieces && row0 + r < M)
-            old[i] = *(const float4*)(dst + (size_t)(row0 + r) * ld + n0 + c0 + 4 * pc);
-        }
-      }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = 4 * i + (lane >> 3);
@@ -259,7 +250,6 @@ __device__ __forceinline__ void staged_rows(uint32_t taddr, uint32_t stage_w, in
           const uint4 u = ld_shared_v4(stage_w + r * 128 + ((pc ^ (r & 7)) << 4));
           float4 o = make_float4(__uint_as_float(u.x), __uint_as_float(u.y),
                                  __uint_as_float(u.z), __uint_as_float(u.w));
-          if (mode == TC_ADD) { o.x += old[i].x; o.y += old[i].y; o.z += old[i].z; o.w += old[i].w; }
           *(float4*)(dst + (size_t)(row0 + r) * ld + n0 + c0 + 4 * pc) = o;
         }
       }
@@ -276,6 +266,77 @@ __device__ __forceinline__ void staged_rows(uint32_t taddr, uint32_t stage_w, in
     __syncwarp();  // the rows are read out before the next columns are laid over them
   }
 }
+
+// The same for a sum into a float32 residual, 32 columns at a time: what stands in the next 32 is asked
+// for before the accumulator's columns are read out, what stands in the first before the accumulator is
+// waited for, and the whole rows are brought into L2 meanwhile. Two or more pieces ahead are slower
+// (a wait for one piece then waits for the later ones' loads too). 2,048 tokens, a graph of ten, asking
+// as it goes -> this: 2,048 x 2,048 24.9 -> 21.0 us, 4,096 x 2,048 35.1 -> 29.0; 4,096 x 256, which is
+// all epilogue, 25.2 -> 18.1; two pieces ahead 32.4.
+struct AddRows {
+  float4 old[8];
+  float* at;          // this lane's place in the tile's first row and piece
+  long long ld;
+  int rows, cols, lane;      // rows from this warp's first on, columns of the tile
+
+  __device__ __forceinline__ void ask(int c) {
+    const bool ok = c + 4 * (lane & 7) < cols;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+          "@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}\n"
+          : "+f"(old[i].x), "+f"(old[i].y), "+f"(old[i].z), "+f"(old[i].w)
+          : "l"(at + c + 4 * i * ld), "r"((int)(ok && 4 * i + (lane >> 3) < rows))
+          : "memory");
+  }
+  __device__ __forceinline__ void ask_first(float* C, long long ldc, int lane_, int row0, int n0, int width,
+                                            int M, int N) {
+    lane = lane_;
+    ld = ldc;
+    rows = M - row0;
+    cols = min(width, N - n0);
+    at = C + (size_t)(row0 + (lane >> 3)) * ldc + n0 + 4 * (lane & 7);
+    if (lane < rows)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                   ::"l"(C + (size_t)(row0 + lane) * ldc + n0), "r"(cols * 4) : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ask(0);
+  }
+  __device__ __forceinline__ void finish(uint32_t taddr, uint32_t stage_w) {
+    const uint32_t mine = stage_w + lane * 128;
+    const int pc = lane & 7;
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 32) {
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        if (c + 16 * g >= cols) break;
+        float v[16];
+        tmem_ld16(taddr + c + 16 * g, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          st_shared_v4(mine + (((4 * g + j) ^ (lane & 7)) << 4),
+                       make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]),
+                                  __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3])));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3);
+        if (c + 4 * pc < cols && r < rows) {
+          const uint4 u = ld_shared_v4(stage_w + r * 128 + ((pc ^ (r & 7)) << 4));
+          const float4 was = old[i];
+          *(float4*)(at + c + 4 * i * ld) =
+              make_float4(__uint_as_float(u.x) + was.x, __uint_as_float(u.y) + was.y,
+                          __uint_as_float(u.z) + was.z, __uint_as_float(u.w) + was.w);
+        }
+      }
+      ask(c + 32);
+      __syncwarp();  // the rows are read out before the next columns are laid over them
+    }
+  }
+};
 
 // rowsA x rowsB outputs: element (a, b) is the dot product of row a of the lanes' operand and
 // row b of the columns' operand. SWAP false: C[a * ldc + b]; true: C[b * ldc + a].
@@ -413,20 +474,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     mb_grid_wait();
     const int q = warp & 3;  // the TMEM lanes a warp may read: 32 * (warp % 4) ..
     const int lane_row = q * 32 + lane;
+    const bool add_rows = !SWAP && staged && mode == TC_ADD && !act;
     int it = 0;
     for (int w = blockIdx.x; w < num_tiles; w += gridDim.x, ++it) {
       const int rem = w % tiles_ab, z = w / tiles_ab;
       const int m0 = (rem % tiles_a) * tile_rows, n0 = (rem / tiles_a) * BN;
       const int b = it & 1;
+      const int a = m0 + lane_row;
+      AddRows add;
+      if (add_rows) add.ask_first((float*)C, ldc, lane, a - lane, n0, BN, rowsA, rowsB);
       mbar_wait(acc_full0 + 8 * b, (it >> 1) & 1, error, 3);
       tc_fence_after_sync();
-      const int a = m0 + lane_row;
       const bool mine = lane_row < tile_rows && a < rowsA;
       const uint32_t taddr = tmem + b * Cfg::COLS + ((uint32_t)(q * 32) << 16);
       float* part = partial ? partial + z * partial_stride : nullptr;
       if (staged) {
-        staged_rows(taddr, stage_w, lane, a - lane, n0, BN, rowsA, rowsB, C, c_dtype, ldc, mode,
-                    part, partial_ld, act);
+        if (add_rows) add.finish(taddr, stage_w);
+        else
+          staged_rows(taddr, stage_w, lane, a - lane, n0, BN, rowsA, rowsB, C, c_dtype, ldc, mode,
+                      part, partial_ld, act);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty0 + 8 * b);
@@ -655,6 +721,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   } else {
     const int q = warp & 3;
     const int lane_row = q * 32 + lane;
+    const bool add_rows = staged && mode == TC_ADD && !act;
     int it = 0;
     for (int w = pair; w < num_tiles; w += pairs, ++it) {
       const int z = w / tiles_mn;
@@ -662,6 +729,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int n0 = mn.y * BN;
       const int a = mn.x * 256 + (int)rank * 128 + lane_row;
       const int b = in_parts ? 0 : it & 1;
+      AddRows add;
+      if (add_rows) add.ask_first((float*)C, ldc, lane, a - lane, n0, BN, M, N);
       mbar_wait(acc_full0 + 8 * b, (it >> 1) & 1, error, 13);
       tc_fence_after_sync();
       if (in_parts) {
@@ -683,7 +752,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
       const uint32_t taddr = tmem + b * TC2_COLS + ((uint32_t)(q * 32) << 16);
       float* part = partial ? partial + z * partial_stride : nullptr;
-      if (staged) {
+      if (add_rows) {
+        add.finish(taddr, stage_w);
+      } else if (staged) {
         staged_rows(taddr, stage_w, lane, a - lane, n0, BN, M, N, C, c_dtype, ldc, mode, part,
                     partial_ld, act);
       } else {
