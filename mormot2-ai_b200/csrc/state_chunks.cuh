@@ -17,12 +17,17 @@
 // Products go through mma.sync (m16n8k16) with every float32 value cut into three exact bfloat16
 // parts (common.cuh), six products of parts, the smallest first: an accumulator cuts off what falls
 // behind its last place, so the leading products come last and few to an accumulator, and sums over
-// warps and chunks are made with float32 additions. Decays are products, never quotients. The state
+// warps and chunks are made with float32 additions. What goes into the state chunk after chunk leans to
+// neither side: the first operand's leading part is the nearest one, and what an accumulator cut off its
+// leading products is made once more and added (2,000 tokens, 128 x 128, delta, the mean over three
+// inputs of the state's relative error against float64: by fours 1.16e-7, this 1.08e-7; on the first of
+// them 0.94e-7 and 1.20e-7, without either 1.67e-7). Decays are products, never quotients. The state
 // stands as fragments in registers, transposed, so that a chunk's result is the next one's operand.
 // What bounds the walk: a chunk's chain of two rounds of MMAs, two barriers and a sum over the warps
 // (some 4,000 cycles, of which the tensor pipe works 1,500); the preparing blocks: instructions (issue
 // slots half busy, most of them cut values). One prompt of 2,048 tokens, 16 heads of 128 x 128, delta:
-// by fours 366 us -> 56 + 150; four prompts of 111 to 900, 8 heads, mlstm: 185 -> 23 + 86. With the
+// by fours 366 us -> 56 + 150; four prompts of 111 to 900, 8 heads, mlstm: 185 -> 23 + 86 (before what
+// keeps the sums from leaning was added: 9 and 7 us more; the whole mixers 491 -> 323, 261 -> 180). With the
 // operands in shared memory and cut there a chunk took twice the instructions (97 + 234 us).
 // What is no number (an infinity, a NaN, an overflow) goes through a form that takes the chunk token
 // by token, so that it reaches no earlier token.
@@ -47,8 +52,18 @@ __host__ __device__ inline size_t sc_chunk_floats(bool delta, int D, int DV) {
 
 struct FragA { uint32_t hi[4], mid[4], lo[4]; };
 struct FragB { uint32_t hi[2], mid[2], lo[2]; };
+// The first operand's cut: the first part is the nearest, so that what the six products leave out (its
+// rest times the second operand's) has either sign
+__device__ __forceinline__ Cut2 cut_near(float a, float b) {
+  Cut2 c;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(c.hi) : "f"(b), "f"(a));
+  const f32_pair v = pair_of(a - __uint_as_float(c.hi << 16), b - __uint_as_float(c.hi & 0xffff0000u));
+  c.mid = upper_halves(v);
+  c.lo = upper_halves(pair_sub_upper(v));
+  return c;
+}
 __device__ __forceinline__ void put_a(FragA& f, int i, float a, float b) {
-  const Cut2 c = cut(a, b);
+  const Cut2 c = cut_near(a, b);
   f.hi[i] = c.hi; f.mid[i] = c.mid; f.lo[i] = c.lo;
 }
 __device__ __forceinline__ void put_b(FragB& f, int i, float a, float b) {
@@ -75,6 +90,20 @@ template <int N> __device__ __forceinline__ void mma_low(float (*d)[4], const Fr
 template <int N> __device__ __forceinline__ void mma_high(float (*d)[4], const FragA& a, const FragB* b) {
 #pragma unroll
   for (int i = 0; i < N; ++i) mma_parts(d[i], a.hi, b[i].hi);
+}
+// The leading products, to which an accumulator that starts at zero leaves what it cuts off: the same
+// products again less their sum
+template <int N> __device__ __forceinline__ void mma_rest(float (*low)[4], const float (*high)[4], const FragA& a, const FragB* b) {
+  float d[N][4];
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[i][e] = -high[i][e];
+  mma_high<N>(d, a, b);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) low[i][e] += d[i][e];
 }
 __device__ __forceinline__ void store_frag(float* at, int lane, const FragB& f) {
   ((uint4*)at)[lane] = make_uint4(f.hi[0], f.hi[1], f.mid[0], f.mid[1]);
@@ -413,11 +442,17 @@ state_chunk_prep_kernel(const WalkArgs g, float* __restrict__ scratch, int chunk
         }
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
-      float acc[2][4] = {};
+      float acc[2][4] = {}, h0[2][4] = {}, h1[2][4] = {};
       mma_low<2>(acc, a[mt][0], f[0]);
       if (mt) mma_low<2>(acc, a[mt][1], f[1]);      // T is zero above its diagonal
-      mma_high<2>(acc, a[mt][0], f[0]);
-      if (mt) mma_high<2>(acc, a[mt][1], f[1]);
+      mma_high<2>(h0, a[mt][0], f[0]);
+      if (mt) mma_high<2>(h1, a[mt][1], f[1]);
+      mma_rest<2>(acc, h0, a[mt][0], f[0]);
+      if (mt) mma_rest<2>(acc, h1, a[mt][1], f[1]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = h0[j][e] + (h1[j][e] + acc[j][e]);
       if (is_u) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -556,7 +591,7 @@ state_chunk_walk_kernel(const WalkArgs g, const float* __restrict__ scratch, int
         if (!DELTA && (norm_col || t >= cn)) u = make_float4(my_col == 0 && t < cn ? 1.f : 0.f, 0.f, 0.f, 0.f);
         if (DELTA) u = make_float4(u.x - v.x, u.y - v.y, u.z - v.z, u.w - v.w);
         odd |= no_number(u);
-        const Cut2 a = cut(u.x, u.y), z = cut(u.z, u.w);
+        const Cut2 a = cut_near(u.x, u.y), z = cut_near(u.z, u.w);
         unsigned short* h = (unsigned short*)up + my_col * 40 + t;
         const uint32_t words[6] = {a.hi, z.hi, a.mid, z.mid, a.lo, z.lo};
 #pragma unroll
@@ -642,13 +677,19 @@ state_chunk_walk_kernel(const WalkArgs g, const float* __restrict__ scratch, int
         ua[k].lo[e] = at[2 * 16 * 20];
       }
     // U^T times k of this warp's rows, and times N of eight tokens: three accumulators
-    float acc[3][4] = {};
+    float acc[3][4] = {}, h0[3][4] = {}, h1[3][4] = {};
     {
       const FragB f0[3] = {fk[0], fk[2], fn[0]}, f1[3] = {fk[1], fk[3], fn[1]};
       mma_low<3>(acc, ua[0], f0);
       mma_low<3>(acc, ua[1], f1);
-      mma_high<3>(acc, ua[0], f0);
-      mma_high<3>(acc, ua[1], f1);
+      mma_high<3>(h0, ua[0], f0);
+      mma_high<3>(h1, ua[1], f1);
+      mma_rest<3>(acc, h0, ua[0], f0);
+      mma_rest<3>(acc, h1, ua[1], f1);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = h0[i][e] + (h1[i][e] + acc[i][e]);
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j)

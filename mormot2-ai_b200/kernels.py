@@ -686,7 +686,8 @@ def walks_in_chunks(step, dim: int, vdim: int, mode: int, heads: int) -> bool:
     370; 63 decoding beside 256 284 | 580. 8 heads of 64 x 128, three prompts of 64 / 128 24 | 26, 36 |
     31, eight of 128 / 200 46 | 46, 63 | 71. Matrix memory, 8 heads of 128 x 128, one prompt of 64 / 96 /
     1,000: 28 | 25, 30 | 27, 164 | 111; eight of 64 / 400 61 | 38, 245 | 123; 63 decoding beside 128
-    153 | 111; 4 heads of 64 x 64, one of 64 / 96 22 | 21, 26 | 24."""
+    153 | 111; 4 heads of 64 x 64, one of 64 / 96 22 | 21, 26 | 24. (Chunks: before their sums were kept
+    from leaning, which takes 3 to 4 in a hundred.)"""
     if mode not in (WALK_DELTA, WALK_MLSTM) or dim % 16 or dim > 128 or vdim % 16:
         return False
     n, pairs = step.max_new, step.B * heads

@@ -57,6 +57,24 @@ def test_long_sequences_as_by_fours(monkeypatch, mode):
     assert torch.equal(state32[0], start[0]) and torch.equal(state32[4], start[4])
 
 
+# Sums that lean to one side add up over the chunks: the delta rule's states and outputs are as near to
+# float64 as by fours, in the mean over three inputs (a tenth more: what the mean of three can vary by)
+def test_as_near_to_float64_as_by_fours(monkeypatch):
+    heads, dim, lens, real = 2, 128, [2000], walk.rows
+    errors = {False: [0.0, 0.0], True: [0.0, 0.0]}
+    for more in (0, 100, 200):
+        monkeypatch.setattr(walk, "rows", lambda shape, seed, *a, **k: real(shape, seed + more, *a, **k))
+        start = walk.rows((1, heads * dim * dim), 9, 0.3)
+        want, states = walk.plain("delta", start, lens, heads, dim, dim, 1, lens[0])
+        for chunks in (False, True):
+            route(monkeypatch, chunks)
+            state, step = start.clone(), make_step([(0, 5, [0] * lens[0], [])])
+            out = walk.run("delta", step, state, lens[0], heads, dim, dim, 1, 0, torch.float32)
+            for i, (got, ref) in enumerate(((out, want), (state, states))):
+                errors[chunks][i] += float((got.double().cpu() - ref).norm() / ref.norm())
+    assert errors[True][0] <= 1.1 * errors[False][0] and errors[True][1] <= 1.1 * errors[False][1]
+
+
 # an infinity among the values or the keys of a token, or in the state
 @pytest.mark.parametrize("mode", ["delta", "mlstm"])
 @pytest.mark.parametrize("what", ["value", "key", "state"])
