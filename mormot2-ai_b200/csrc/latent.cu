@@ -103,10 +103,12 @@ latent_prep_kernel(const T* __restrict__ f, int ld, int q_col, int kv_col, int q
     dst[kv_rank + i] = from_f32<T>(rotated(br, i, rot_dims, inv_freq, pos, amplitude));
 }
 
-// The same for steps of many tokens in bfloat16, a warp a token: 16 bytes a lane and load, all of a
-// row's on their way at once with the norms' weights, and no barrier. Rows of up to 256 LQ and 256 LC
-// values. Bound by its 5.2 bytes a value; 2,048 tokens of 768 and 512 + 64 values, a block of 128
-// threads a token 20.6 us from memory (a chain of loads, sums and barriers), a warp 7.0.
+// The same for steps of many tokens in bfloat16, a warp a token: all of a row on its way at once with the
+// norms' weights, and no barrier. A lane has the values 4 lane + 128 j .. + 3: those of four neighbouring
+// threads of the block of 128 above, added up in the same chains and the same order, so that both forms
+// give the same bits. Rows of up to 256 LQ and 256 LC values. Bound by its 5.2 bytes a value; 2,048
+// tokens of 768 and 512 + 64 values, a graph of eight: a block a token 12.3 us (a chain of loads, sums
+// and barriers), a warp 4.0; 256 tokens 6.6 and 3.5; the latent attention mixer 173 -> 162.
 template <int LQ, int LC>
 __global__ void __launch_bounds__(256)
 latent_prep_rows_kernel(const __nv_bfloat16* __restrict__ f, int ld, int q_col, int kv_col, int q_rank,
@@ -123,66 +125,73 @@ latent_prep_rows_kernel(const __nv_bfloat16* __restrict__ f, int ld, int q_col, 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * 8 + warp;
   if (t >= T) return;
   const __nv_bfloat16* row = f + (size_t)t * ld;
-  uint4 q[LQ], c[LC], wq[LQ], wc[LC];
-  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  uint2 q[2 * LQ], c[2 * LC], wq[2 * LQ], wc[2 * LC];
+  const uint2 none = make_uint2(0u, 0u);
 #pragma unroll
-  for (int j = 0; j < LQ; ++j) {
-    const int i = 8 * lane + 256 * j;
-    q[j] = i < q_rank ? *(const uint4*)(row + q_col + i) : none;
-    wq[j] = i < q_rank ? *(const uint4*)(w_q + i) : none;
+  for (int j = 0; j < 2 * LQ; ++j) {
+    const int i = 4 * lane + 128 * j;
+    q[j] = i < q_rank ? *(const uint2*)(row + q_col + i) : none;
+    wq[j] = i < q_rank ? *(const uint2*)(w_q + i) : none;
   }
 #pragma unroll
-  for (int j = 0; j < LC; ++j) {
-    const int i = 8 * lane + 256 * j;
-    c[j] = i < kv_rank ? *(const uint4*)(row + kv_col + i) : none;
-    wc[j] = i < kv_rank ? *(const uint4*)(w_kv + i) : none;
+  for (int j = 0; j < 2 * LC; ++j) {
+    const int i = 4 * lane + 128 * j;
+    c[j] = i < kv_rank ? *(const uint2*)(row + kv_col + i) : none;
+    wc[j] = i < kv_rank ? *(const uint2*)(w_kv + i) : none;
   }
   for (int i = lane; i < rot_dim; i += 32) turn[warp][i] = __bfloat162float(row[kv_col + kv_rank + i]);
   const int pos = tok_pos[t], slot = tok_slot[t];
-  // the sum of squares: eight chains a lane, then by pairs
-  auto normed = [&](const uint4* v, int n, int size, float& inv) {
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  auto normed = [&](const uint2* v, int n, int size, float& inv) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < n; ++j) {
-      const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+      const uint32_t w[2] = {v[j].x, v[j].y};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2; ++e) {
         const float a = __uint_as_float(w[e] << 16), b = __uint_as_float(w[e] & 0xffff0000u);
         s[2 * e] = fmaf(a, a, s[2 * e]);
         s[2 * e + 1] = fmaf(b, b, s[2 * e + 1]);
       }
     }
-    const float sum = warp_sum(((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+    // block_sum's order: eight lanes are a warp of the block, whose sums meet 16, 8, 4, 2 and 1 threads
+    // apart; then the four warps' sums, two and one apart
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+    float sum = (s[0] + s[2]) + (s[1] + s[3]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
     inv = 1.0f / sqrtf(sum / (float)size + eps);
   };
-  auto put = [&](__nv_bfloat16* to, const uint4& v, const uint4& w, float inv) {
-    const uint32_t x[4] = {v.x, v.y, v.z, v.w}, y[4] = {w.x, w.y, w.z, w.w};
-    uint32_t o[4];
+  auto put = [&](__nv_bfloat16* to, const uint2& v, const uint2& w, float inv) {
+    const uint32_t x[2] = {v.x, v.y}, y[2] = {w.x, w.y};
+    uint32_t o[2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int e = 0; e < 2; ++e) {
       const __nv_bfloat162 r = __floats2bfloat162_rn(
           __uint_as_float(y[e] << 16) * (__uint_as_float(x[e] << 16) * inv),
           __uint_as_float(y[e] & 0xffff0000u) * (__uint_as_float(x[e] & 0xffff0000u) * inv));
       o[e] = *(const uint32_t*)&r;
     }
-    *(uint4*)to = make_uint4(o[0], o[1], o[2], o[3]);
+    *(uint2*)to = make_uint2(o[0], o[1]);
   };
   float inv_q, inv_c;
   if (q_rank > 0) {
-    normed(q, LQ, q_rank, inv_q);
+    normed(q, 2 * LQ, q_rank, inv_q);
 #pragma unroll
-    for (int j = 0; j < LQ; ++j) {
-      const int i = 8 * lane + 256 * j;
+    for (int j = 0; j < 2 * LQ; ++j) {
+      const int i = 4 * lane + 128 * j;
       if (i < q_rank) put(cq_out + (size_t)t * q_rank + i, q[j], wq[j], inv_q);
     }
   }
   if (!write_cache) return;
   __nv_bfloat16* dst = pool + kv_row(page_table, max_pages, ring_pages, slot, pos, 1, 0) *
                                   (size_t)(kv_rank + rot_dim);
-  normed(c, LC, kv_rank, inv_c);
+  normed(c, 2 * LC, kv_rank, inv_c);
 #pragma unroll
-  for (int j = 0; j < LC; ++j) {
-    const int i = 8 * lane + 256 * j;
+  for (int j = 0; j < 2 * LC; ++j) {
+    const int i = 4 * lane + 128 * j;
     if (i < kv_rank) put(dst + i, c[j], wc[j], inv_c);
   }
   __syncwarp();

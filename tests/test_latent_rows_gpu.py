@@ -47,3 +47,26 @@ def test_latent_rows(T, qr, kvr, rd, dims, shift):
     for g in got:
         assert ((g - want).abs() <= (2.0 ** -8 + 1e-5) * want.abs() + 2e-4).all()
     assert (got[0] - got[1]).norm() <= 1e-4 * want.norm()      # other sums: few values round otherwise
+
+
+# both forms add the squares up in the same order: a step of many tokens leaves the bits that steps of few leave
+@pytest.mark.parametrize("T", [256, 777])
+@pytest.mark.parametrize("qr, kvr, rd, dims", [(768, 512, 64, 64), (512, 256, 32, 32), (1024, 264, 40, 24), (0, 128, 64, 32),
+                                               (8, 8, 8, 0), (136, 24, 16, 16)])
+def test_the_bits_of_few_tokens(T, qr, kvr, rd, dims):
+    gen = torch.Generator().manual_seed(T + qr)
+    draw = lambda *s: torch.randn(s, generator=gen).bfloat16().to(DEV)
+    f, wq, wkv = draw(T, qr + kvr + rd), draw(max(qr, 1)), draw(kvr)
+    f[3] *= 1e-3      # the norm's eps counts
+    f[5, 0] = float("inf")
+    inv_freq = torch.rand(max(dims // 2, 1), generator=gen).to(DEV)
+    got = []
+    for n in (T, 100):
+        line = make_line(1, T, 1, kvr + rd, torch.bfloat16, seed=3)
+        cq = torch.zeros((T, qr), dtype=torch.bfloat16, device=DEV)
+        for a in range(0, T, n):
+            m = min(n, T - a)
+            K.latent_prep(f[a:a + m], 0, qr, qr, kvr, rd, wq, wkv, 1e-5, inv_freq, dims, 1.0,
+                          make_step([(0, a, [0] * m, [])]), line, cq[a:a + m], True)
+        got.append(torch.cat([cq.flatten().view(torch.int16), line.k.flatten().view(torch.int16)]))
+    assert torch.equal(got[0], got[1])
