@@ -233,15 +233,20 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// v[i] summed over the warp's lanes, value i's sum in lane i: every round halves what a lane keeps.
-__device__ __forceinline__ float sum32_by_lane(float* v, int lane) {
+// The `N` values of v summed over the warp's lanes, value i's sum in the 32 / N lanes from 32 / N i on:
+// every round halves what a lane keeps.
+template <int N> __device__ __forceinline__ float sums_by_lane(float* v, int lane) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool up = lane & o;
+  for (int o = 16, n = N / 2; o > 0; o >>= 1, n >>= 1) {
+    if (n > 0) {
+      const bool up = lane & o;
 #pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      for (int i = 0; i < n; ++i) {
+        const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     }
   }
   return v[0];

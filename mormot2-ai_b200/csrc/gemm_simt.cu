@@ -106,11 +106,15 @@ gemm_swiglu_halves_kernel(const TA* __restrict__ A, int lda, const TW* __restric
 // work at a time, over the border from one group of rows to the next, and the blocks stay for the
 // whole weight, so that enough bytes are asked for at every moment; the rows of A lie in shared
 // memory where they fit (FEW_STAGED: two blocks a multiprocessor) and a warp has work enough, and come
-// four reads at a time elsewhere, with two chunks under way. The 32 sums are reduced by halves, a
-// value a lane at the end. A weight with few rows has KW warps of a block share each four rows along
-// K. Eight rows, float32, from memory, one chunk ahead and a block for every eight groups -> this
-// form: 151,936 x 1,024 163 -> 119 us (5.2 TB/s), 2 x 12,288 x 4,096 182 -> 123, 4,096 x 12,288 147 ->
-// 84, 2 x 3,072 x 1,024 27 -> 18.5, 1,024 x 3,072 18.5 -> 13.3.
+// four reads at a time elsewhere, with two chunks under way. One or two rows' values are asked for with
+// the weight's (four reads of which three are the same row's took a quarter longer). More than eight
+// rows take two passes, group by group where all rows lie in shared memory, else over the whole weight.
+// The 32 sums are reduced by halves, a value a lane at the end. A weight with few rows has KW warps of a
+// block share each four rows along K. Eight rows, float32, from memory, one chunk ahead and a block for
+// every eight groups -> this form: 151,936 x 1,024 163 -> 119 us (5.2 TB/s), 2 x 12,288 x 4,096 182 ->
+// 123, 4,096 x 12,288 147 -> 84, 2 x 3,072 x 1,024 27 -> 18.5, 1,024 x 3,072 18.5 -> 13.3. One row, in a
+// graph: 151,936 x 1,024 117 -> 89, 1,024 x 3,072 4.3 -> 3.5, 1,024 x 1,024 2.5 -> 2.4; nine rows,
+// 151,936 x 1,024 190 -> 154 (a walk through the weight for each pass: 190).
 // A weight row's values are used once: they pass by the L1 cache. Predicated, zeros where not `ok`: a
 // load behind a branch would be waited for where the branch ends.
 template <typename T> __device__ __forceinline__ float4 load4_once(const T* p, bool ok);
@@ -138,104 +142,170 @@ template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __
   return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
+// The same of a value that is used again
+template <typename T> __device__ __forceinline__ float4 load4_ok(const T* p, bool ok);
+template <> __device__ __forceinline__ float4 load4_ok<float>(const float* p, bool ok) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+      "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+      "@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}\n"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+      : "l"(p), "r"((int)ok)
+      : "memory");
+  return v;
+}
+template <> __device__ __forceinline__ float4 load4_ok<__nv_bfloat16>(const __nv_bfloat16* p, bool ok) {
+  uint2 raw;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t"
+      "@p ld.global.v2.u32 {%0, %1}, [%2];\n\t}\n"
+      : "=&r"(raw.x), "=&r"(raw.y)
+      : "l"(p), "r"((int)ok)
+      : "memory");
+  const float2 lo = __bfloat1622float2(*(const __nv_bfloat162*)&raw.x);
+  const float2 hi = __bfloat1622float2(*(const __nv_bfloat162*)&raw.y);
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
 #define FEW_ROWS 8   // rows of A in one pass
 #define FEW_MAX 16   // the most rows that take this kernel
 
 #define FEW_STAGED (96 * 1024)   // bytes of A's rows that still go into shared memory
 
-template <typename TA, typename TW, int EPI, bool STAGED>
+// ROWS: rows of A in one pass. TWO_PASSES (STAGED only): more than ROWS of them lie in shared memory, and
+// a group's weights are read for all passes before the next group's, the second time from L2.
+template <typename TA, typename TW, int EPI, int ROWS, bool STAGED, bool TWO_PASSES>
 __global__ void __launch_bounds__(256, 2)
 gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
                      void* __restrict__ C, int c_bf16, int ldc, int M, int N, int K, int KW,
                      int groups, int settled) {
   constexpr bool GLU = EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_PAIRS;
   constexpr int FEATS = GLU ? 2 : 4;  // output features of a warp
-  constexpr int DEPTH = STAGED ? 3 : 2;      // chunks under way or at work
-  extern __shared__ __align__(16) float As[];      // STAGED: [min(M, 8)][K]
+  constexpr bool AHEAD = ROWS <= 2;   // A's values are asked for with the weights'
+  constexpr int DEPTH = STAGED || AHEAD ? 3 : 2;      // chunks under way or at work
+  extern __shared__ __align__(16) float As[];      // STAGED: [rows of a walk through the weight][K]
   __shared__ float part[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per_block = 8 / KW, kw = warp % KW, step = gridDim.x * per_block;
   const int k_first = kw * 128 + lane * 4, k_step = KW * 128;
   const int chunks = (K + k_step - 1) / k_step;
   const int g_block = blockIdx.x * per_block, g0 = g_block + warp / KW;
-  // the chunk that is asked for next: its group, place and the group's four weight rows; a row beyond
-  // the weight is read as its last and not stored
-  int ask_g, ask_k;
+  // the chunk that is asked for next: its group and pass (rows of A), place and the group's four weight
+  // rows; a row beyond the weight is read as its last and not stored
+  int ask_g, ask_m, ask_k;
   const TW* wr[4];
   auto enter = [&](int g) {
     ask_g = g;
+    ask_m = 0;
     ask_k = k_first;
     const int n0 = g * FEATS;
+    if (g < groups) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int row;
-      if (EPI == EPI_SWIGLU) row = (j >> 1) * N + min(n0 + (j & 1), N - 1);     // g0 g1 u0 u1
-      else if (EPI == EPI_SWIGLU_PAIRS) row = 2 * min(n0 + (j >> 1), N - 1) + (j & 1);  // g0 u0 g1 u1
-      else row = min(n0 + j, N - 1);
-      wr[j] = W + (size_t)row * K;
+      for (int j = 0; j < 4; ++j) {
+        int row;
+        if (EPI == EPI_SWIGLU) row = (j >> 1) * N + min(n0 + (j & 1), N - 1);     // g0 g1 u0 u1
+        else if (EPI == EPI_SWIGLU_PAIRS) row = 2 * min(n0 + (j >> 1), N - 1) + (j & 1);  // g0 u0 g1 u1
+        else row = min(n0 + j, N - 1);
+        wr[j] = W + (size_t)row * K;
+      }
     }
   };
-  auto ask = [&](float4* w) {
+  struct Chunk { float4 w[4], a[AHEAD ? ROWS : 1]; };
+  auto ask_a = [&](Chunk& c, int k, bool ok) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = load4_once<TW>(wr[j] + ask_k, ask_k < K && ask_g < groups);
-    ask_k += k_step;
-    if (ask_k - k_first >= chunks * k_step) enter(ask_g + step);
+    for (int i = 0; i < ROWS; ++i) c.a[i] = load4_ok<TA>(A + (size_t)i * lda + k, ok && i < M);
   };
-  float4 w0[4], w1[4], w2[4];
+  auto ask = [&](Chunk& c, bool rows) {
+    const bool ok = ask_k < K && ask_g < groups;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c.w[j] = load4_once<TW>(wr[j] + ask_k, ok);
+    if (AHEAD && rows) ask_a(c, ask_k, ok);
+    ask_k += k_step;
+    if (ask_k - k_first >= chunks * k_step) {
+      ask_k = k_first;
+      if (!TWO_PASSES || (ask_m += ROWS) >= M) enter(ask_g + step);
+    }
+  };
+  Chunk c0, c1, c2;
   auto begin = [&]() {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) wr[j] = W;
     enter(g0);
-    ask(w0);
-    ask(w1);
-    if (DEPTH > 2) ask(w2);
+    ask(c0, false);
+    ask(c1, false);
+    if (DEPTH > 2) ask(c2, false);
   };
   // the first chunks ahead of the wait, where the kernel before does not write the weight
   if (settled) begin();
   mb_grid_wait();
   mb_grid_launch_next();
   if (!settled) begin();
-  for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
-    const int rows = min(M - m0, FEW_ROWS);
-    if (m0) begin();
+  if (AHEAD) {
+    int k = k_first, left = chunks;
+    auto next = [&](Chunk& c) {
+      ask_a(c, k, k < K);
+      k += k_step;
+      if (--left == 0) { left = chunks; k = k_first; }
+    };
+    next(c0);
+    next(c1);
+    next(c2);
+  }
+  // walks through the weight, one for all rows (TWO_PASSES) or one for every ROWS of them
+  const int per_walk = TWO_PASSES ? M : ROWS;
+  for (int m_walk = 0; m_walk < M; m_walk += per_walk) {
+    const int walk_rows = min(M - m_walk, per_walk);
+    if (m_walk) begin();
     if (STAGED) {
-      if (m0) __syncthreads();
+      if (m_walk) __syncthreads();
       const int per_row = K >> 2;
-      for (int m = 0; m < rows; ++m)
+      for (int m = 0; m < walk_rows; ++m)
         for (int i = threadIdx.x; i < per_row; i += 256)
-          *(float4*)(As + m * K + 4 * i) = load4<TA>(A + (size_t)(m0 + m) * lda + 4 * i);
+          *(float4*)(As + m * K + 4 * i) = load4<TA>(A + (size_t)(m_walk + m) * lda + 4 * i);
       __syncthreads();
     }
-    float acc[4 * FEW_ROWS];
-    int g = g0, k = k_first, chunk = 0;
+    float acc[4 * ROWS];
+    int g = g0, m0 = 0, k = k_first, chunk = 0;
     bool more = g_block < groups;      // the same for the whole block
-    auto work = [&](float4* w) {
+    auto row_of = [&](const Chunk& c, float4 a, int m) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float& s = acc[j * ROWS + m];
+        s = fmaf(a.x, c.w[j].x, fmaf(a.y, c.w[j].y, fmaf(a.z, c.w[j].z, fmaf(a.w, c.w[j].w, s))));
+      }
+    };
+    auto work = [&](Chunk& c) {
       if (chunk == 0) {
 #pragma unroll
-        for (int j = 0; j < 4 * FEW_ROWS; ++j) acc[j] = 0.f;
+        for (int j = 0; j < 4 * ROWS; ++j) acc[j] = 0.f;
       }
-      if (k < K) {
+      const int rows = walk_rows - m0;      // ROWS of them, or what is left: the same for the block
+      if (AHEAD) {
+#pragma unroll
+        for (int m = 0; m < ROWS; ++m)
+          if (m < rows) row_of(c, c.a[m], m);
+      } else if (k < K) {
         constexpr int BATCH = STAGED ? 1 : 4;      // reads of A under way together
 #pragma unroll
-        for (int mb = 0; mb < FEW_ROWS; mb += BATCH) {
-          if (mb >= rows) break;  // uniform over the block
+        for (int mb = 0; mb < ROWS; mb += BATCH) {
+          if (mb >= rows) break;
           float4 a[BATCH];
 #pragma unroll
           for (int i = 0; i < BATCH; ++i)
-            a[i] = STAGED ? *(const float4*)(As + mb * K + k)
-                          : load4<TA>(A + (size_t)(m0 + min(mb + i, rows - 1)) * lda + k);
+            a[i] = STAGED ? *(const float4*)(As + (m0 + mb) * K + k)
+                          : load4<TA>(A + (size_t)(m_walk + min(mb + i, rows - 1)) * lda + k);
 #pragma unroll
-          for (int i = 0; i < BATCH; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float& s = acc[j * FEW_ROWS + mb + i];
-              s = fmaf(a[i].x, w[j].x, fmaf(a[i].y, w[j].y, fmaf(a[i].z, w[j].z, fmaf(a[i].w, w[j].w, s))));
-            }
+          for (int i = 0; i < BATCH; ++i) row_of(c, a[i], mb + i);
         }
       }
-      ask(w);
+      ask(c, true);
       k += k_step;
       if (++chunk < chunks) return;
       // the group's end
-      float v = sum32_by_lane(acc, lane);      // lane 8 j + m: weight row j, row m0 + m of A
+      float v = sums_by_lane<4 * ROWS>(acc, lane);
       if (KW > 1) {
         __syncthreads();      // the sums of the group before have been read
         part[warp][lane] = v;
@@ -243,21 +313,24 @@ gemm_few_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
         if (kw == 0)
           for (int i = 1; i < KW; ++i) v += part[warp + i][lane];
       }
-      const int j = lane >> 3, m = m0 + (lane & 7);
+      constexpr int EACH = 8 / ROWS;      // lanes that have the sum of weight row j and row m of A
+      const int j = lane >> 3, m = m_walk + m0 + (lane & 7) / EACH;
       const float up = GLU ? __shfl_sync(0xffffffffu, v, (lane + (EPI == EPI_SWIGLU ? 16 : 8)) & 31) : 0.f;
       const int f = EPI == EPI_SWIGLU_PAIRS ? j >> 1 : j, n0 = g * FEATS;
-      const bool has = EPI == EPI_SWIGLU_PAIRS ? !(j & 1) : (EPI != EPI_SWIGLU || j < 2);
+      const bool has = (EPI == EPI_SWIGLU_PAIRS ? !(j & 1) : (EPI != EPI_SWIGLU || j < 2)) && lane % EACH == 0;
       if (kw == 0 && m < M && has && n0 + f < N)
         put_out(C, c_bf16, (size_t)m * ldc + n0 + f, GLU ? v / (1.0f + expf(-v)) * up : v, EPI == EPI_ADD);
       chunk = 0;
       k = k_first;
+      if (TWO_PASSES && (m0 += ROWS) < walk_rows) return;
+      m0 = 0;
       g += step;
       more = g - warp / KW < groups;
     };
     while (more) {
-      work(w0);
-      if (more) work(w1);
-      if (DEPTH > 2 && more) work(w2);
+      work(c0);
+      if (more) work(c1);
+      if (DEPTH > 2 && more) work(c2);
     }
   }
 }
@@ -440,31 +513,35 @@ static int launch(const void* A, int lda, const void* W, void* C, int c_bf16, in
     const int room = 2 * sms;
     int kw = 1;
     long long least = 1ll << 60;
-    for (int n = 1; n <= 8 && (n == 1 || (n - 1) * 128 < K); n *= 2) {
+    for (int n = 1; n <= 8 && (n == 1 || n / 2 * 128 < K); n *= 2) {
       const long long work = (long long)((groups + (8 / n) * room - 1) / ((8 / n) * room)) *
                              ((K + 128 * n - 1) / (128 * n) + 1);
       if (work < least) { least = work; kw = n; }
     }
     const int all = (groups + 8 / kw - 1) / (8 / kw), blocks = all < room ? all : room;
-    const int rows = M < FEW_ROWS ? M : FEW_ROWS;
-    const size_t bytes = (size_t)rows * K * sizeof(float);
+    // the rows of A that a walk through the weight has in shared memory: all of them where they fit
+    const int walk_rows = M <= FEW_ROWS || (size_t)M * K * sizeof(float) <= FEW_STAGED ? M : FEW_ROWS;
+    const size_t bytes = (size_t)walk_rows * K * sizeof(float);
     // The rows of A into shared memory where a warp has at least eight chunks: the copy costs a wait
     // of its own. Eight rows, us with | without: 151,936 x 1,024 119 | 134 and 2 x 3,072 x 1,024 (8
     // chunks a warp) 18.5 | 20.5, but 4,096 x 1,024 (4) 16.4 | 14.5 and 1,024 x 3,072 (3) 16.4 | 13.3.
     const long long rounds = (groups + (8 / kw) * (long long)blocks - 1) / ((8 / kw) * (long long)blocks);
     const bool staged = bytes <= FEW_STAGED && rounds * ((K + 128 * kw - 1) / (128 * kw)) >= 8;
-#define FEW2(E, S_)                                                                           \
+#define FEW2(E, R_, S_, T_)                                                                   \
   {                                                                                           \
     static unsigned long long allowed = 0;                                                    \
+    const auto kernel = gemm_few_rows_kernel<TA, TW, E, R_, S_, T_>;                          \
     const cudaError_t e =                                                                     \
-        S_ ? mb_allow_smem((const void*)gemm_few_rows_kernel<TA, TW, E, S_>, FEW_STAGED, &allowed) \
-           : cudaSuccess;                                                                     \
+        S_ ? mb_allow_smem((const void*)kernel, FEW_STAGED, &allowed) : cudaSuccess;          \
     if (e != cudaSuccess) MB_FAIL("mb_gemm_simt: %s", cudaGetErrorString(e));                 \
-    mb_launch(gemm_few_rows_kernel<TA, TW, E, S_>, dim3(blocks), dim3(256), S_ ? bytes : 0, s, \
-              (const TA*)A, lda, (const TW*)W, C, c_bf16, ldc, M, N, K, kw, groups, settled); \
+    mb_launch(kernel, dim3(blocks), dim3(256), S_ ? bytes : 0, s, (const TA*)A, lda,          \
+              (const TW*)W, C, c_bf16, ldc, M, N, K, kw, groups, settled);                    \
   }
 #define FEW(E)                                                                                \
-  if (staged) FEW2(E, true) else FEW2(E, false)
+  if (M <= 2) FEW2(E, 2, false, false)                                                        \
+  else if (!staged) FEW2(E, FEW_ROWS, false, false)                                           \
+  else if (walk_rows > FEW_ROWS) FEW2(E, FEW_ROWS, true, true)                                \
+  else FEW2(E, FEW_ROWS, true, false)
     switch (epi) {
       case EPI_STORE: FEW(EPI_STORE) break;
       case EPI_ADD: FEW(EPI_ADD) break;

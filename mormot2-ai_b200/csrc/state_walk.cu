@@ -282,7 +282,7 @@ state_walk_kernel(const WalkArgs g, int P, int CW, int CT) {
           }
         }
       }
-      const float sum = sum32_by_lane(sums, lane);
+      const float sum = sums_by_lane<32>(sums, lane);
       const int t = (lane >> 2) & 3, s = lane & 3;
       const float qk = __shfl_sync(0xffffffffu, sum, t * (t + 1) / 2 + min(s, t));
       if (CHANNEL) {

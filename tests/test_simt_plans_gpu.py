@@ -55,3 +55,25 @@ def test_a_weight_of_the_kernel_before(M):
         K.gemm_simt(left, right, w)
         K.gemm_simt(a, w, out)
         assert torch.equal(out.double(), exact)
+
+
+# few rows of A: one or two, whose values are asked for with the weight's; up to eight and more than eight in
+# shared memory (a large weight), the last of them in two passes a group; whole numbers, every pair of types
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 13, 16])
+@pytest.mark.parametrize("N, Kd", [(20001, 516), (6000, 1024), (7, 4096), (20, 64)])
+@pytest.mark.parametrize("types", ["ff", "fb", "bb", "bf"])
+def test_few_rows(M, N, Kd, types):
+    kind = {"f": torch.float32, "b": torch.bfloat16}
+    a, w, c = whole((M, Kd), 1).to(kind[types[0]]), whole((2 * N, Kd), 2).to(kind[types[1]]), whole((M, N), 3, 50)
+    exact = a.float() @ w.float().t()
+    out = torch.empty((M, 2 * N), device=DEV)
+    K.gemm_simt(a, w, out, settled=True)
+    assert torch.equal(out, exact)
+    K.gemm_simt(a, w[:N], c_add := c.clone(), K.EPI_ADD)
+    assert torch.equal(c_add, c + exact[:, :N])
+    a, w = a * 0.0625, w * 0.25      # exact in bfloat16 too
+    z = exact.double() / 64
+    for epilogue, g, u in ((K.EPI_SWIGLU_PAIRS, z[:, 0::2], z[:, 1::2]), (K.EPI_SWIGLU, z[:, :N], z[:, N:])):
+        K.gemm_simt(a, w, out := torch.empty((M, N), device=DEV), epilogue)
+        want = torch.nn.functional.silu(g) * u
+        assert (out.double() - want).norm() <= 2e-6 * want.norm()      # exact sums, expf and a division
