@@ -266,10 +266,13 @@ __device__ __forceinline__ float pair_half(f32_pair v, int h) {
 
 // A float32 value as the exact sum of three bfloat16 parts of 8 significant bits each: its upper half,
 // the upper half of what is left, and the rest. Of two neighbouring values, as they stand in memory.
-// An infinity's first part is that infinity, its others are NaN.
+// Exact from 2^-110 up: a smaller value may have bits below bfloat16's last place, 2^-133. `rest` tells:
+// its lower 16 bits are zero where both sums are exact, and not zero for an infinity (whose first part is
+// that infinity, the others NaN) or a NaN.
 struct Cut2 {
-  uint32_t hi, mid, lo;
+  uint32_t hi, mid, lo, rest;
 };
+__device__ __forceinline__ bool cut_is_inexact(uint32_t rest) { return (rest & 0xffffu) != 0; }
 __device__ __forceinline__ f32_pair pair_sub_upper(f32_pair v) {      // v less its upper halves
   f32_pair r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -283,7 +286,7 @@ __device__ __forceinline__ Cut2 cut(float a, float b) {
   f32_pair v;      // a NaN whose upper half alone would read as an infinity becomes the common one
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(pair_of(a, b)), "l"(0x8000000080000000ull));
   const f32_pair r = pair_sub_upper(v), q = pair_sub_upper(r);
-  return {upper_halves(v), upper_halves(r), upper_halves(q)};
+  return {upper_halves(v), upper_halves(r), upper_halves(q), (uint32_t)q | (uint32_t)(q >> 32)};
 }
 
 __device__ __forceinline__ void pair_fma(f32_pair& s, f32_pair a, f32_pair b) {   // s += a b

@@ -1,6 +1,6 @@
 // y = x · Wᵀ of float32 operands on the tensor cores, for more rows than gemm_simt.cu's kernel of
-// few rows takes. Every float32 value is the exact sum of three bfloat16 parts of 8 significant
-// bits each (hi + mid + lo: its 24 bits cut in three), so a product of two values is a sum of nine
+// few rows takes. Every float32 value from 2^-110 up is the exact sum of three bfloat16 parts of 8
+// significant bits each (hi + mid + lo: its 24 bits cut in three), so a product of two values is a sum of nine
 // products of parts; six of them are computed, the other three lie 2^-24 and less below the whole.
 // tcgen05 multiplies exactly and adds in float32, but cuts off what falls behind the accumulator's
 // last place instead of rounding. So no long sum is left to it: hi·hi is drained from tensor memory
@@ -22,8 +22,11 @@
 // 1,728 rows, 4,096 x 1,024 376 -> 93 us (156 TFLOP/s of float32 products), 1,024 x 3,072 316 -> 87,
 // 6,144 x 1,024 with SwiGLU 525 -> 142; 24 rows, 1,024 x 2,048 41 -> 19; 400 rows 72 -> 28.
 //
-// Infinities: hi of an infinity is that infinity and its other parts are NaN; hi·hi is then
-// infinite or NaN as the whole product would be, and stands alone for the result.
+// Values that the parts do not sum up to (below 2^-110, where bits fall behind bfloat16's last place;
+// infinities and NaNs) get a NaN for their lo, so that what they take part in comes out as a NaN of the
+// smaller products' accumulator. Results that are no numbers, those and overflows, are made again by a
+// chain of multiply-adds in the drain (`again`): a value's loss, and what it costs, stays with the rows
+// that have it.
 #include <cooperative_groups.h>
 
 #include "attention_tc.cuh"
@@ -43,6 +46,7 @@ constexpr int GS_A_MAX = 4, GS_B_MAX = 6;    // stages, at most
 constexpr int GS_A_COLS = 3 * GS_K / 2;      // tensor memory of a stage: hi, mid, lo
 constexpr int GS_THREADS = 32 * 20;  // 8 warps cut the weight, 8 drain, 1 loads, 2 issue, 1 has no part
 constexpr int GS_SMEM = 200 * 1024;  // of the stages of x
+constexpr uint32_t GS_NAN2 = 0x7fff7fffu;    // two bfloat16 NaNs
 
 // 16 lanes x 16 columns of tensor memory: registers 4 j .. 4 j + 3 hold columns 8 j + 2 (lane % 4)
 // and the next of row lane / 4, then of row lane / 4 + 8
@@ -97,7 +101,9 @@ cut_rows_kernel(const float* __restrict__ A, int lda, int M, int K, int Kp,
     const int m = (int)(i / per_row), k = 8 * (int)(i - (long long)m * per_row);
     const float* at = A + (size_t)m * lda + k;
     const float4 u = piece4<VEC>(at, K - k), v = piece4<VEC>(at + 4, K - k - 4);
-    const Cut2 c[4] = {cut(u.x, u.y), cut(u.z, u.w), cut(v.x, v.y), cut(v.z, v.w)};
+    Cut2 c[4] = {cut(u.x, u.y), cut(u.z, u.w), cut(v.x, v.y), cut(v.z, v.w)};
+    if (cut_is_inexact(c[0].rest | c[1].rest | c[2].rest | c[3].rest))
+      c[0].lo = c[1].lo = c[2].lo = c[3].lo = GS_NAN2;
     uint4* out = (uint4*)(planes + (size_t)m * Kp + k);
     const size_t plane = (size_t)M * Kp / 8;
     out[0] = make_uint4(c[0].hi, c[1].hi, c[2].hi, c[3].hi);
@@ -108,9 +114,9 @@ cut_rows_kernel(const float* __restrict__ A, int lda, int M, int K, int Kp,
 
 // ---------------------------------------------------------------------------- the product
 struct SplitArgs {
-  const float* W;
+  const float *A, *W;
   void* C;
-  int ldc, c_bf16, M, NW, K, epi;
+  int lda, ldc, c_bf16, M, NW, K, epi;
   int cols, a_stages, b_stages, splits, k_split, tiles_m, num_tiles;
   int* error;
 };
@@ -220,7 +226,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const SplitArgs p) {
       if (kb >= nkb) enter();
       more = tile < p.num_tiles;
       const uint32_t ph = ((it / p.a_stages) & 1) ^ 1;
-      uint32_t hi[16], mid[16], lo[16];
+      uint32_t hi[16], mid[16], lo[16], rest = 0;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -228,9 +234,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const SplitArgs p) {
           const Cut2 a = cut(r[i].x, r[i].y), b = cut(r[i].z, r[i].w);
           hi[2 * i] = a.hi; mid[2 * i] = a.mid; lo[2 * i] = a.lo;
           hi[2 * i + 1] = b.hi; mid[2 * i + 1] = b.mid; lo[2 * i + 1] = b.lo;
+          rest |= a.rest | b.rest;
         }
         if (more) fetch(h);
       }
+      if (cut_is_inexact(rest)) {      // somewhere in this thread's four rows
+#pragma unroll
+        for (int i = 0; i < 16; ++i) lo[i] = GS_NAN2;
+      }
+      __syncwarp();
       mbar_wait(a_empty0 + 8 * st, ph, p.error, 41);
       tc_fence_after_sync();
 #pragma unroll
@@ -351,6 +363,36 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const SplitArgs p) {
     const int row = 32 * q + lane;
     int g = 0;
     uint32_t low_ph = 0;
+    // results that are no numbers, by multiply-adds over this CTA's share of K
+    auto again = [&](float (&s)[4][16], int tile) {
+      float t[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) t[i] = s[i / 16][i % 16];
+      const int n = (tile / p.tiles_m) * GS_ROWS + row, m0 = (tile % p.tiles_m) * p.cols + c0;
+      const int valid = n < p.NW ? min(16 * parts, p.M - m0) : 0;
+#pragma unroll 1
+      for (int c = 0; c < valid; ++c) {
+        if (fabsf(t[c]) <= 3.402823466e38f) continue;
+        const float *x = p.A + (size_t)(m0 + c) * p.lda, *w = p.W + (size_t)n * p.K;
+        float v = 0.f;
+#pragma unroll 1
+        for (int k = k_lo; k < k_hi; k += 64) {      // (one chain over all of K would round more often)
+          const int end = min(k + 64, k_hi);
+          float u[4] = {0.f, 0.f, 0.f, 0.f};
+          int i = k;
+#pragma unroll 1
+          for (; i + 4 <= end; i += 4)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) u[e] = fmaf(x[i + e], w[i + e], u[e]);
+          for (; i < end; ++i) u[0] = fmaf(x[i], w[i], u[0]);
+          v += (u[0] + u[1]) + (u[2] + u[3]);
+        }
+        t[c] = v;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 64; ++i) s[i / 16][i % 16] = t[i];
+    };
     for (int tile = tile0; tile < p.num_tiles; tile += tile_step) {
       float s[4][16];
 #pragma unroll
@@ -376,19 +418,23 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const SplitArgs p) {
       mbar_wait(low_full, low_ph, p.error, 46);
       low_ph ^= 1;
       tc_fence_after_sync();
+      float no_number = 0.f;      // turns NaN
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (i < parts) {
           float v[16];
           tmem_ld16(t_low + lanes + 16 * i, v);
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (fabsf(s[i][j]) <= 3.402823466e38f) s[i][j] += v[j];
+          for (int j = 0; j < 16; ++j) {
+            s[i][j] += v[j];
+            no_number = fmaf(s[i][j], 0.f, no_number);
+          }
         }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(low_empty);
+      if (__any_sync(0xffffffffu, no_number != 0.f)) again(s, tile);
       if (p.splits > 1) {      // [rows of x][weight rows], over the stages that nobody reads any more
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -532,8 +578,8 @@ MB_EXPORT int mb_gemm_split(const void* A, int lda, const void* W, void* C, int 
   cudaStream_t s = (cudaStream_t)stream;
   const int Kp = (int)padded_k(K);
   SplitArgs p;
-  p.W = (const float*)W; p.C = C;
-  p.ldc = ldc; p.c_bf16 = c_dtype == MB_BF16; p.M = M; p.K = K; p.epi = epilogue;
+  p.A = (const float*)A; p.W = (const float*)W; p.C = C;
+  p.lda = lda; p.ldc = ldc; p.c_bf16 = c_dtype == MB_BF16; p.M = M; p.K = K; p.epi = epilogue;
   p.NW = epilogue == EPI_SWIGLU_PAIRS ? 2 * N : N;
   p.error = (int*)error;
   const int tiles_n = (p.NW + GS_ROWS - 1) / GS_ROWS;

@@ -88,3 +88,33 @@ def test_error_against_float64(Kd):
     K.gemm_simt(a, w, out)
     want = a.double() @ w.double().t()
     assert (out.double() - want).norm() <= 4e-7 * want.norm()
+
+
+# Values below 2^-110 have bits that no bfloat16 part holds: what they take part in is multiplied and added
+# in float32, and errs by no more than such a chain: 4e-7 of the result as above, and of results below
+# float32's normal range half a last place, 2^-150, a step
+@pytest.mark.parametrize("M, N, Kd", [(40, 130, 160), (150, 70, 1095)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_small_values(M, N, Kd, splits):
+    splits = splits if Kd >= 128 * splits else 0
+    a, w, c = drawn((M, Kd), 11), drawn((N, Kd), 12), drawn((M, N), 13)
+    small = {3: -104, 17: -111, 18: -120, 30: -126, 31: -140}
+    for row, e in small.items():
+        a[row] *= 2.0 ** e
+    w[9] *= 2.0 ** -118
+    a[6, 20] = 2.0 ** -119 * 1.0000001      # one beside others
+    error, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.empty((M, N), device=DEV)
+    K.gemm_split(a, w, out, K.EPI_STORE, error, 0, splits)
+    want = a.double() @ w.double().t()
+    err = (out.double() - want).abs()
+    near = lambda x, y: x.norm() <= 4e-7 * y.norm() + Kd * 2.0 ** -150 * y.numel() ** 0.5
+    for row in (*small, 0, 6, M - 1):
+        assert near(err[row], want[row]), (row, err[row].norm() / want[row].norm())
+    assert near(err[:, 9], want[:, 9])
+    a[0, 5], w[11, 5] = float("inf"), 2.0 ** -140      # infinity, not 0 * infinity, whose first part is zero
+    K.gemm_split(a, w, c_add := c.clone(), K.EPI_ADD, error, 0, splits)
+    want = c.double() + a.double() @ w.double().t()
+    assert torch.equal(c_add.isposinf(), want.isposinf()) and torch.equal(c_add.isneginf(), want.isneginf())
+    assert not c_add.isnan().any()
+    fine = want.isfinite()
+    assert (c_add.double() - want)[fine].norm() <= 4e-7 * want[fine].norm() and int(error) == 0
