@@ -1,5 +1,5 @@
 // Causal attention of many new tokens in float32 on the tensor cores, for heads of 128 values: every
-// float32 value is cut into three exact bfloat16 parts (common.cuh), and both products are sums of six
+// float32 value is cut into three bfloat16 parts that sum up to it (common.cuh), and both products are sums of six
 // products of parts, as in gemm_split.cu. 128 new tokens of one sequence and one head per CTA, a
 // page of 64 keys at a time.
 //
@@ -12,8 +12,10 @@
 // an accumulator (two, and one for all the rest), the output's a page; sums over those are float32
 // additions. The softmax is the float32 kernel's, with all its options.
 //
-// A CTA whose inputs or results are no numbers somewhere (an infinity, a NaN, a row that sees no key)
-// says so in `redo`, and attention_many_kernel, launched behind, does that tile again.
+// A CTA whose inputs may be no exact sums of three parts (values below 2^-110, infinities, NaNs) or whose
+// results are no numbers somewhere (an overflow, a row that sees no key) says so in `redo`, and
+// attention_many_kernel, launched behind, does that tile again. A probability below 2^-110 may lose up
+// to 2^-133, beside a sum of at least one.
 //
 // What bounds it: a page's chain, products of scores, softmax (64 exponentials and cuts a thread), products
 // of values, one after the other, since tensor memory has no room for a second tile. 1,728 tokens of
@@ -118,7 +120,7 @@ attention_split_kernel(const AttArgs<float> a, int fewest, int* __restrict__ red
           v[i] = as_load4(at + (size_t)(8 * (i & 1)) * a.q_stride + 32 * kb + 16 * (i >> 1), row + 8 * (i & 1) < cnt);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          odd |= as_no_number(v[i]);
+          odd |= as_no_number(v[i]) | too_small_to_cut(v[i]);
           const Cut2 x = cut(v[i].x, v[i].y), y = cut(v[i].z, v[i].w);
           hi[2 * i] = x.hi; mid[2 * i] = x.mid; lo[2 * i] = x.lo;
           hi[2 * i + 1] = y.hi; mid[2 * i + 1] = y.mid; lo[2 * i + 1] = y.lo;
@@ -147,7 +149,7 @@ attention_split_kernel(const AttArgs<float> a, int fewest, int* __restrict__ red
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = warp + 8 * i;
-        odd |= as_no_number(r[i]);
+        odd |= as_no_number(r[i]) | too_small_to_cut(r[i]);
         const Cut2 x = cut(r[i].x, r[i].y), y = cut(r[i].z, r[i].w);
         const uint32_t p = at + row * 128 + ((ch ^ (row & 7)) << 4);
         as_st_v2(p, x.hi, y.hi);

@@ -289,6 +289,13 @@ __device__ __forceinline__ Cut2 cut(float a, float b) {
   return {upper_halves(v), upper_halves(r), upper_halves(q), (uint32_t)q | (uint32_t)(q >> 32)};
 }
 
+// Whether one of four values is not zero and below 2^-110, where its three parts may be no exact sum
+__device__ __forceinline__ bool too_small_to_cut(float4 v) {
+  const uint32_t least = min(min((__float_as_uint(v.x) << 1) - 1, (__float_as_uint(v.y) << 1) - 1),
+                             min((__float_as_uint(v.z) << 1) - 1, (__float_as_uint(v.w) << 1) - 1));
+  return least < (17u << 24) - 1;
+}
+
 __device__ __forceinline__ void pair_fma(f32_pair& s, f32_pair a, f32_pair b) {   // s += a b
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
 }

@@ -78,3 +78,22 @@ def test_error(n, past, monkeypatch):
     errors = [((run(k, v, q, past, split, monkeypatch, 4, 2).double().cpu() - want).norm() / want.norm()).item()
               for split in (False, True)]
     assert errors[1] <= 1.2 * errors[0] and errors[1] <= 1e-6, errors
+
+
+# queries, keys or values below 2^-110 may be no exact sums of three parts: their tiles go through the
+# float32 kernel, the same bits
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+def test_small_values(where, monkeypatch):
+    n, past = 300, 20
+    k, v, q = draw(n, past, 5)
+    if where == "q":
+        q[130] *= 2.0 ** -118
+        q[130, 128:] = 0.0      # the second head: zeros are cut exactly
+    else:
+        (k if where == "k" else v)[:, 0, 3] *= 2.0 ** -118
+    want, got = (run(k, v, q, past, split, monkeypatch) for split in (False, True))
+    if where == "q":
+        assert torch.equal(got[128:256, :128], want[128:256, :128])
+        assert not torch.equal(got[128:256, 128:], want[128:256, 128:])
+    else:
+        assert torch.equal(got, want)
