@@ -29,8 +29,10 @@
 // by fours 366 us -> 56 + 150; four prompts of 111 to 900, 8 heads, mlstm: 185 -> 23 + 86 (before what
 // keeps the sums from leaning was added: 9 and 7 us more; the whole mixers 491 -> 323, 261 -> 180). With the
 // operands in shared memory and cut there a chunk took twice the instructions (97 + 234 us).
-// What is no number (an infinity, a NaN, an overflow) goes through a form that takes the chunk token
-// by token, so that it reaches no earlier token.
+// Keys, queries, a state or an update that may be no exact sums of three parts (an infinity, a NaN, a value
+// below 2^-110) take the chunk through a form that goes token by token, so that they reach no earlier
+// token and keep their 24 bits. Factors with decays in them may lose up to 2^-133, bfloat16's last place,
+// beside the token's own, which is not decayed.
 #pragma once
 #include "mma_common.cuh"
 
@@ -59,12 +61,15 @@ __device__ __forceinline__ Cut2 cut_near(float a, float b) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(c.hi) : "f"(b), "f"(a));
   const f32_pair v = pair_of(a - __uint_as_float(c.hi << 16), b - __uint_as_float(c.hi & 0xffff0000u));
   c.mid = upper_halves(v);
-  c.lo = upper_halves(pair_sub_upper(v));
+  const f32_pair q = pair_sub_upper(v);
+  c.lo = upper_halves(q);
+  c.rest = (uint32_t)q | (uint32_t)(q >> 32);
   return c;
 }
-__device__ __forceinline__ void put_a(FragA& f, int i, float a, float b) {
+__device__ __forceinline__ uint32_t put_a(FragA& f, int i, float a, float b) {      // gives the cut's rest
   const Cut2 c = cut_near(a, b);
   f.hi[i] = c.hi; f.mid[i] = c.mid; f.lo[i] = c.lo;
+  return c.rest;
 }
 __device__ __forceinline__ void put_b(FragB& f, int i, float a, float b) {
   const Cut2 c = cut(a, b);
@@ -136,7 +141,7 @@ __device__ __forceinline__ void sc_copy16(float* dst, const float* src, bool val
 // Block (sequence and chunk of this pass, head). `chunk0`: the pass's first chunk of every sequence,
 // `per_seq` chunks of each; `m_in`, `m_out`: mlstm's running maxima at the pass's ends, [B][H] each.
 template <bool DELTA>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, DELTA ? 2 : 3)
 state_chunk_prep_kernel(const WalkArgs g, float* __restrict__ scratch, int chunk0, int per_seq,
                         const float* __restrict__ m_in, float* __restrict__ m_out) {
   mb_grid_wait();
@@ -199,8 +204,11 @@ state_chunk_prep_kernel(const WalkArgs g, float* __restrict__ scratch, int chunk
         odd |= !(0.f * fq + 0.f * fk == 0.f);
       }
       if (i < D) {
-        *(float4*)(qs + t * DP + i) = make_float4(q[r].x * fq, q[r].y * fq, q[r].z * fq, q[r].w * fq);
-        *(float4*)(ks + t * DP + i) = make_float4(k[r].x * fk, k[r].y * fk, k[r].z * fk, k[r].w * fk);
+        const float4 x = make_float4(q[r].x * fq, q[r].y * fq, q[r].z * fq, q[r].w * fq);
+        const float4 y = make_float4(k[r].x * fk, k[r].y * fk, k[r].z * fk, k[r].w * fk);
+        odd |= too_small_to_cut(x) | too_small_to_cut(y);
+        *(float4*)(qs + t * DP + i) = x;
+        *(float4*)(ks + t * DP + i) = y;
       }
       if (lane == 0) {
         out[SC_FQ + t] = fq;
@@ -555,10 +563,8 @@ state_chunk_walk_kernel(const WalkArgs g, const float* __restrict__ scratch, int
     if (own) {
       // S0^T [16 x 16 of this warp's rows] times the rows of W and q
       FragA a;
-      put_a(a, 0, S[0][0], S[0][1]);
-      put_a(a, 1, S[0][2], S[0][3]);
-      put_a(a, 2, S[1][0], S[1][1]);
-      put_a(a, 3, S[1][2], S[1][3]);
+      odd |= cut_is_inexact(put_a(a, 0, S[0][0], S[0][1]) | put_a(a, 1, S[0][2], S[0][3]) |
+                            put_a(a, 2, S[1][0], S[1][1]) | put_a(a, 3, S[1][2], S[1][3]));
       float acc[NT][4] = {};
       mma_low<NT>(acc, a, fr);
       mma_high<NT>(acc, a, fr);
@@ -590,8 +596,8 @@ state_chunk_walk_kernel(const WalkArgs g, const float* __restrict__ scratch, int
         float4 u = u1;
         if (!DELTA && (norm_col || t >= cn)) u = make_float4(my_col == 0 && t < cn ? 1.f : 0.f, 0.f, 0.f, 0.f);
         if (DELTA) u = make_float4(u.x - v.x, u.y - v.y, u.z - v.z, u.w - v.w);
-        odd |= no_number(u);
         const Cut2 a = cut_near(u.x, u.y), z = cut_near(u.z, u.w);
+        odd |= cut_is_inexact(a.rest | z.rest);
         unsigned short* h = (unsigned short*)up + my_col * 40 + t;
         const uint32_t words[6] = {a.hi, z.hi, a.mid, z.mid, a.lo, z.lo};
 #pragma unroll

@@ -126,3 +126,27 @@ def test_rule(lens, by):
     got = tuple(K.walks_in_chunks(step, dim, 128, mode, heads) for mode, heads, dim in
                 ((K.WALK_DELTA, 16, 128), (K.WALK_DELTA, 8, 64), (K.WALK_MLSTM, 8, 128)))
     assert got == by
+
+
+# States and values below 2^-110, which three bfloat16 parts do not hold: the state's error is that of the
+# normal range (float32 roundings of the tokens' updates, whose size does not depend on the exponent)
+@pytest.mark.parametrize("mode", ["delta", "mlstm"])
+@pytest.mark.parametrize("exponent", [-100, -112, -118])
+def test_small_states(monkeypatch, mode, exponent):
+    lens, heads, dim, vdim = [96, 40], 2, 64, 32
+    T, real, per = sum(lens), walk.rows, dim * vdim + (dim + 1 if mode == "mlstm" else 0)
+
+    def small(shape, seed, *a, **k):
+        t = real(shape, seed, *a, **k)
+        if seed == 1:
+            t[:, 2 * heads * dim:2 * heads * dim + heads * vdim] *= 2.0 ** exponent
+        return t
+    monkeypatch.setattr(walk, "rows", small)
+    start = real((len(lens), size_of(mode, heads, dim, vdim)), 9, 0.3)
+    start.view(len(lens), heads, per)[:, :, :dim * vdim] *= 2.0 ** exponent
+    _, states = walk.plain(mode, start, lens, heads, dim, vdim, 1, T)
+    route(monkeypatch, True)
+    state, step = start.clone(), make_step([(i, 5, [0] * n, []) for i, n in enumerate(lens)])
+    walk.run(mode, step, state, T, heads, dim, vdim, 1, 0, torch.float32)
+    got, want = (s.double().cpu().view(len(lens), heads, per)[:, :, :dim * vdim] for s in (state, states))
+    assert (got - want).norm() <= 1e-6 * want.norm()
