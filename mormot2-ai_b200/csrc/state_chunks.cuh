@@ -30,9 +30,10 @@
 // keeps the sums from leaning was added: 9 and 7 us more; the whole mixers 491 -> 323, 261 -> 180). With the
 // operands in shared memory and cut there a chunk took twice the instructions (97 + 234 us).
 // Keys, queries, a state or an update that may be no exact sums of three parts (an infinity, a NaN, a value
-// below 2^-110) take the chunk through a form that goes token by token, so that they reach no earlier
-// token and keep their 24 bits. Factors with decays in them may lose up to 2^-133, bfloat16's last place,
-// beside the token's own, which is not decayed.
+// below 2^-110) and products of keys and queries that overflow take the chunk through a form that goes
+// token by token, so that they reach no earlier token and keep their 24 bits. A state or an output that
+// overflows at the end of a chunk is an infinity there. Factors with decays in them may lose up to 2^-133,
+// bfloat16's last place, beside the token's own, which is not decayed.
 #pragma once
 #include "mma_common.cuh"
 
@@ -298,8 +299,7 @@ state_chunk_prep_kernel(const WalkArgs g, float* __restrict__ scratch, int chunk
       Dm[t * 33 + lane] = t >= lane ? p : 0.f;
     }
   }
-  if (__syncthreads_or(odd) && threadIdx.x == 0) out[1] = 1.f;
-  else if (threadIdx.x == 0) out[1] = 0.f;
+  __syncthreads();
 
   // q . k and k . k: warps of (which, 16 rows t, 16 columns s)
   const int gr = lane >> 2, tq = lane & 3;
@@ -343,6 +343,7 @@ state_chunk_prep_kernel(const WalkArgs g, float* __restrict__ scratch, int chunk
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const float x = sum[j][2 * r + e] + low[j][2 * r + e];
+            odd |= !(fabsf(x) <= 3.402823466e38f);      // an overflow
             if (!kk) v[e] = s + e <= t ? x * Dm[t * 33 + s + e] : 0.f;
             else v[e] = s + e < t ? beta[t] * Dm[t * 33 + s + e] * x : 0.f;
           }
@@ -355,8 +356,9 @@ state_chunk_prep_kernel(const WalkArgs g, float* __restrict__ scratch, int chunk
       }
     }
   }
+  const int any_odd = __syncthreads_or(odd);
+  if (threadIdx.x == 0) out[1] = any_odd ? 1.f : 0.f;
   if (DELTA) {
-    __syncthreads();
     // T = (I + M)^-1: its two blocks of 16 on the diagonal by forward substitution, a column a lane,
     // then the one below them
     if (warp == 0) {
@@ -695,7 +697,11 @@ state_chunk_walk_kernel(const WalkArgs g, const float* __restrict__ scratch, int
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[i][e] = h0[i][e] + (h1[i][e] + acc[i][e]);
+        for (int e = 0; e < 4; ++e) {
+          // an overflow of the leading products stands for itself: what they cut off is no number then
+          const float sum = h0[i][e] + (h1[i][e] + acc[i][e]);
+          acc[i][e] = sum == sum ? sum : h0[i][e] + h1[i][e];
+        }
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j)

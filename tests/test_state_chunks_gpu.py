@@ -150,3 +150,26 @@ def test_small_states(monkeypatch, mode, exponent):
     walk.run(mode, step, state, T, heads, dim, vdim, 1, 0, torch.float32)
     got, want = (s.double().cpu().view(len(lens), heads, per)[:, :, :dim * vdim] for s in (state, states))
     assert (got - want).norm() <= 1e-6 * want.norm()
+
+
+# a state that overflows in a sequence's last token is an infinity, as by fours
+def test_an_update_that_overflows(monkeypatch):
+    T, heads, dim, real, states = 64, 2, 64, walk.rows, []
+
+    def large(shape, seed, *a, **k):
+        t = real(shape, seed, *a, **k)
+        if seed == 1:
+            t[T - 1, heads * dim:2 * heads * dim] *= 40.0
+            t[T - 1, 2 * heads * dim:3 * heads * dim] *= 5e37
+        return t
+    monkeypatch.setattr(walk, "rows", large)
+    step = make_step([(0, 0, [0] * T, [])])
+    for chunks in (False, True):
+        route(monkeypatch, chunks)
+        state = torch.zeros((1, size_of("mlstm", heads, dim, dim)), device=DEV)
+        walk.run("mlstm", step, state, T, heads, dim, dim, 1, 0, torch.float32)
+        states.append(state)
+    want, got = states
+    assert want.isposinf().any() and want.isneginf().any() and not want.isnan().any()
+    assert torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+    assert not got.isnan().any()
