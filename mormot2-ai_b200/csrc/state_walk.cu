@@ -676,7 +676,7 @@ MB_EXPORT long long mb_state_chunks_scratch(int mode, int B, int H, int D, int D
 }
 
 MB_EXPORT int mb_state_chunks(const WalkArgs* args, float* scratch, long long scratch_floats, int longest,
-                              void* stream) {
+                              int sms, void* stream) {
   const WalkArgs g = *args;
   if (g.T <= 0 || g.B <= 0) return 0;
   const bool delta = g.mode == WALK_DELTA;
@@ -696,7 +696,13 @@ MB_EXPORT int mb_state_chunks(const WalkArgs* args, float* scratch, long long sc
   const size_t prep_smem = (2 * SC_C * (g.D + 8) + SC_C * 33 + 2 * SC_C * 36 + 16 * 17 + 3 * SC_C +
                             (delta ? (g.DV <= SC_V_HERE ? SC_C * (size_t)(g.DV + 8) : 0) : 2 * (size_t)per_seq)) * 4;
   const int warps = g.D / 16, rows = delta ? 2 * SC_C : SC_C, threads = 32 * (warps < 4 ? 4 : warps);
-  const size_t walk_smem = ((size_t)warps * rows * SC_PART + SC_C * SC_PART + 3 * SC_COLS * 20) * 4;
+  const dim3 walk(g.B, g.H, g.DV / SC_COLS + (delta ? 0 : 1));
+  size_t walk_smem = ((size_t)warps * rows * SC_PART + SC_C * SC_PART + 3 * SC_COLS * 20) * 4;
+  // Where every walking CTA can have a multiprocessor for itself it asks for more than half of the shared
+  // memory: the CTAs come while preparing blocks still run, and two of them on one multiprocessor made
+  // the walk a fifth longer (mlstm, 1,000 tokens, us of the whole call without | with: 8 heads of 128 x
+  // 128 124 | 104, 16 of 64 x 128 120 | 105; delta, 8 heads of 64 x 128 98 | 89).
+  if ((long long)walk.x * walk.y * walk.z <= sms && walk_smem < 116 * 1024) walk_smem = 116 * 1024;
   if (prep_smem > 200 * 1024) MB_FAIL("mb_state_chunks: %d chunks in one pass", per_seq);
   static unsigned long long allowed[4] = {0, 0, 0, 0};
   const void* kernels[4] = {(const void*)state_chunk_prep_kernel<false>, (const void*)state_chunk_prep_kernel<true>,
@@ -709,7 +715,7 @@ MB_EXPORT int mb_state_chunks(const WalkArgs* args, float* scratch, long long sc
   int pass = 0;
   for (int c = 0; c < all; c += per_seq, ++pass) {
     const int now = all - c < per_seq ? all - c : per_seq;
-    const dim3 grid((unsigned)(g.B * now), g.H), walk(g.B, g.H, g.DV / SC_COLS + (delta ? 0 : 1));
+    const dim3 grid((unsigned)(g.B * now), g.H);
     if (delta) {
       mb_launch(state_chunk_prep_kernel<true>, grid, dim3(256), prep_smem, s, g, scratch, c, now,
                 (const float*)m[pass & 1], m[1 - (pass & 1)]);

@@ -719,8 +719,8 @@ def _state_walk(step, state, out, heads, dim, vdim, raw, *, mode, q, k, v, gate,
         pairs = step.B * heads
         passes = min(chunks, max(1, CHUNK_SCRATCH // (4 * pairs * each)))
         scratch = torch.empty(pairs * (each * passes + 2), dtype=torch.float32, device=out.device)
-        _call("state_walk", "mb_state_chunks", [_c.c_char_p, _vp, _ll, _i, _vp], args, _ptr(scratch),
-              scratch.numel(), step.max_new, _stream(), launches=2 * -(-chunks // passes) + 1)
+        _call("state_walk", "mb_state_chunks", [_c.c_char_p, _vp, _ll, _i, _i, _vp], args, _ptr(scratch),
+              scratch.numel(), step.max_new, _sms(), _stream(), launches=2 * -(-chunks // passes) + 1)
         return
     _call("state_walk", "mb_state_walk", [_c.c_char_p, _i, _vp], args, _sms(), _stream(), launches=2)
 
