@@ -556,26 +556,16 @@ static int clusters_at_once(SplitKernel kernel, int n, int smem) {
 // The values of a row of the planes: K up to whole 16 bytes.
 static long long padded_k(int K) { return (K + 7ll) / 8 * 8; }
 
-// Bytes of scratch that mb_gemm_split needs for M rows.
-MB_EXPORT long long mb_gemm_split_scratch(int M, int K) { return 6ll * M * padded_k(K); }
+// Bytes of scratch of a product of M rows, with no more than `most` (but one row's).
+MB_EXPORT long long mb_gemm_split_scratch(int M, int K, long long most) {
+  const long long row = 6 * padded_k(K), fit = most / row;
+  return row * (M <= fit ? M : fit >= GS_COLS ? fit / GS_COLS * GS_COLS : fit > 0 ? fit : 1);
+}
 
-// C[M, N] (row stride ldc) = A[M, K] (row stride lda) · W[N, K]ᵀ, all float32 (C may be bfloat16,
-// except for EPI_ADD). For EPI_SWIGLU_PAIRS, W is [2N, K] and its rows alternate gate and up.
-// `scratch`: mb_gemm_split_scratch(M, K) bytes on a 16-byte boundary. `force_cols`,
-// `force_splits`: 0 for the rule's choice.
-MB_EXPORT int mb_gemm_split(const void* A, int lda, const void* W, void* C, int c_dtype, int ldc,
-                            int M, int N, int K, int epilogue, int sms, int force_cols,
-                            int force_splits, void* scratch, long long scratch_bytes, void* error,
-                            void* stream) {
-  if (M <= 0 || N <= 0) return 0;
-  if (K <= 0) MB_FAIL("mb_gemm_split: K = %d", K);
-  if (epilogue != EPI_STORE && epilogue != EPI_ADD && epilogue != EPI_SWIGLU_PAIRS)
-    MB_FAIL("mb_gemm_split: epilogue %d", epilogue);
-  if (epilogue == EPI_ADD && c_dtype != MB_F32) MB_FAIL("mb_gemm_split: the residual is float32");
-  if (scratch_bytes < mb_gemm_split_scratch(M, K))
-    MB_FAIL("mb_gemm_split: %lld bytes of scratch, %lld needed", scratch_bytes, mb_gemm_split_scratch(M, K));
-  if (M > 0x7fffffff / 3) MB_FAIL("mb_gemm_split: %d rows are too many for one launch", M);
-  cudaStream_t s = (cudaStream_t)stream;
+// M rows whose parts fit into the scratch: the two kernels
+static int split_rows(const void* A, int lda, const void* W, void* C, int c_dtype, int ldc, int M, int N,
+                      int K, int epilogue, int sms, int force_cols, int force_splits, void* scratch,
+                      void* error, cudaStream_t s) {
   const int Kp = (int)padded_k(K);
   SplitArgs p;
   p.A = (const float*)A; p.W = (const float*)W; p.C = C;
@@ -633,4 +623,31 @@ MB_EXPORT int mb_gemm_split(const void* A, int lda, const void* W, void* C, int 
   else
     mb_launch(kernel, dim3(grid), dim3(GS_THREADS), smem, s, map, p);
   MB_CHECK_LAUNCH("mb_gemm_split");
+}
+
+// C[M, N] (row stride ldc) = A[M, K] (row stride lda) · W[N, K]ᵀ, all float32 (C may be bfloat16,
+// except for EPI_ADD). For EPI_SWIGLU_PAIRS, W is [2N, K] and its rows alternate gate and up.
+// `scratch`: on a 16-byte boundary, mb_gemm_split_scratch bytes; with less than all rows' room the rows
+// go in bands, one after the other through the same scratch (a band's cut waits for the product
+// before it). `force_cols`, `force_splits`: 0 for the rule's choice.
+MB_EXPORT int mb_gemm_split(const void* A, int lda, const void* W, void* C, int c_dtype, int ldc,
+                            int M, int N, int K, int epilogue, int sms, int force_cols,
+                            int force_splits, void* scratch, long long scratch_bytes, void* error,
+                            void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0) MB_FAIL("mb_gemm_split: K = %d", K);
+  if (epilogue != EPI_STORE && epilogue != EPI_ADD && epilogue != EPI_SWIGLU_PAIRS)
+    MB_FAIL("mb_gemm_split: epilogue %d", epilogue);
+  if (epilogue == EPI_ADD && c_dtype != MB_F32) MB_FAIL("mb_gemm_split: the residual is float32");
+  const long long fit = scratch_bytes / (6 * padded_k(K));
+  if (fit < 1) MB_FAIL("mb_gemm_split: %lld bytes of scratch, a row needs %lld", scratch_bytes, 6 * padded_k(K));
+  if ((fit < M ? fit : M) > 0x7fffffff / 3) MB_FAIL("mb_gemm_split: %d rows are too many for one launch", M);
+  for (long long m = 0; m < M; m += fit) {
+    const int rows = (int)(M - m < fit ? M - m : fit);
+    const int rc = split_rows((const float*)A + m * lda, lda, W,
+                              (char*)C + m * ldc * (c_dtype == MB_BF16 ? 2 : 4), c_dtype, ldc, rows, N, K,
+                              epilogue, sms, force_cols, force_splits, scratch, error, (cudaStream_t)stream);
+    if (rc) return rc;
+  }
+  return 0;
 }

@@ -171,13 +171,13 @@ def read_trace() -> list:
 _functions: dict = {}      # entry points by name, with their library, once they were called
 
 
-def _function(libname: str, fn: str, argtypes):
+def _function(libname: str, fn: str, argtypes, restype=_i):
     """The library's entry point with its argument types set, and the library. Found once: a
     step of a few tokens is bound by what the host does for each of its launches."""
     lib = build.load_library(libname)
     f = getattr(lib, fn)
     f.argtypes = argtypes
-    f.restype = _i
+    f.restype = restype
     _functions[fn] = f, lib
     return f, lib
 
@@ -1347,6 +1347,13 @@ def attention_diff_prefill_tc(q: torch.Tensor, out: torch.Tensor, step, line, nh
 # (17 rows, 64 x 64 back to back: 10.3 us with fma, 11 to 17; 17 rows, 128 x 128: 17.4 and 16.4; 24
 # rows, 1,024 x 2,048: 41 and 19.5).
 SPLIT_ROWS, SPLIT_K = 16, 64
+SPLIT_SCRATCH = 256 << 20       # bytes of the rows' parts; more rows go in bands
+
+
+@functools.lru_cache(maxsize=1024)
+def _split_scratch(M: int, K: int, most: int) -> int:
+    f, _ = _function("gemm_split", "mb_gemm_split_scratch", [_i, _i, _ll], _ll)
+    return f(M, K, most)
 
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPI_STORE,
@@ -1377,11 +1384,12 @@ def gemm_split(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int 
     """``gemm_simt`` of float32 operands on the tensor cores, every value in three bfloat16 parts
     (``csrc/gemm_split.cu``). ``cols`` and ``splits``: 0, or a tile's rows of a and K's parts."""
     M, Kd = a.shape
-    scratch = torch.empty(6 * M * (-(-Kd // 8) * 8), dtype=torch.uint8, device=a.device)
+    scratch = torch.empty(_split_scratch(M, Kd, SPLIT_SCRATCH), dtype=torch.uint8, device=a.device)
     _call("gemm_split", "mb_gemm_split",
           [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _ll, _vp, _vp],
           _ptr(a), a.stride(0), _ptr(w), _ptr(c), code_of(c.dtype), c.stride(0), M, c.shape[1], Kd,
-          epilogue, _sms(), cols, splits, _ptr(scratch), scratch.numel(), _ptr(error), _stream(), launches=2)
+          epilogue, _sms(), cols, splits, _ptr(scratch), scratch.numel(), _ptr(error), _stream(),
+          launches=2 * -(-M // (scratch.numel() // _split_scratch(1, Kd, SPLIT_SCRATCH))))
 
 
 # ------------------------------------------------------------------------------ attention

@@ -118,3 +118,36 @@ def test_small_values(M, N, Kd, splits):
     assert not c_add.isnan().any()
     fine = want.isfinite()
     assert (c_add.double() - want)[fine].norm() <= 4e-7 * want[fine].norm() and int(error) == 0
+
+
+# the rows' parts take no more than SPLIT_SCRATCH: more rows go in bands of whole tiles through the same
+# scratch, whole numbers so that every sum is exact
+@pytest.mark.parametrize("rows", [1, 100, 128, 300])
+@pytest.mark.parametrize("epilogue", [K.EPI_STORE, K.EPI_ADD, K.EPI_SWIGLU_PAIRS])
+def test_bands(monkeypatch, rows, epilogue):
+    M, N, Kd = 411, 260, 1090
+    a, w, c = drawn((M, Kd + 3), 1, True)[:, :Kd], drawn((N, Kd), 2, True), drawn((M, N), 3, True)
+    if epilogue == K.EPI_SWIGLU_PAIRS:
+        a, w, c = a * 0.05, w * 0.25, c[:, :N // 2].bfloat16()
+    want = c.clone()
+    K.gemm_split(a, w, want, epilogue)
+    monkeypatch.setattr(K, "SPLIT_SCRATCH", 6 * 1096 * rows + 7)
+    if rows == 1:
+        a, c, want = a[:5], c[:5], want[:5]
+    K.gemm_split(a, w, c, epilogue, cols=0 if epilogue != K.EPI_SWIGLU_PAIRS else 128)
+    if epilogue == K.EPI_SWIGLU_PAIRS:      # other tiles, other sums: half a place of bfloat16
+        assert (c.double() - want.double()).norm() <= 2.0 ** -8 * want.double().norm()
+    else:
+        assert torch.equal(c, want)
+
+
+# a prefill of the default step size: 16,384 rows of 12,288 values
+def test_memory():
+    a, w = torch.zeros((16384, 12288), device=DEV), torch.zeros((128, 12288), device=DEV)
+    out = torch.empty((16384, 128), device=DEV)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    K.gemm_simt(a, w, out)
+    assert torch.cuda.max_memory_allocated() - before <= 256 << 20
+    assert not out.any()
