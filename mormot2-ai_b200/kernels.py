@@ -677,22 +677,31 @@ CHUNK = 32                      # SC_C of csrc/state_chunks.cuh
 CHUNK_SCRATCH = 160 << 20       # bytes of chunks' factors that a pass may take
 
 
+@functools.lru_cache(maxsize=1024)
+def _chunk_floats(mode: int, B: int, heads: int, dim: int, vdim: int, chunks: int) -> int:
+    """Floats of scratch for so many chunks of every sequence."""
+    f, _ = _function("state_walk", "mb_state_chunks_scratch", [_i] * 6, _ll)
+    return f(mode, B, heads, dim, vdim, chunks)
+
+
 def walks_in_chunks(step, dim: int, vdim: int, mode: int, heads: int) -> bool:
     """Whether a step that goes by fours goes in chunks of 32 tokens instead (csrc/state_chunks.cuh).
-    That takes a third of the time for a long sequence's tokens and 10 us before the first, and pays
-    less the more (sequence, head) pairs there are to fill the device by fours already. Measured, walk
-    and norm, us by fours | in chunks: delta rule, 16 heads of 128 x 128, one prompt of 64 / 128 / 1,000:
-    30 | 35, 41 | 39, 202 | 117; three 54 | 40, 87 | 57, 551 | 345; eight of 64 / 400 101 | 78, 464 |
-    370; 63 decoding beside 256 284 | 580. 8 heads of 64 x 128, three prompts of 64 / 128 24 | 26, 36 |
-    31, eight of 128 / 200 46 | 46, 63 | 71. Matrix memory, 8 heads of 128 x 128, one prompt of 64 / 96 /
-    1,000: 28 | 25, 30 | 27, 164 | 111; eight of 64 / 400 61 | 38, 245 | 123; 63 decoding beside 128
-    153 | 111; 4 heads of 64 x 64, one of 64 / 96 22 | 21, 26 | 24. (Chunks: before their sums were kept
-    from leaning, which takes 3 to 4 in a hundred.)"""
+    That takes half the time for a long sequence's tokens and 10 us before the first, and pays less the
+    more (sequence, head) pairs there are to fill the device by fours already. Measured, walk and norm, us
+    by fours | in chunks: delta rule, 16 heads of 128 x 128, one prompt of 64 / 128 / 1,000: 25.2 | 25.4,
+    38 | 31, 222 | 150; two of 64 31.4 | 32.4; three of 64 / 128 / 1,000 53 | 39, 89 | 60, 640 | 447; eight
+    of 64 / 400 103 | 77, 518 | 435; 63 decoding beside 256 286 | 579. 8 heads of 64 x 128, one prompt of
+    96 / 128 26 | 23, 32 | 25, four of 64 23.8 | 24.1, six
+    of 200 68.6 | 70.9, of 400 128 | 128, eight of 200 / 400 66 | 74, 127 | 131. Matrix memory, 8 heads of
+    128 x 128, one prompt of 64 / 96 / 1,000: 23.7 | 20.1, 29 | 23, 172 | 104; eight of 64 / 400 61 | 36,
+    270 | 151; 63 decoding beside 128 147 | 112; 4 heads of 64 x 64, one of 64 / 96 20 | 17, 24 | 19. Where
+    one chunk of every sequence takes more scratch than CHUNK_SCRATCH, by fours."""
     if mode not in (WALK_DELTA, WALK_MLSTM) or dim % 16 or dim > 128 or vdim % 16:
         return False
     n, pairs = step.max_new, step.B * heads
     if mode == WALK_MLSTM:
-        return n >= (64 if pairs >= 64 else 96)
+        return (n >= (64 if pairs >= 64 else 96)
+                and 4 * _chunk_floats(mode, step.B, heads, dim, vdim, 1) <= CHUNK_SCRATCH)
     return n >= (64 if pairs > 24 else 128) and pairs <= (48 if dim <= 64 else 128)
 
 
@@ -714,13 +723,12 @@ def _state_walk(step, state, out, heads, dim, vdim, raw, *, mode, q, k, v, gate,
     if (walks_in_chunks(step, dim, vdim, mode, heads) and ldq % 4 == 0 and ldk % 4 == 0
             and ldv % 4 == 0 and (q | k | v) % 16 == 0):
         chunks = -(-step.max_new // CHUNK)
-        each = 1728 + dim // 16 * 192 * (12 if mode == WALK_DELTA else 8) + (
-            CHUNK * vdim if mode == WALK_DELTA else 0)      # sc_chunk_floats of csrc/state_chunks.cuh
-        pairs = step.B * heads
-        passes = min(chunks, max(1, CHUNK_SCRATCH // (4 * pairs * each)))
-        scratch = torch.empty(pairs * (each * passes + 2), dtype=torch.float32, device=out.device)
+        each = _chunk_floats(mode, step.B, heads, dim, vdim, 1)
+        per_pass = min(chunks, max(1, CHUNK_SCRATCH // (4 * each)))
+        scratch = torch.empty(_chunk_floats(mode, step.B, heads, dim, vdim, per_pass),
+                              dtype=torch.float32, device=out.device)
         _call("state_walk", "mb_state_chunks", [_c.c_char_p, _vp, _ll, _i, _i, _vp], args, _ptr(scratch),
-              scratch.numel(), step.max_new, _sms(), _stream(), launches=2 * -(-chunks // passes) + 1)
+              scratch.numel(), step.max_new, _sms(), _stream(), launches=2 * -(-chunks // per_pass) + 1)
         return
     _call("state_walk", "mb_state_walk", [_c.c_char_p, _i, _vp], args, _sms(), _stream(), launches=2)
 

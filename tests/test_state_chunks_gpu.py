@@ -1,5 +1,7 @@
 """The delta rule and the matrix memory in chunks of 32 tokens: outputs and states against float64 and
 against the same four tokens at a time, in one pass and in several, and what is no number."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -173,3 +175,10 @@ def test_an_update_that_overflows(monkeypatch):
     assert want.isposinf().any() and want.isneginf().any() and not want.isnan().any()
     assert torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
     assert not got.isnan().any()
+
+
+# the matrix memory's chunks take scratch for one chunk of every sequence at least (56 KB a head of 128 x 128):
+# where that is more than CHUNK_SCRATCH the step goes by fours
+def test_rule_of_the_scratch():
+    got = [K.walks_in_chunks(SimpleNamespace(B=B, max_new=96), 128, 128, K.WALK_MLSTM, 8) for B in (64, 350, 380, 4000)]
+    assert got == [True, True, False, False]
