@@ -1,6 +1,8 @@
-"""The float32 products' forms at their edges: rows up to 16 (warps that share a weight row's K)
-and more (tiles of 64 x 128, K dealt out over a cluster). Small whole numbers make every sum
-exact, so the results must equal the oracle's bit for bit; SwiGLU is compared in float64."""
+"""The float32 products' forms at their edges: rows up to 16 (warps that share a weight row's K) and
+more: float32 operands on the tensor cores where K is above 64 (test_split_products_gpu.py has that
+form's own edges), an operand in bfloat16 in tiles of 64 x 128, K dealt out over a cluster. Small
+whole numbers make every sum exact, so the results must equal the oracle's bit for bit; SwiGLU is
+compared in float64."""
 import pytest
 import torch
 
@@ -75,5 +77,25 @@ def test_few_rows(M, N, Kd, types):
     z = exact.double() / 64
     for epilogue, g, u in ((K.EPI_SWIGLU_PAIRS, z[:, 0::2], z[:, 1::2]), (K.EPI_SWIGLU, z[:, :N], z[:, N:])):
         K.gemm_simt(a, w, out := torch.empty((M, N), device=DEV), epilogue)
+        want = torch.nn.functional.silu(g) * u
+        assert (out.double() - want).norm() <= 2e-6 * want.norm()      # exact sums, expf and a division
+
+
+# many rows with an operand in bfloat16: tiles of 64 x 128, K dealt out over up to eight CTAs (2,048 and 4,096),
+# a ragged last step (132), no whole pieces of four values (1,030, 37)
+@pytest.mark.parametrize("M", [17, 64, 65, 200])
+@pytest.mark.parametrize("N, Kd", [(3, 37), (130, 132), (96, 1030), (1024, 2048), (260, 4096)])
+@pytest.mark.parametrize("types", ["fb", "bb", "bf"])
+def test_many_rows_in_bfloat16(M, N, Kd, types):
+    kind = {"f": torch.float32, "b": torch.bfloat16}
+    a, w, c = whole((M, Kd), 1).to(kind[types[0]]), whole((2 * N, Kd), 2).to(kind[types[1]]), whole((M, N), 3, 50)
+    exact = a.float() @ w.float().t()
+    K.gemm_simt(a, w, out := torch.empty((M, 2 * N), device=DEV))
+    assert torch.equal(out, exact)
+    K.gemm_simt(a, w[:N], c_add := c.clone(), K.EPI_ADD)
+    assert torch.equal(c_add, c + exact[:, :N])
+    z = exact.double() / 64
+    for epilogue, g, u in ((K.EPI_SWIGLU_PAIRS, z[:, 0::2], z[:, 1::2]), (K.EPI_SWIGLU, z[:, :N], z[:, N:])):
+        K.gemm_simt(a * 0.0625, w * 0.25, out := torch.empty((M, N), device=DEV), epilogue)
         want = torch.nn.functional.silu(g) * u
         assert (out.double() - want).norm() <= 2e-6 * want.norm()      # exact sums, expf and a division
