@@ -14,8 +14,8 @@
 // per head and 16 columns of the state; its operands come straight from L2 into registers, a chunk
 // ahead.
 //
-// Products go through mma.sync (m16n8k16) with every float32 value cut into three exact bfloat16
-// parts (common.cuh), six products of parts, the smallest first: an accumulator cuts off what falls
+// Products go through mma.sync (m16n8k16) with every float32 value cut into three bfloat16 parts that
+// sum up to it (common.cuh), six products of parts, the smallest first: an accumulator cuts off what falls
 // behind its last place, so the leading products come last and few to an accumulator, and sums over
 // warps and chunks are made with float32 additions. What goes into the state chunk after chunk leans to
 // neither side: the first operand's leading part is the nearest one, and what an accumulator cut off its

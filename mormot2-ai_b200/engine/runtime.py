@@ -25,8 +25,9 @@ class Runtime:
         self.guards = guards
         self.dtype = dtype
         self.device = torch.device(device)
-        # the tensor-core kernels serve the bfloat16 path only; the 32-bit path multiplies and
-        # adds in float32 throughout
+        # the bfloat16 tensor-core kernels serve the bfloat16 path only; the 32-bit path multiplies
+        # and adds in float32, or on the tensor cores with every value in three bfloat16 parts
+        # (csrc/gemm_split.cu, csrc/attention_split.cuh, csrc/state_chunks.cuh)
         self.fast_kernels = fast_kernels and dtype == torch.bfloat16
         # True: the tensors handed to ``bind`` belong to the engine alone, and a part that
         # re-lays a weight out (fused q/k/v, interleaved gate and up) drops the original
@@ -78,8 +79,10 @@ class Runtime:
     def _raise_if(self, code: int) -> None:
         if code:
             self.error_word.zero_()
-            raise KernelError(f"a kernel gave up a wait (code {code}: 1 load, 2 MMA, "
-                              "3 epilogue; 4-5, 9-19 attention); its result is not valid")
+            raise KernelError(f"a kernel gave up a wait (code {code}: 1 load, 2 MMA, 3 epilogue, "
+                              "6 accumulator; 4-5, 9-18 attention, 11-13 and 16 a product of CTA "
+                              "pairs too; 41-48 float32 products in parts; 51-59 float32 attention "
+                              "in parts); its result is not valid")
 
     def token_box(self, rows: int) -> Optional[torch.Tensor]:
         """Where a sampler may leave ``rows`` chosen tokens for ``read_tokens`` (None: too many)."""

@@ -3,8 +3,8 @@ with the epilogue fused: store, add into the float32 residual, or SwiGLU over ga
 
 The kernel is chosen by the operand types and sizes: the tensor-core kernels for bfloat16
 operands whose sizes they take, else the float32 products: multiply-adds for few rows and for
-mixed types, the tensor cores with every value cut into three exact bfloat16 parts for more rows
-of float32 (a weight stored in 32 bits stays so, and its products are those of 32 bits).
+mixed types, the tensor cores with every value cut into three bfloat16 parts that sum up to it for
+more rows of float32 (a weight stored in 32 bits stays so, and its products are those of 32 bits).
 """
 from __future__ import annotations
 

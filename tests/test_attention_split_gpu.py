@@ -66,7 +66,8 @@ def test_what_is_no_number(where, monkeypatch):
     assert (got[fine] - want[fine]).abs().max() <= 1e-5 if fine.any() else True
 
 
-# the error against float64 is no larger than that of the float32 kernel's multiply-adds
+# the error against float64 is at most a fifth above that of the float32 kernel's multiply-adds (measured:
+# below it; single inputs vary)
 @pytest.mark.parametrize("n, past", [(128, 0), (200, 1500)])
 def test_error(n, past, monkeypatch):
     k, v, q = draw(n, past, 4, 4, 2)
