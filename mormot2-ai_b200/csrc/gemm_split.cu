@@ -2,6 +2,8 @@
 // few rows takes. Every float32 value from 2^-110 up is the exact sum of three bfloat16 parts of 8
 // significant bits each (hi + mid + lo: its 24 bits cut in three), so a product of two values is a sum of nine
 // products of parts; six of them are computed, the other three lie 2^-24 and less below the whole.
+// (The method: G. Henry, P. Tang, A. Heinecke, Leveraging the bfloat16 artificial intelligence datatype
+// for higher-precision computations, 2019.)
 // tcgen05 multiplies exactly and adds in float32, but cuts off what falls behind the accumulator's
 // last place instead of rounding. So no long sum is left to it: hi·hi is drained from tensor memory
 // every 64 values of K and added up in registers, rounded to nearest; only the five products that

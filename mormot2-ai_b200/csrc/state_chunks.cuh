@@ -8,6 +8,9 @@
 //   both     o_t = G_t q_t . S0 + sum_{s <= t} N_ts u_s,  N_ts = D_ts (q_t . k_s) (mlstm: times b_s)
 //            S = G_31 S0 + sum_s D_31,s k_s u_s^T (mlstm: times b_s)
 //
+// (The delta rule in chunks: S. Yang et al., Parallelizing linear transformers with the delta rule over
+// sequence length, 2024.)
+//
 // All that does not need S0 is made by a block per chunk and head (state_chunk_prep_kernel), all chunks
 // at once, and left in scratch as the operands that the walk's lanes will hold. The walk
 // (state_chunk_walk_kernel) is then three small products a chunk with two barriers between them, a CTA
